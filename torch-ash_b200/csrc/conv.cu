@@ -264,6 +264,92 @@ __global__ void __launch_bounds__(256) conv_separable_kernel(const float* __rest
     }
 }
 
+// The same filter for the block edges and radii that are compiled in (G of 4, 8, 16 and R of 1, 2, 3).
+// Bound by shared-memory accesses and instruction issue, so the tile is touched as little as possible:
+// a thread takes one line of the tile (one channel of a row, a column or a pillar), reads it once into
+// registers, slides the window over it there and writes the sums back in the line's own place.  A line
+// is read and written by its own thread alone, so one buffer serves all three passes (47 KB at G = 8,
+// R = 3, four channels: four CTAs per SM instead of three with the 70 KB of conv_separable_kernel) and a
+// tile value costs one access per pass instead of 2R + 1.  Rows are T + 1 cells apart: T is even, so eight
+// rows start in different bank groups.  The halo arrives by cp.async, absent blocks as zero-filled copies.
+// Every sum has the terms and the order of conv_separable_kernel, which stays for all other sizes.
+template <int BYTES>
+__device__ __forceinline__ void copy_async(float* dst, const float* src, bool present) {
+    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"(d), "l"(src), "n"(BYTES), "r"(present ? BYTES : 0)
+                 : "memory");
+}
+
+// out[o] = sum over k of w[k] * line[o + k], in place, the line's values `stride` floats apart.
+template <int N, int S, class Store>
+__device__ __forceinline__ void filter_line(const float* line, int stride, const float* w, int w_stride, Store&& store) {
+    float wv[S], v[N + S - 1];
+#pragma unroll
+    for (int k = 0; k < S; ++k) wv[k] = w[k * w_stride];
+#pragma unroll
+    for (int i = 0; i < N + S - 1; ++i) v[i] = line[i * stride];
+#pragma unroll
+    for (int o = 0; o < N; ++o) {
+        float acc = 0.f;
+#pragma unroll
+        for (int k = 0; k < S; ++k) acc += v[o + k] * wv[k];
+        store(o, acc);
+    }
+}
+
+template <int CH, int G, int R>
+__global__ void __launch_bounds__(256) conv_separable_lines_kernel(const float* __restrict__ in,
+                                                                   const float* __restrict__ w1,
+                                                                   const int64_t* __restrict__ grid_indices,
+                                                                   const int64_t* __restrict__ g2g27,
+                                                                   float* __restrict__ out, int D, int64_t n_emb) {
+    constexpr int S = 2 * R + 1, T = G + 2 * R, ROW = (T + 1) * CH, SLAB = T * ROW, CELLS = G * G * G;
+    extern __shared__ __align__(16) float tile[];   // [T][T][T + 1][CH]
+    __shared__ float wsm[3 * S * CH];
+    __shared__ const float* nb[27];
+    const int64_t gidx = grid_indices[blockIdx.x];
+    const bool ok = gidx >= 0 && gidx < n_emb;
+    if (threadIdx.x < 27) {
+        const int64_t g = ok ? g2g27[gidx * 27 + threadIdx.x] : -1;
+        nb[threadIdx.x] = g >= 0 && g < n_emb ? in + g * CELLS * D : nullptr;
+    }
+    __syncthreads();
+    if (!ok) return;
+    for (int ch0 = 0; ch0 < D; ch0 += CH) {
+        for (int h = threadIdx.x; h < T * T * T; h += blockDim.x) {
+            const int hx = h % T, hy = (h / T) % T, hz = h / (T * T);
+            const int cx = hx - R, cy = hy - R, cz = hz - R;
+            const int bx = cx < 0 ? -1 : (cx >= G ? 1 : 0), by = cy < 0 ? -1 : (cy >= G ? 1 : 0),
+                      bz = cz < 0 ? -1 : (cz >= G ? 1 : 0);
+            const float* block = nb[(bx + 1) + (by + 1) * 3 + (bz + 1) * 9];
+            const int lin = (cx - bx * G) + ((cy - by * G) + (cz - bz * G) * G) * G;
+            copy_async<CH * 4>(tile + (hz * T + hy) * ROW + hx * CH, block ? block + lin * D + ch0 : in, block != nullptr);
+        }
+        for (int k = threadIdx.x; k < 3 * S * CH; k += blockDim.x) wsm[k] = w1[(int64_t)(k / CH) * D + ch0 + (k % CH)];
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        __syncthreads();
+        for (int i = threadIdx.x; i < T * T * CH; i += blockDim.x) {   // rows, along x
+            const int c = i % CH;
+            float* line = tile + (i / CH) * ROW + c;
+            filter_line<G, S>(line, CH, wsm + c, CH, [&](int o, float v) { line[o * CH] = v; });
+        }
+        __syncthreads();
+        for (int i = threadIdx.x; i < T * G * CH; i += blockDim.x) {   // columns, along y
+            const int c = i % CH;
+            float* line = tile + (i / (G * CH)) * SLAB + i % (G * CH);
+            filter_line<G, S>(line, ROW, wsm + S * CH + c, CH, [&](int o, float v) { line[o * ROW] = v; });
+        }
+        __syncthreads();
+        for (int i = threadIdx.x; i < G * G * CH; i += blockDim.x) {   // pillars, along z
+            const int c = i % CH, xy = i / CH;
+            const float* line = tile + (xy / G) * ROW + i % (G * CH);
+            float* dst = out + (gidx * CELLS + xy) * D + ch0 + c;
+            filter_line<G, S>(line, SLAB, wsm + 2 * S * CH + c, CH, [&](int o, float v) { dst[(int64_t)o * G * G * D] = v; });
+        }
+        __syncthreads();
+    }
+}
+
 }  // namespace ashb
 
 using namespace ashb;
@@ -365,8 +451,29 @@ int ashb_conv_forward_separable(const float* inputs, const float* weights_1d, co
     if (zero_output) ASHB_CUDA_TRY(cudaMemsetAsync(outputs, 0, (size_t)n_emb * cells * D * sizeof(float), st));
     if (num_grids == 0) return ASHB_OK;
     ASHB_REQUIRE(inputs && weights_1d && grid_indices && lut_grid_nb27, "null buffer");
-    const int ch = (D % 4 == 0 && ((((uintptr_t)inputs) | ((uintptr_t)outputs)) & 15) == 0) ? 4 : (D % 2 == 0 ? 2 : 1);
+    const uintptr_t bits = (uintptr_t)inputs | (uintptr_t)outputs;
+    const int ch = D % 4 == 0 && (bits & 15) == 0 ? 4 : (D % 2 == 0 && (bits & 7) == 0 ? 2 : 1);
     const int T = G + 2 * radius, S = 2 * radius + 1;
+#define ASHB_SEP_LINES(CH, GG, RR)                                                                                      \
+    if (ch == CH && G == GG && radius == RR) {                                                                          \
+        constexpr int TT = GG + 2 * RR;                                                                                 \
+        constexpr size_t bytes = (size_t)TT * TT * (TT + 1) * CH * sizeof(float);                                       \
+        if (bytes > 48 * 1024)                                                                                          \
+            ASHB_CUDA_TRY(cudaFuncSetAttribute(conv_separable_lines_kernel<CH, GG, RR>,                                 \
+                                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));               \
+        conv_separable_lines_kernel<CH, GG, RR><<<(unsigned)num_grids, GG == 4 ? 128 : 256, bytes, st>>>(               \
+                inputs, weights_1d, grid_indices, lut_grid_nb27, outputs, (int)D, n_emb);                               \
+        ASHB_LAUNCH_CHECK();                                                                                            \
+        return ASHB_OK;                                                                                                 \
+    }
+#define ASHB_SEP_LINES_R(CH, GG) ASHB_SEP_LINES(CH, GG, 1) ASHB_SEP_LINES(CH, GG, 2) ASHB_SEP_LINES(CH, GG, 3)
+#define ASHB_SEP_LINES_G(CH) ASHB_SEP_LINES_R(CH, 4) ASHB_SEP_LINES_R(CH, 8) ASHB_SEP_LINES_R(CH, 16)
+    ASHB_SEP_LINES_G(4)
+    ASHB_SEP_LINES_G(2)
+    ASHB_SEP_LINES_G(1)
+#undef ASHB_SEP_LINES_G
+#undef ASHB_SEP_LINES_R
+#undef ASHB_SEP_LINES
     const size_t smem = ((size_t)T * T * T + (size_t)T * T * G + (size_t)3 * S) * ch * sizeof(float);
     ASHB_REQUIRE(smem <= 200 * 1024, "halo tile of %zu bytes does not fit in shared memory", smem);
 #define ASHB_SEP_LAUNCH(CH)                                                                                   \
