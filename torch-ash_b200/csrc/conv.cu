@@ -276,23 +276,24 @@ __global__ void __launch_bounds__(256) conv_separable_kernel(const float* __rest
 template <int BYTES>
 __device__ __forceinline__ void copy_async(float* dst, const float* src, bool present) {
     const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"(d), "l"(src), "n"(BYTES), "r"(present ? BYTES : 0)
-                 : "memory");
+    if constexpr (BYTES == 16)   // past L1: a CTA reads a cell once
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(present ? 16 : 0) : "memory");
+    else
+        asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"(d), "l"(src), "n"(BYTES), "r"(present ? BYTES : 0)
+                     : "memory");
 }
 
-// out[o] = sum over k of w[k] * line[o + k], in place, the line's values `stride` floats apart.
-template <int N, int S, class Store>
-__device__ __forceinline__ void filter_line(const float* line, int stride, const float* w, int w_stride, Store&& store) {
-    float wv[S], v[N + S - 1];
+// store(o, sum over k of w[k] * line[o + k]) for N sums of a line whose values are STRIDE floats apart.
+template <int N, int S, int STRIDE, class Store>
+__device__ __forceinline__ void filter_line(const float* line, const float* w, Store&& store) {
+    float v[N + S - 1];
 #pragma unroll
-    for (int k = 0; k < S; ++k) wv[k] = w[k * w_stride];
-#pragma unroll
-    for (int i = 0; i < N + S - 1; ++i) v[i] = line[i * stride];
+    for (int i = 0; i < N + S - 1; ++i) v[i] = line[i * STRIDE];
 #pragma unroll
     for (int o = 0; o < N; ++o) {
         float acc = 0.f;
 #pragma unroll
-        for (int k = 0; k < S; ++k) acc += v[o + k] * wv[k];
+        for (int k = 0; k < S; ++k) acc += v[o + k] * w[k];
         store(o, acc);
     }
 }
@@ -304,6 +305,7 @@ __global__ void __launch_bounds__(256) conv_separable_lines_kernel(const float* 
                                                                    const int64_t* __restrict__ g2g27,
                                                                    float* __restrict__ out, int D, int64_t n_emb) {
     constexpr int S = 2 * R + 1, T = G + 2 * R, ROW = (T + 1) * CH, SLAB = T * ROW, CELLS = G * G * G;
+    constexpr int WIDE = T <= 8 ? 8 : (T <= 16 ? 16 : 32);
     extern __shared__ __align__(16) float tile[];   // [T][T][T + 1][CH]
     __shared__ float wsm[3 * S * CH];
     __shared__ const float* nb[27];
@@ -316,35 +318,54 @@ __global__ void __launch_bounds__(256) conv_separable_lines_kernel(const float* 
     __syncthreads();
     if (!ok) return;
     for (int ch0 = 0; ch0 < D; ch0 += CH) {
-        for (int h = threadIdx.x; h < T * T * T; h += blockDim.x) {
-            const int hx = h % T, hy = (h / T) % T, hz = h / (T * T);
-            const int cx = hx - R, cy = hy - R, cz = hz - R;
-            const int bx = cx < 0 ? -1 : (cx >= G ? 1 : 0), by = cy < 0 ? -1 : (cy >= G ? 1 : 0),
-                      bz = cz < 0 ? -1 : (cz >= G ? 1 : 0);
-            const float* block = nb[(bx + 1) + (by + 1) * 3 + (bz + 1) * 9];
-            const int lin = (cx - bx * G) + ((cy - by * G) + (cz - bz * G) * G) * G;
-            copy_async<CH * 4>(tile + (hz * T + hy) * ROW + hx * CH, block ? block + lin * D + ch0 : in, block != nullptr);
+        // a thread keeps its (x, y) of the tile and walks the slabs: the three blocks it reads are three pointers
+        for (int hy = threadIdx.x / WIDE; hy < T; hy += blockDim.x / WIDE) {
+            const int hx = threadIdx.x % WIDE;
+            if (hx >= T) break;
+            const int bx = (hx >= R) + (hx >= G + R), by = (hy >= R) + (hy >= G + R);
+            const int xy = (hx + G - R) % G + (hy + G - R) % G * G;
+            const float* from[3];
+            bool present[3];
+#pragma unroll
+            for (int bz = 0; bz < 3; ++bz) {
+                const float* block = nb[bx + by * 3 + bz * 9];
+                present[bz] = block != nullptr;
+                from[bz] = (present[bz] ? block : in) + xy * D + ch0;
+            }
+            float* to = tile + hy * ROW + hx * CH;
+#pragma unroll
+            for (int hz = 0; hz < T; ++hz) {
+                const int bz = (hz >= R) + (hz >= G + R);
+                copy_async<CH * 4>(to + hz * SLAB, from[bz] + (hz + G - R) % G * (G * G) * D, present[bz]);
+            }
         }
         for (int k = threadIdx.x; k < 3 * S * CH; k += blockDim.x) wsm[k] = w1[(int64_t)(k / CH) * D + ch0 + (k % CH)];
         asm volatile("cp.async.wait_all;" ::: "memory");
         __syncthreads();
+        // the block size is a multiple of CH: a thread stays with one channel and its weights
+        const int c = threadIdx.x % CH;
+        float w[S];
+#pragma unroll
+        for (int k = 0; k < S; ++k) w[k] = wsm[k * CH + c];
         for (int i = threadIdx.x; i < T * T * CH; i += blockDim.x) {   // rows, along x
-            const int c = i % CH;
             float* line = tile + (i / CH) * ROW + c;
-            filter_line<G, S>(line, CH, wsm + c, CH, [&](int o, float v) { line[o * CH] = v; });
+            filter_line<G, S, CH>(line, w, [&](int o, float v) { line[o * CH] = v; });
         }
+#pragma unroll
+        for (int k = 0; k < S; ++k) w[k] = wsm[(S + k) * CH + c];
         __syncthreads();
         for (int i = threadIdx.x; i < T * G * CH; i += blockDim.x) {   // columns, along y
-            const int c = i % CH;
             float* line = tile + (i / (G * CH)) * SLAB + i % (G * CH);
-            filter_line<G, S>(line, ROW, wsm + S * CH + c, CH, [&](int o, float v) { line[o * ROW] = v; });
+            filter_line<G, S, ROW>(line, w, [&](int o, float v) { line[o * ROW] = v; });
         }
+#pragma unroll
+        for (int k = 0; k < S; ++k) w[k] = wsm[(2 * S + k) * CH + c];
         __syncthreads();
         for (int i = threadIdx.x; i < G * G * CH; i += blockDim.x) {   // pillars, along z
-            const int c = i % CH, xy = i / CH;
+            const int xy = i / CH;
             const float* line = tile + (xy / G) * ROW + i % (G * CH);
             float* dst = out + (gidx * CELLS + xy) * D + ch0 + c;
-            filter_line<G, S>(line, SLAB, wsm + 2 * S * CH + c, CH, [&](int o, float v) { dst[(int64_t)o * G * G * D] = v; });
+            filter_line<G, S, SLAB>(line, w, [&](int o, float v) { dst[(int64_t)o * G * G * D] = v; });
         }
         __syncthreads();
     }
