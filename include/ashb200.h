@@ -191,6 +191,13 @@ int ashb_query_backward_backward(int dtype, int interp, const void* grad_grad_of
 int ashb_grid_build_neighbor_lut(ashb_map* map, int32_t* nb_lut, int32_t* grid_coords, int64_t n_emb,
                                  void* stream);
 
+/* The block window of any radius, one-sided (offsets 0..radius) or two-sided (-radius..radius), as the
+ * int64 table lut [n_emb][window^3] of SparseDenseGrid.construct_grid_neighbor_lut (ash/grid.py:566-617):
+ * x fastest, -1 for absent neighbours and in the rows of inactive indices; grid_coords as above.  list
+ * int32 [n_emb] and list_count (both or neither) receive the active rows in no particular order. */
+int ashb_grid_build_window_lut(ashb_map* map, int radius, int bidirectional, int64_t* lut, int32_t* grid_coords,
+                               int64_t n_emb, int32_t* list, int32_t* list_count, void* stream);
+
 /* out [n][D]; masks uint8 [n] = hash hit (a query whose neighbour block is absent keeps mask 1
  * and gets a zero row, as ash/src/grid.cu:109-111); block_idx_out int32 [n] (optional) = block
  * index per query, -1 on a miss, to be handed to the two backward entry points. */

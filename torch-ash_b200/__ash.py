@@ -65,6 +65,7 @@ _lib.ashb_tsdf_fuse_frame_static.argtypes = [_vp, _vp, _i64, _int, _i64, _vp, _v
                                              _vp, _int, _vp, _vp, _f32, _int, _int, _int, _vp]
 _lib.ashb_tsdf_copy_timeouts.argtypes = [_vp]
 _lib.ashb_grid_build_neighbor_lut.argtypes = [_vp, _vp, _vp, _i64, _vp]
+_lib.ashb_grid_build_window_lut.argtypes = [_vp, _int, _int, _vp, _vp, _i64, _vp, _vp, _vp]
 _lib.ashb_grid_query_forward.argtypes = [_vp, _int, _int, _vp, _vp, _c.c_double, _vp, _int, _vp, _vp, _vp, _vp, _i64, _i64, _i64, _vp]
 _lib.ashb_grid_query_backward.argtypes = [_vp, _int, _int, _vp, _vp, _vp, _c.c_double, _vp, _int, _vp, _vp, _vp, _vp, _int,
                                           _i64, _i64, _i64, _vp]
@@ -699,6 +700,19 @@ def grid_build_neighbor_lut(hashmap, num_embeddings, with_coords=False):
     _check(_lib.ashb_grid_build_neighbor_lut(
         hashmap._h, lut.data_ptr(), coords.data_ptr() if with_coords else None, num_embeddings, _stream(dev)))
     return (lut, coords) if with_coords else lut
+
+
+def grid_build_window_lut(hashmap, num_embeddings, radius, bidirectional):
+    """(grid_coords int32 (num_embeddings, 3), lut int64 (num_embeddings, window^3)) of the active blocks, -1 for
+    absent; the content of ash/grid.py:566-617 for any radius."""
+    dev = hashmap.device()
+    window = 2 * radius + 1 if bidirectional else radius + 1
+    lut = torch.empty((num_embeddings, window**3), dtype=torch.int64, device=dev)
+    coords = torch.empty((num_embeddings, 3), dtype=torch.int32, device=dev)
+    _check(_lib.ashb_grid_build_window_lut(
+        hashmap._h, int(radius), int(bool(bidirectional)), lut.data_ptr(), coords.data_ptr(), num_embeddings, None, None,
+        _stream(dev)))
+    return coords, lut
 
 
 def _fused_args(hashmap, embeddings, x, nb_lut):

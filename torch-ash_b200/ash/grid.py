@@ -405,6 +405,9 @@ class SparseDenseGrid(ASHModule):
         """Per-block tables ``(grid_coords (num_embeddings, 3) int32, lut_grid_nb2grid_idx
         (num_embeddings, K) int64)``; rows of inactive blocks and absent neighbours hold -1
         (ash/grid.py:566-617)."""
+        if self.device.type == "cuda" and hasattr(backend, "grid_build_window_lut"):
+            # one table scan in which a warp probes a block's window; no enumeration, no host read
+            return backend.grid_build_window_lut(self.engine.backend, self.num_embeddings, radius, bidirectional)
         coords, indices = self.engine.items()
         offsets, _ = enumerate_neighbor_coord_offsets(self.in_dim, radius, bidirectional, self.device)
         K = offsets.shape[0]

@@ -761,6 +761,37 @@ __global__ void __launch_bounds__(256) build_nb_lut_kernel(Table16 t, int32_t* _
     }
 }
 
+// The same for any block window [lo, hi]^3 of w = hi - lo + 1 offsets per axis (x fastest), as the int64
+// table of ash/grid.py:566-617.  A warp reads 32 slots; for each live one its lanes share out the w^3
+// neighbours, so the probes of a block run side by side (one lane after the other they were the kernel's
+// whole time) and its row leaves as one coalesced store.  With `list` the live rows are appended to it.
+__global__ void __launch_bounds__(256) build_window_lut_kernel(Table16 t, int lo, int w, int64_t* __restrict__ lut,
+                                                               int32_t* __restrict__ coords, int64_t n_emb,
+                                                               int32_t* __restrict__ list, int32_t* list_count) {
+    const int lane = threadIdx.x & 31, n_nb = w * w * w;
+    const uint64_t n_slots = (uint64_t)t.mask + 1;   // a power of two >= 32
+    const uint64_t warps = (uint64_t)gridDim.x * (blockDim.x >> 5);
+    for (uint64_t s0 = ((uint64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * 32; s0 < n_slots; s0 += warps * 32) {
+        const Entry e = t.read_const((uint32_t)s0 + lane);
+        const bool mine = e.val >= 0 && e.val < n_emb;
+        unsigned live = __ballot_sync(0xffffffffu, mine);
+        if (list && live) {
+            int at = 0;
+            if (lane == 0) at = atomicAdd(list_count, __popc(live));
+            at = __shfl_sync(0xffffffffu, at, 0);
+            if (mine) list[at + __popc(live & lanemask_lt())] = e.val;
+        }
+        for (; live; live &= live - 1) {
+            const int from = __ffs(live) - 1;
+            const int k0 = __shfl_sync(0xffffffffu, e.k0, from), k1 = __shfl_sync(0xffffffffu, e.k1, from),
+                      k2 = __shfl_sync(0xffffffffu, e.k2, from), row = __shfl_sync(0xffffffffu, e.val, from);
+            for (int k = lane; k < n_nb; k += 32)
+                lut[(int64_t)row * n_nb + k] = lookup(t, k0 + lo + k % w, k1 + lo + k / w % w, k2 + lo + k / (w * w), 0);
+            if (coords && lane < 3) coords[3 * (int64_t)row + lane] = lane == 0 ? k0 : (lane == 1 ? k1 : k2);
+        }
+    }
+}
+
 static int make_fused_source(ashb_map* m, const float* x, double cell_size, const float* origin, int G,
                              const int32_t* nb_lut, const int32_t* gi_in, int32_t* gi_out, uint8_t* mask_out,
                              int64_t n_emb, FusedSource* out) {
@@ -868,6 +899,24 @@ int ashb_grid_build_neighbor_lut(ashb_map* m, int32_t* lut, int32_t* grid_coords
     if (grid_coords) ASHB_CUDA_TRY(cudaMemsetAsync(grid_coords, 0xFF, (size_t)n_emb * 3 * sizeof(int32_t), st));
     build_nb_lut_kernel<<<wave_grid((int64_t)m->n_slots, 256, 8), 256, 0, st>>>(table16_of(m), lut, grid_coords,
                                                                                  n_emb);
+    ASHB_LAUNCH_CHECK();
+    return ASHB_OK;
+}
+
+int ashb_grid_build_window_lut(ashb_map* m, int radius, int bidirectional, int64_t* lut, int32_t* grid_coords,
+                               int64_t n_emb, int32_t* list, int32_t* list_count, void* stream) {
+    ASHB_REQUIRE(m != nullptr && m->slots != nullptr, "null or destroyed map");
+    ASHB_REQUIRE(m->key_dim == 3 && lut != nullptr && n_emb >= 1, "needs a 3-D map and an output table");
+    ASHB_REQUIRE(radius >= 0 && radius <= 64, "window radius %d not in 0..64", radius);
+    ASHB_REQUIRE((list == nullptr) == (list_count == nullptr), "pass both the list and its counter, or neither");
+    DeviceGuard guard(m->device);
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    const int lo = bidirectional ? -radius : 0, w = radius - lo + 1;
+    ASHB_CUDA_TRY(cudaMemsetAsync(lut, 0xFF, (size_t)n_emb * w * w * w * sizeof(int64_t), st));
+    if (grid_coords) ASHB_CUDA_TRY(cudaMemsetAsync(grid_coords, 0xFF, (size_t)n_emb * 3 * sizeof(int32_t), st));
+    if (list) ASHB_CUDA_TRY(cudaMemsetAsync(list_count, 0, sizeof(int32_t), st));
+    build_window_lut_kernel<<<wave_grid((int64_t)m->n_slots, 256, 8), 256, 0, st>>>(table16_of(m), lo, w, lut, grid_coords,
+                                                                                     n_emb, list, list_count);
     ASHB_LAUNCH_CHECK();
     return ASHB_OK;
 }
