@@ -300,6 +300,14 @@ int ashb_conv_forward_separable(const float* inputs, const float* weights_1d, co
                                 const int64_t* lut_grid_nb27, float* outputs, int zero_output, int64_t num_grids,
                                 int64_t n_emb, int G, int radius, int64_t D, void* stream);
 
+/* The same filter applied in place to every active block of a table values [n_emb][G^3][D]: rows of
+ * inactive indices become zero.  list / list_count and lut_grid_nb27 as ashb_grid_build_window_lut
+ * (radius 1, two-sided) leaves them; scratch is shaped like values, its contents are undefined
+ * afterwards.  Nothing is read back to the host. */
+int ashb_filter_separable_inplace(float* values, float* scratch, const float* weights_1d, const int32_t* list,
+                                  const int32_t* list_count, const int64_t* lut_grid_nb27, int64_t n_emb, int G,
+                                  int radius, int64_t D, void* stream);
+
 /* ---------------------------------------------------------------- iso-surface vertices */
 
 /* Replaces isosurface_extraction_kernel + isosurface_extraction (ash/src/grid.cu:453-604),

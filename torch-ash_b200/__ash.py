@@ -73,6 +73,7 @@ _lib.ashb_grid_query_backward_backward.argtypes = [_vp, _int, _int, _vp, _vp, _v
                                                    _vp, _int, _i64, _i64, _i64, _vp]
 _lib.ashb_conv_forward_tiled.argtypes = [_vp, _vp, _vp, _vp, _vp, _int, _i64, _i64, _int, _int, _i64, _vp]
 _lib.ashb_conv_forward_separable.argtypes = [_vp, _vp, _vp, _vp, _vp, _int, _i64, _i64, _int, _int, _i64, _vp]
+_lib.ashb_filter_separable_inplace.argtypes = [_vp] * 6 + [_i64, _int, _int, _i64, _vp]
 _lib.ashb_grid_spatial_init.argtypes = [_vp, _vp, _i64, _c.c_double, _vp, _int, _int, _int, _vp, _vp, _vp, _vp, _c.c_uint32,
                                         _vp, _vp, _vp]
 _lib.ashb_route_by_owner.argtypes = [_vp, _i64, _int, _int, _vp, _vp, _vp, _vp, _vp]
@@ -878,6 +879,26 @@ def convolution_forward_separable(inputs, weights_1d, grid_indices, lut_grid_nb2
             inp.data_ptr(), w.data_ptr(), gi.data_ptr(), g27.data_ptr(), out.data_ptr(), 1, gi.shape[0], n_emb,
             int(grid_dim), int(radius), D, _stream(inp.device)))
     return out
+
+
+def filter_separable_(values, weights_1d, hashmap, grid_dim, radius):
+    """``values`` (num_embeddings, G^3, D) float32, filtered in place over the active blocks of ``hashmap`` with the x, y and
+    z factors ``weights_1d`` (3, 2R+1, D); rows of inactive indices become zero.  No host synchronisation."""
+    v = _cuda(values, "values", torch.float32)
+    w = _cuda(weights_1d, "weights_1d", torch.float32)
+    n_emb, cells, D = v.shape
+    if v.data_ptr() != values.data_ptr() or cells != int(grid_dim) ** 3 or w.shape != (3, 2 * int(radius) + 1, D):
+        raise RuntimeError("filter_separable_: values must be contiguous and shaped for (grid_dim, radius)")
+    dev = v.device
+    scratch = torch.empty_like(v)
+    lut = torch.empty((n_emb, 27), dtype=torch.int64, device=dev)
+    rows = torch.empty(n_emb + 1, dtype=torch.int32, device=dev)
+    count = rows[n_emb:]
+    st = _stream(dev)
+    with torch.cuda.device(dev):
+        _check(_lib.ashb_grid_build_window_lut(hashmap._h, 1, 1, lut.data_ptr(), None, n_emb, rows.data_ptr(), count.data_ptr(), st))
+        _check(_lib.ashb_filter_separable_inplace(v.data_ptr(), scratch.data_ptr(), w.data_ptr(), rows.data_ptr(), count.data_ptr(),
+                                                  lut.data_ptr(), n_emb, int(grid_dim), int(radius), D, st))
 
 
 def grid_spatial_init(hashmap, points, cell_size, origin, grid_dim, dilation, bidirectional, grid_coords, touched,

@@ -343,13 +343,11 @@ class SparseDenseGrid(ASHModule):
         radius = size // 2
         emb = self.embeddings
         if (self.separable_gaussian and self.tiled_convolution and emb.is_cuda and emb.dtype == torch.float32
-                and 1 <= radius <= self.grid_dim and hasattr(backend, "convolution_forward_separable")):
+                and 1 <= radius <= self.grid_dim and hasattr(backend, "filter_separable_")):
             k1 = self._gaussian_weights_1d(size, sigma)
             k1 = k1 / k1.sum()                       # (k1 (x) k1 (x) k1) / sum = product of the normalised factors
-            w1 = torch.from_numpy(k1).float().view(1, size, 1).repeat(3, 1, channels).contiguous().to(emb.device)
-            _, lut_g2g = self.construct_grid_neighbor_lut(1, bidirectional=True)
-            _, _, grid_indices, _ = self.items()
-            emb.copy_(backend.convolution_forward_separable(emb.data, w1, grid_indices, lut_g2g, self.grid_dim, radius))
+            w1 = torch.from_numpy(k1).float().view(1, size, 1).repeat(3, 1, channels).contiguous()
+            backend.filter_separable_(emb.data, w1.to(emb.device), self.engine.backend, self.grid_dim, radius)
             return
         weights = self._gaussian_weights(size, sigma).view(size, size, size, 1).repeat(1, 1, 1, channels)
         self.embeddings.copy_(self.convolution(self.embeddings, weights.to(self.embeddings.device)))

@@ -165,6 +165,14 @@ __global__ void __launch_bounds__(256) conv_tiled_kernel(const float* __restrict
     }
 }
 
+// The blocks to filter: `grid_indices` with one CTA each, or the first *count rows of `list`, which the CTAs
+// that are resident at once share out.
+struct FilterBlocks {
+    const int64_t* __restrict__ grid_indices;
+    const int32_t* __restrict__ list;
+    const int32_t* __restrict__ count;
+};
+
 // Separable window: weights[z][y][x][c] = wz[z][c] * wy[y][c] * wx[x][c] (a Gaussian is one).  The
 // same halo tile is staged, then three 1-D passes run inside shared memory -- along x over the
 // whole (G+2R)^2 cross-section, along y over the (G+2R) slabs that remain, along z -- so a
@@ -173,7 +181,7 @@ __global__ void __launch_bounds__(256) conv_tiled_kernel(const float* __restrict
 // exactly as in the full window).  w1: [3][S][D], axis 0 = x.
 template <int CH>
 __global__ void __launch_bounds__(256) conv_separable_kernel(const float* __restrict__ in, const float* __restrict__ w1,
-                                                             const int64_t* __restrict__ grid_indices,
+                                                             FilterBlocks blocks,
                                                              const int64_t* __restrict__ g2g27, float* __restrict__ out,
                                                              int G, int R, int D, int64_t n_emb) {
     extern __shared__ float smem[];
@@ -183,7 +191,8 @@ __global__ void __launch_bounds__(256) conv_separable_kernel(const float* __rest
     float* t1 = smem + (size_t)tile_cells * CH;           // x-pass sums [T][T][G][CH]
     float* wsm = t1 + (size_t)T * T * G * CH;             // [3][S][CH]
     __shared__ int64_t nb[27];
-    const int64_t gidx = grid_indices[blockIdx.x];
+    if (blocks.list && (int)blockIdx.x >= *blocks.count) return;
+    const int64_t gidx = blocks.list ? blocks.list[blockIdx.x] : blocks.grid_indices[blockIdx.x];
     const bool ok = gidx >= 0 && gidx < n_emb;
     if (threadIdx.x < 27) nb[threadIdx.x] = ok ? g2g27[gidx * 27 + threadIdx.x] : -1;
     __syncthreads();
@@ -300,8 +309,7 @@ __device__ __forceinline__ void filter_line(const float* line, const float* w, S
 
 template <int CH, int G, int R>
 __global__ void __launch_bounds__(256) conv_separable_lines_kernel(const float* __restrict__ in,
-                                                                   const float* __restrict__ w1,
-                                                                   const int64_t* __restrict__ grid_indices,
+                                                                   const float* __restrict__ w1, FilterBlocks blocks,
                                                                    const int64_t* __restrict__ g2g27,
                                                                    float* __restrict__ out, int D, int64_t n_emb) {
     constexpr int S = 2 * R + 1, T = G + 2 * R, ROW = (T + 1) * CH, SLAB = T * ROW, CELLS = G * G * G;
@@ -309,65 +317,84 @@ __global__ void __launch_bounds__(256) conv_separable_lines_kernel(const float* 
     extern __shared__ __align__(16) float tile[];   // [T][T][T + 1][CH]
     __shared__ float wsm[3 * S * CH];
     __shared__ const float* nb[27];
-    const int64_t gidx = grid_indices[blockIdx.x];
-    const bool ok = gidx >= 0 && gidx < n_emb;
-    if (threadIdx.x < 27) {
-        const int64_t g = ok ? g2g27[gidx * 27 + threadIdx.x] : -1;
-        nb[threadIdx.x] = g >= 0 && g < n_emb ? in + g * CELLS * D : nullptr;
+    const int n_items = blocks.list ? *blocks.count : (int)gridDim.x;
+    for (int item = blockIdx.x; item < n_items; item += gridDim.x) {
+        const int64_t gidx = blocks.list ? blocks.list[item] : blocks.grid_indices[item];
+        if (gidx < 0 || gidx >= n_emb) continue;
+        if (threadIdx.x < 27) {
+            const int64_t g = g2g27[gidx * 27 + threadIdx.x];
+            nb[threadIdx.x] = g >= 0 && g < n_emb ? in + g * CELLS * D : nullptr;
+        }
+        __syncthreads();
+        for (int ch0 = 0; ch0 < D; ch0 += CH) {
+            // a thread keeps its (x, y) of the tile and walks the slabs: the three blocks it reads are three pointers
+            for (int hy = threadIdx.x / WIDE; hy < T; hy += blockDim.x / WIDE) {
+                const int hx = threadIdx.x % WIDE;
+                if (hx >= T) break;
+                const int bx = (hx >= R) + (hx >= G + R), by = (hy >= R) + (hy >= G + R);
+                const int xy = (hx + G - R) % G + (hy + G - R) % G * G;
+                const float* from[3];
+                bool present[3];
+#pragma unroll
+                for (int bz = 0; bz < 3; ++bz) {
+                    const float* block = nb[bx + by * 3 + bz * 9];
+                    present[bz] = block != nullptr;
+                    from[bz] = (present[bz] ? block : in) + xy * D + ch0;
+                }
+                float* to = tile + hy * ROW + hx * CH;
+#pragma unroll
+                for (int hz = 0; hz < T; ++hz) {
+                    const int bz = (hz >= R) + (hz >= G + R);
+                    copy_async<CH * 4>(to + hz * SLAB, from[bz] + (hz + G - R) % G * (G * G) * D, present[bz]);
+                }
+            }
+            for (int k = threadIdx.x; k < 3 * S * CH; k += blockDim.x) wsm[k] = w1[(int64_t)(k / CH) * D + ch0 + (k % CH)];
+            asm volatile("cp.async.wait_all;" ::: "memory");
+            __syncthreads();
+            // the block size is a multiple of CH: a thread stays with one channel and its weights
+            const int c = threadIdx.x % CH;
+            float w[S];
+#pragma unroll
+            for (int k = 0; k < S; ++k) w[k] = wsm[k * CH + c];
+            for (int i = threadIdx.x; i < T * T * CH; i += blockDim.x) {   // rows, along x
+                float* line = tile + (i / CH) * ROW + c;
+                filter_line<G, S, CH>(line, w, [&](int o, float v) { line[o * CH] = v; });
+            }
+#pragma unroll
+            for (int k = 0; k < S; ++k) w[k] = wsm[(S + k) * CH + c];
+            __syncthreads();
+            for (int i = threadIdx.x; i < T * G * CH; i += blockDim.x) {   // columns, along y
+                float* line = tile + (i / (G * CH)) * SLAB + i % (G * CH);
+                filter_line<G, S, ROW>(line, w, [&](int o, float v) { line[o * ROW] = v; });
+            }
+#pragma unroll
+            for (int k = 0; k < S; ++k) w[k] = wsm[(2 * S + k) * CH + c];
+            __syncthreads();
+            for (int i = threadIdx.x; i < G * G * CH; i += blockDim.x) {   // pillars, along z
+                const int xy = i / CH;
+                const float* line = tile + (xy / G) * ROW + i % (G * CH);
+                float* dst = out + (gidx * CELLS + xy) * D + ch0 + c;
+                filter_line<G, S, SLAB>(line, w, [&](int o, float v) { dst[(int64_t)o * G * G * D] = v; });
+            }
+            __syncthreads();
+        }
     }
-    __syncthreads();
-    if (!ok) return;
-    for (int ch0 = 0; ch0 < D; ch0 += CH) {
-        // a thread keeps its (x, y) of the tile and walks the slabs: the three blocks it reads are three pointers
-        for (int hy = threadIdx.x / WIDE; hy < T; hy += blockDim.x / WIDE) {
-            const int hx = threadIdx.x % WIDE;
-            if (hx >= T) break;
-            const int bx = (hx >= R) + (hx >= G + R), by = (hy >= R) + (hy >= G + R);
-            const int xy = (hx + G - R) % G + (hy + G - R) % G * G;
-            const float* from[3];
-            bool present[3];
-#pragma unroll
-            for (int bz = 0; bz < 3; ++bz) {
-                const float* block = nb[bx + by * 3 + bz * 9];
-                present[bz] = block != nullptr;
-                from[bz] = (present[bz] ? block : in) + xy * D + ch0;
-            }
-            float* to = tile + hy * ROW + hx * CH;
-#pragma unroll
-            for (int hz = 0; hz < T; ++hz) {
-                const int bz = (hz >= R) + (hz >= G + R);
-                copy_async<CH * 4>(to + hz * SLAB, from[bz] + (hz + G - R) % G * (G * G) * D, present[bz]);
-            }
+}
+
+// values[row] = filtered[row] for the active rows (whose own entry of the block table is the row itself), zero for
+// the others: the second half of an in-place filter.  `vec` 16-byte words (or floats) a row.
+template <typename V>
+__global__ void __launch_bounds__(256) restore_rows_kernel(V* __restrict__ values, const V* __restrict__ filtered,
+                                                           const int64_t* __restrict__ g2g27, int64_t n_emb, int vec) {
+    for (int64_t row = blockIdx.x; row < n_emb; row += gridDim.x) {
+        const bool active = g2g27[row * 27 + 13] == row;
+        V* to = values + row * vec;
+        const V* from = filtered + row * vec;
+        if (active) {
+            for (int i = threadIdx.x; i < vec; i += blockDim.x) to[i] = __ldcs(from + i);
+        } else {
+            for (int i = threadIdx.x; i < vec; i += blockDim.x) to[i] = V{};
         }
-        for (int k = threadIdx.x; k < 3 * S * CH; k += blockDim.x) wsm[k] = w1[(int64_t)(k / CH) * D + ch0 + (k % CH)];
-        asm volatile("cp.async.wait_all;" ::: "memory");
-        __syncthreads();
-        // the block size is a multiple of CH: a thread stays with one channel and its weights
-        const int c = threadIdx.x % CH;
-        float w[S];
-#pragma unroll
-        for (int k = 0; k < S; ++k) w[k] = wsm[k * CH + c];
-        for (int i = threadIdx.x; i < T * T * CH; i += blockDim.x) {   // rows, along x
-            float* line = tile + (i / CH) * ROW + c;
-            filter_line<G, S, CH>(line, w, [&](int o, float v) { line[o * CH] = v; });
-        }
-#pragma unroll
-        for (int k = 0; k < S; ++k) w[k] = wsm[(S + k) * CH + c];
-        __syncthreads();
-        for (int i = threadIdx.x; i < T * G * CH; i += blockDim.x) {   // columns, along y
-            float* line = tile + (i / (G * CH)) * SLAB + i % (G * CH);
-            filter_line<G, S, ROW>(line, w, [&](int o, float v) { line[o * ROW] = v; });
-        }
-#pragma unroll
-        for (int k = 0; k < S; ++k) w[k] = wsm[(2 * S + k) * CH + c];
-        __syncthreads();
-        for (int i = threadIdx.x; i < G * G * CH; i += blockDim.x) {   // pillars, along z
-            const int xy = i / CH;
-            const float* line = tile + (xy / G) * ROW + i % (G * CH);
-            float* dst = out + (gidx * CELLS + xy) * D + ch0 + c;
-            filter_line<G, S, SLAB>(line, w, [&](int o, float v) { dst[(int64_t)o * G * G * D] = v; });
-        }
-        __syncthreads();
     }
 }
 
@@ -460,30 +487,31 @@ int ashb_conv_forward_tiled(const float* inputs, const float* weights, const int
     return ASHB_OK;
 }
 
-int ashb_conv_forward_separable(const float* inputs, const float* weights_1d, const int64_t* grid_indices,
-                                const int64_t* lut_grid_nb27, float* outputs, int zero_output, int64_t num_grids,
-                                int64_t n_emb, int G, int radius, int64_t D, void* stream) {
-    ASHB_REQUIRE(D >= 1 && D <= 16, "embedding_dim %lld not in 1..16", (long long)D);
-    ASHB_REQUIRE(G >= 1 && G <= 16 && radius >= 1 && radius <= G, "window radius %d must be within one block (G=%d)",
-                 radius, G);
-    ASHB_REQUIRE(num_grids >= 0 && n_emb >= 1 && outputs != nullptr, "bad sizes");
-    cudaStream_t st = static_cast<cudaStream_t>(stream);
-    const int64_t cells = (int64_t)G * G * G;
-    if (zero_output) ASHB_CUDA_TRY(cudaMemsetAsync(outputs, 0, (size_t)n_emb * cells * D * sizeof(float), st));
-    if (num_grids == 0) return ASHB_OK;
-    ASHB_REQUIRE(inputs && weights_1d && grid_indices && lut_grid_nb27, "null buffer");
+}  // extern "C"
+
+// Filter the blocks of `grid_indices` (num_grids of them) or of `list` (at most n_emb, counted on the device).
+static int separable_impl(const float* inputs, const float* weights_1d, const int64_t* grid_indices, const int32_t* list,
+                          const int32_t* list_count, const int64_t* lut_grid_nb27, float* outputs, int64_t num_grids,
+                          int64_t n_emb, int G, int radius, int64_t D, cudaStream_t st) {
     const uintptr_t bits = (uintptr_t)inputs | (uintptr_t)outputs;
     const int ch = D % 4 == 0 && (bits & 15) == 0 ? 4 : (D % 2 == 0 && (bits & 7) == 0 ? 2 : 1);
     const int T = G + 2 * radius, S = 2 * radius + 1;
+    const FilterBlocks blocks{grid_indices, list, list_count};
 #define ASHB_SEP_LINES(CH, GG, RR)                                                                                      \
     if (ch == CH && G == GG && radius == RR) {                                                                          \
-        constexpr int TT = GG + 2 * RR;                                                                                 \
+        constexpr int TT = GG + 2 * RR, threads = GG == 4 ? 128 : 256;                                                  \
         constexpr size_t bytes = (size_t)TT * TT * (TT + 1) * CH * sizeof(float);                                       \
+        const auto fn = conv_separable_lines_kernel<CH, GG, RR>;                                                        \
         if (bytes > 48 * 1024)                                                                                          \
-            ASHB_CUDA_TRY(cudaFuncSetAttribute(conv_separable_lines_kernel<CH, GG, RR>,                                 \
-                                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));               \
-        conv_separable_lines_kernel<CH, GG, RR><<<(unsigned)num_grids, GG == 4 ? 128 : 256, bytes, st>>>(               \
-                inputs, weights_1d, grid_indices, lut_grid_nb27, outputs, (int)D, n_emb);                               \
+            ASHB_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));           \
+        int64_t ctas = num_grids;                                                                                       \
+        if (list) {                                                                                                     \
+            int per_sm = 0;                                                                                             \
+            ASHB_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, bytes));                  \
+            const int64_t resident = (int64_t)sm_count() * (per_sm > 0 ? per_sm : 1);                                   \
+            ctas = n_emb < resident ? n_emb : resident;                                                                 \
+        }                                                                                                               \
+        fn<<<(unsigned)ctas, threads, bytes, st>>>(inputs, weights_1d, blocks, lut_grid_nb27, outputs, (int)D, n_emb);  \
         ASHB_LAUNCH_CHECK();                                                                                            \
         return ASHB_OK;                                                                                                 \
     }
@@ -497,19 +525,61 @@ int ashb_conv_forward_separable(const float* inputs, const float* weights_1d, co
 #undef ASHB_SEP_LINES
     const size_t smem = ((size_t)T * T * T + (size_t)T * T * G + (size_t)3 * S) * ch * sizeof(float);
     ASHB_REQUIRE(smem <= 200 * 1024, "halo tile of %zu bytes does not fit in shared memory", smem);
+    const unsigned ctas = (unsigned)(list ? n_emb : num_grids);
 #define ASHB_SEP_LAUNCH(CH)                                                                                   \
     {                                                                                                         \
         if (smem > 48 * 1024)                                                                                 \
             ASHB_CUDA_TRY(cudaFuncSetAttribute(conv_separable_kernel<CH>,                                     \
                                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));     \
-        conv_separable_kernel<CH><<<(unsigned)num_grids, 256, smem, st>>>(inputs, weights_1d, grid_indices,   \
-                                                                           lut_grid_nb27, outputs, G, radius, \
-                                                                           (int)D, n_emb);                    \
+        conv_separable_kernel<CH><<<ctas, 256, smem, st>>>(inputs, weights_1d, blocks, lut_grid_nb27, outputs, \
+                                                            G, radius, (int)D, n_emb);                        \
     }
     if (ch == 4) ASHB_SEP_LAUNCH(4)
     else if (ch == 2) ASHB_SEP_LAUNCH(2)
     else ASHB_SEP_LAUNCH(1)
 #undef ASHB_SEP_LAUNCH
+    ASHB_LAUNCH_CHECK();
+    return ASHB_OK;
+}
+
+extern "C" {
+
+int ashb_conv_forward_separable(const float* inputs, const float* weights_1d, const int64_t* grid_indices,
+                                const int64_t* lut_grid_nb27, float* outputs, int zero_output, int64_t num_grids,
+                                int64_t n_emb, int G, int radius, int64_t D, void* stream) {
+    ASHB_REQUIRE(D >= 1 && D <= 16, "embedding_dim %lld not in 1..16", (long long)D);
+    ASHB_REQUIRE(G >= 1 && G <= 16 && radius >= 1 && radius <= G, "window radius %d must be within one block (G=%d)",
+                 radius, G);
+    ASHB_REQUIRE(num_grids >= 0 && n_emb >= 1 && outputs != nullptr, "bad sizes");
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    const int64_t cells = (int64_t)G * G * G;
+    if (zero_output) ASHB_CUDA_TRY(cudaMemsetAsync(outputs, 0, (size_t)n_emb * cells * D * sizeof(float), st));
+    if (num_grids == 0) return ASHB_OK;
+    ASHB_REQUIRE(inputs && weights_1d && grid_indices && lut_grid_nb27, "null buffer");
+    return separable_impl(inputs, weights_1d, grid_indices, nullptr, nullptr, lut_grid_nb27, outputs, num_grids, n_emb, G,
+                          radius, D, st);
+}
+
+int ashb_filter_separable_inplace(float* values, float* scratch, const float* weights_1d, const int32_t* list,
+                                  const int32_t* list_count, const int64_t* lut_grid_nb27, int64_t n_emb, int G,
+                                  int radius, int64_t D, void* stream) {
+    ASHB_REQUIRE(D >= 1 && D <= 16, "embedding_dim %lld not in 1..16", (long long)D);
+    ASHB_REQUIRE(G >= 1 && G <= 16 && radius >= 1 && radius <= G, "window radius %d must be within one block (G=%d)",
+                 radius, G);
+    ASHB_REQUIRE(n_emb >= 1 && n_emb <= 0x7fffffffll, "bad sizes");
+    ASHB_REQUIRE(values && scratch && weights_1d && list && list_count && lut_grid_nb27, "null buffer");
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    if (int rc = separable_impl(values, weights_1d, nullptr, list, list_count, lut_grid_nb27, scratch, 0, n_emb, G, radius, D,
+                                st))
+        return rc;
+    const int64_t row = (int64_t)G * G * G * D;
+    const unsigned ctas = (unsigned)(n_emb < sm_count() * 8ll ? n_emb : sm_count() * 8ll);
+    if (row % 4 == 0 && (((uintptr_t)values | (uintptr_t)scratch) & 15) == 0)
+        restore_rows_kernel<float4><<<ctas, 256, 0, st>>>(reinterpret_cast<float4*>(values),
+                                                          reinterpret_cast<const float4*>(scratch), lut_grid_nb27, n_emb,
+                                                          (int)(row / 4));
+    else
+        restore_rows_kernel<float><<<ctas, 256, 0, st>>>(values, scratch, lut_grid_nb27, n_emb, (int)row);
     ASHB_LAUNCH_CHECK();
     return ASHB_OK;
 }
