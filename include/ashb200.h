@@ -332,7 +332,7 @@ int ashb_isosurface_extraction(const float* sdfs, const float* weights, const in
  * weight_thr; corner c is inside when sdf - iso_value < 0.
  *   _count classifies every cube into codes uint8 [num_grids * cells_per_grid], requests the
  *          vertices of cut edges in edge_vertex int32 [n_emb * cells_per_grid * 3] (both are
- *          caller-allocated scratch, passed on to _fill) and returns the number of distinct
+ *          caller-allocated scratch without a meaning of their own, passed on to _fill) and returns the number of distinct
  *          vertices and of triangles (HOST).  Synchronises `stream`.
  *   _fill  writes vertices float32 [n_vertices][3] (cell units, the reference's interpolation)
  *          and triangles int32 [n_triangles][3] (vertex ids).  No host synchronisation.

@@ -1068,7 +1068,7 @@ def marching_cubes(sdfs, weights, grid_indices, grid_coords_table, lut_grid_nb2g
     if gct.shape != (n_emb, 3) or cct.shape != (cells, 3) or c2c.shape != (cells, 8) or c2g.shape != (cells, 8):
         raise RuntimeError("marching_cubes: table shapes do not match sdfs")
     codes = torch.empty(max(gi.shape[0] * cells, 1), dtype=torch.uint8, device=dev)
-    edge_vertex = torch.empty(n_emb * cells * 3, dtype=torch.int32, device=dev)
+    edge_vertex = torch.empty(n_emb * cells * 3, dtype=torch.int32, device=dev)   # scratch, five of its twelve bytes a cell used
     counters = torch.empty(2, dtype=torch.int64, device=dev)
     nv, nt = _i64(), _i64()
     with torch.cuda.device(dev):

@@ -6,18 +6,24 @@
 // cube gets one vertex, owned by the cell at the edge's lower corner, placed by linear
 // interpolation; triangles index those vertices.
 //
-//   classify   per cell: corner pattern -> codes[]; each cut edge is requested at its owner with an
-//              atomic exchange, so the number of distinct vertices is counted in the same pass, as
-//              is the number of triangles (one atomic per warp each)
+//   classify   per tile of blocks: corner pattern -> codes[]; each cut edge is requested at its owner
+//              as one bit of a byte per cell, so the number of distinct vertices is counted in the
+//              same pass, as is the number of triangles
 //   (host reads the two counts and allocates)
-//   vertices   per cell and direction: requested edges get a slot (one atomic per warp) and a position
-//   triangles  per cell: slots for its triangles (warp scan + one atomic per warp), vertex ids
-//              looked up at the owners
+//   vertices   per 1024 cells: requested edges get consecutive slots and positions
+//   triangles  per 1024 cells: triangles get consecutive slots, vertex ids looked up at the owners
+//
+// All three are bound by memory latency, not bytes: what they shed is work per CELL where only one
+// cell in twelve carries surface.  24,000 blocks of 8^3 on a B200: 444 + 114 + 107 us when every cell
+// read its eight corners through the tables, each warp bumped the shared counters and an edge took
+// four bytes of a 147 MB table that had to be filled, written and read.
 //
 // The triangulation table is this repository's own (mc_tables.h, derived by gen_mc_tables.py):
 // the reference's table is not reproduced, so which diagonal splits an ambiguous pattern, the
 // order of a triangle's corners and the output order are not comparable with the reference;
 // vertex positions are.
+#include <algorithm>
+
 #include "common.cuh"
 
 #define ASHB_MC_TABLE static __device__ const
@@ -25,8 +31,15 @@
 
 namespace ashb {
 
-constexpr int kEdgeUnwanted = (int)0xFEFEFEFE;  // what a byte-wise fill with 0xFE leaves
-constexpr int kEdgeWanted = -1;
+// Scratch of a surface (ashb200.h: edge_vertex): the id of the first vertex of every cell, then one byte
+// per cell -- bits 0..2: the edge along x / y / z leaving the cell is cut by a valid cube; bit 3: its
+// vertices have ids -- and a word that says the cell tables are not the usual ones.
+constexpr uint32_t kHasVertices = 8;
+struct McEdges {
+    int* __restrict__ first_vertex;
+    uint8_t* __restrict__ wanted;
+    uint32_t* __restrict__ odd_tables;
+};
 
 struct McLuts {
     const int64_t* __restrict__ grid_indices;
@@ -34,6 +47,18 @@ struct McLuts {
     const int64_t* __restrict__ c2c;
     const int64_t* __restrict__ c2g;
     int64_t cells, n_emb, len;
+    int shift;  // log2(cells), or -1
+
+    // Position in the block list and cell of the i-th cell of the list.
+    __device__ __forceinline__ void split(int64_t i, int64_t& pos, int64_t& cell) const {
+        if (shift >= 0) {   // a 64-bit division costs more than the rest of an inactive cell
+            pos = i >> shift;
+            cell = i & (cells - 1);
+        } else {
+            pos = i / cells;
+            cell = i - pos * cells;
+        }
+    }
 };
 
 // Flat (embedding row * cells + cell) address of corner c of the cube at (grid_idx, cell_idx), or -1.
@@ -50,82 +75,253 @@ __device__ __forceinline__ int edge_lower_corner(int e) {
     return ((j & 1) << ((d + 1) % 3)) | ((j >> 1) << ((d + 2) % 3));
 }
 
-__global__ void __launch_bounds__(256) mc_classify_kernel(const float* __restrict__ sdfs,
-                                                          const float* __restrict__ weights, McLuts L,
-                                                          uint8_t* __restrict__ codes, int* __restrict__ edge_vertex,
-                                                          unsigned long long* __restrict__ counters, float iso_value,
-                                                          float weight_thr) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    int code = 0;
-    int64_t corner[8];
-    if (i < L.len) {
-        const int64_t grid_idx = L.grid_indices[i / L.cells];
-        const int64_t cell_idx = i % L.cells;
-        bool valid = grid_idx >= 0 && grid_idx < L.n_emb;
-#pragma unroll
-        for (int c = 0; c < 8; ++c) {
-            corner[c] = valid ? corner_address(L, grid_idx, cell_idx, c) : -1;
-            valid = valid && corner[c] >= 0;
-        }
-        if (valid) {
-#pragma unroll
-            for (int c = 0; c < 8; ++c) {
-                valid = valid && weights[corner[c]] >= weight_thr;
-                code |= (int)((sdfs[corner[c]] - iso_value) < 0.f) << c;
-            }
-        }
-        if (!valid || code == 255) code = 0;
-        codes[i] = (uint8_t)code;
-    }
-    int new_vertices = 0;
-    if (code) {
-        const int mask = kMcEdgeMask[code];
-#pragma unroll
-        for (int e = 0; e < 12; ++e) {
-            if (!(mask & (1 << e))) continue;
-            const int old = atomicExch(edge_vertex + corner[edge_lower_corner(e)] * 3 + (e >> 2), kEdgeWanted);
-            new_vertices += old == kEdgeUnwanted;
-        }
-    }
-    const int v = __reduce_add_sync(0xffffffffu, new_vertices);
-    const int t = __reduce_add_sync(0xffffffffu, code ? (int)kMcTriCount[code] : 0);
-    if ((threadIdx.x & 31) == 0) {
-        if (v) atomicAdd(counters, (unsigned long long)v);
-        if (t) atomicAdd(counters + 1, (unsigned long long)t);
-    }
+// Requests edges (bits 0..2 of `bits`) of the cell at flat address `a`; returns how many are new.
+__device__ __forceinline__ int request_edges(uint8_t* wanted, int64_t a, uint32_t bits) {
+    const int at = (int)(a & 3) * 8;
+    const uint32_t old = atomicOr(reinterpret_cast<uint32_t*>(wanted + (a - (a & 3))), bits << at);
+    return __popc(bits & ~(old >> at));
 }
 
+// Raises odd_tables unless corner k of cell (x, y, z) is, in both cell tables, the cell at + k's offsets.
+__global__ void __launch_bounds__(256) mc_check_tables_kernel(McLuts L, McEdges edges, int G) {
+    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= L.cells * 8) return;
+    const int cell = e >> 3;
+    const int x = cell % G + (e & 1), y = cell / G % G + ((e >> 1) & 1), z = cell / (G * G) + ((e >> 2) & 1);
+    const int nb = (x == G) | (y == G) << 1 | (z == G) << 2;
+    const int at = x % G + (y % G + z % G * G) * G;
+    if ((L.c2g[e] & 7) != nb || L.c2c[e] != at) atomicExch(edges.odd_tables, 1u);
+}
+
+constexpr int kMaxTileBlocks = 32;
+constexpr int kMaxFastEdge = 16;
+constexpr int kClassifyCtas = 6;   // per SM: what 40 registers allow
+
+// A CTA walks tiles of max(1, 256 / G^3) blocks.  It stages one state byte per cell of the block AND of the
+// layer that its upper neighbours add, (G + 1)^3 in all, so every value is read once (G = 8: 1.4 loads
+// of sdf and weight per cell instead of 8 of each behind 24 table reads); cubes then read bytes of
+// shared memory.  Requests for the block's own edges meet in shared memory and go out a word at a
+// time; the two counters see one atomic per CTA.  GT: the block edge where it is known when compiling
+// (the halo's divisions), 0 otherwise.  Cell tables that are not the usual ones (odd_tables), and edges
+// beyond kMaxFastEdge (G = 0), take the corners from the tables.
+template <int GT>
+__global__ void __launch_bounds__(256, kClassifyCtas) mc_classify_kernel(const float* __restrict__ sdfs,
+                                                          const float* __restrict__ weights, McLuts L,
+                                                          uint8_t* __restrict__ codes, McEdges edges,
+                                                          unsigned long long* __restrict__ counters, float iso_value,
+                                                          float weight_thr, int G_arg, int64_t num_grids) {
+    __shared__ uint8_t state[(kMaxFastEdge + 1) * (kMaxFastEdge + 1) * (kMaxFastEdge + 1) + 15];
+    __shared__ uint32_t own[kMaxFastEdge * kMaxFastEdge * kMaxFastEdge / 4];
+    __shared__ int64_t rows[kMaxTileBlocks * 8];
+    __shared__ uint16_t edge_mask[256];
+    __shared__ uint8_t tri_count[256];
+    const int tid = threadIdx.x;
+    edge_mask[tid] = kMcEdgeMask[tid];   // launched with 256 threads
+    tri_count[tid] = kMcTriCount[tid];
+    __syncthreads();
+    int n_vertices = 0, n_triangles = 0;
+    const int G = GT ? GT : G_arg;
+    if (G == 0 || *edges.odd_tables != 0) {
+        for (int64_t i = (int64_t)blockIdx.x * 256 + tid; i < L.len; i += (int64_t)gridDim.x * 256) {
+            int64_t pos, cell_idx, corner[8];
+            L.split(i, pos, cell_idx);
+            const int64_t grid_idx = L.grid_indices[pos];
+            bool valid = grid_idx >= 0 && grid_idx < L.n_emb;
+            int code = 0;
+#pragma unroll
+            for (int c = 0; c < 8; ++c) {
+                corner[c] = valid ? corner_address(L, grid_idx, cell_idx, c) : -1;
+                valid = valid && corner[c] >= 0;
+            }
+            if (valid) {
+#pragma unroll
+                for (int c = 0; c < 8; ++c) {
+                    valid = valid && weights[corner[c]] >= weight_thr;
+                    code |= (int)((sdfs[corner[c]] - iso_value) < 0.f) << c;
+                }
+            }
+            if (!valid || code == 255) code = 0;
+            codes[i] = (uint8_t)code;
+            const int mask = edge_mask[code];
+#pragma unroll
+            for (int e = 0; e < 12; ++e)
+                if (mask & (1 << e)) n_vertices += request_edges(edges.wanted, corner[edge_lower_corner(e)], 1u << (e >> 2));
+            n_triangles += tri_count[code];
+        }
+    } else {
+        const int H = G + 1, halo = H * H * H, cells = G * G * G;
+        const int per_tile = cells >= 256 ? 1 : min(256 / cells, kMaxTileBlocks);
+        const int64_t n_tiles = (num_grids + per_tile - 1) / per_tile;
+        for (int64_t tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
+            const int64_t first = tile * per_tile;
+            const int blocks = (int)min((int64_t)per_tile, num_grids - first);
+            if (tid < blocks * 8) {
+                const int64_t g = L.grid_indices[first + (tid >> 3)];
+                const int64_t nb = g >= 0 && g < L.n_emb ? L.g2g[g * 8 + (tid & 7)] : -1;
+                rows[tid] = nb < L.n_emb ? nb : -1;
+            }
+            for (int w = tid; w < (blocks * cells + 3) / 4; w += 256) own[w] = 0;
+            __syncthreads();
+#pragma unroll 3
+            for (int h = tid; h < blocks * halo; h += 256) {
+                const int b = per_tile == 1 ? 0 : h / halo, r = h - b * halo;
+                const int x = r % H, y = r / H % H, z = r / (H * H);
+                const int64_t g = rows[b * 8 + ((x == G) | (y == G) << 1 | (z == G) << 2)];
+                uint8_t s = 0;   // bit 0: observed, bit 1: inside
+                if (g >= 0) {
+                    const int64_t a = g * cells + (x == G ? 0 : x) + ((y == G ? 0 : y) + (z == G ? 0 : z) * G) * G;
+                    const float d = sdfs[a];
+                    s = weights[a] >= weight_thr ? (d - iso_value < 0.f ? 3 : 1) : 0;
+                }
+                state[h] = s;
+            }
+            __syncthreads();
+            for (int c = tid; c < blocks * cells; c += 256) {
+                const int b = per_tile == 1 ? 0 : c / cells, cell = c - b * cells;
+                const int x = cell % G, y = cell / G % G, z = cell / (G * G);
+                const uint8_t* s = state + b * halo + x + (y + z * H) * H;
+                unsigned seen = 1, code = 0;
+#pragma unroll
+                for (int k = 0; k < 8; ++k) {
+                    const unsigned v = s[(k & 1) + (((k >> 1) & 1) + (k >> 2) * H) * H];
+                    seen &= v;
+                    code |= (v >> 1) << k;
+                }
+                if (!seen || code == 255) code = 0;
+                codes[first * cells + c] = (uint8_t)code;
+                if (code == 0) continue;
+                n_triangles += tri_count[code];
+                const int mask = edge_mask[code];
+#pragma unroll
+                for (int k = 0; k < 7; ++k) {   // the edges that leave corner k of the cube
+                    uint32_t bits = 0;
+#pragma unroll
+                    for (int e = 0; e < 12; ++e)
+                        if (edge_lower_corner(e) == k) bits |= (uint32_t)((mask >> e) & 1) << (e >> 2);
+                    if (bits == 0) continue;
+                    const int cx = x + (k & 1), cy = y + ((k >> 1) & 1), cz = z + (k >> 2);
+                    const int nb = (cx == G) | (cy == G) << 1 | (cz == G) << 2;
+                    const int at = (cx == G ? 0 : cx) + ((cy == G ? 0 : cy) + (cz == G ? 0 : cz) * G) * G;
+                    if (nb == 0) {
+                        const int o = b * cells + at;
+                        atomicOr(own + (o >> 2), bits << ((o & 3) * 8));
+                    } else {
+                        n_vertices += request_edges(edges.wanted, rows[b * 8 + nb] * cells + at, bits);
+                    }
+                }
+            }
+            __syncthreads();
+            for (int w = tid; w < (blocks * cells + 3) / 4; w += 256) {
+                const uint32_t bits = own[w];
+                if (bits == 0) continue;
+                if ((cells & 3) == 0) {   // the word is one of the block's
+                    const int b = per_tile == 1 ? 0 : 4 * w / cells;
+                    const int64_t a = rows[b * 8] * cells + (4 * w - b * cells);
+                    n_vertices += __popc(bits & ~atomicOr(reinterpret_cast<uint32_t*>(edges.wanted + a), bits));
+                } else {
+                    for (int j = 0; j < 4; ++j) {
+                        const uint32_t one = (bits >> (8 * j)) & 7u;
+                        const int b = (4 * w + j) / cells;
+                        if (one) n_vertices += request_edges(edges.wanted, rows[b * 8] * cells + (4 * w + j - b * cells), one);
+                    }
+                }
+            }
+            __syncthreads();   // rows and the two tiles are used again
+        }
+    }
+    __shared__ int sums[2];
+    if (tid < 2) sums[tid] = 0;
+    __syncthreads();
+    n_vertices = __reduce_add_sync(0xffffffffu, n_vertices);
+    n_triangles = __reduce_add_sync(0xffffffffu, n_triangles);
+    if ((tid & 31) == 0) {
+        if (n_vertices) atomicAdd(sums, n_vertices);
+        if (n_triangles) atomicAdd(sums + 1, n_triangles);
+    }
+    __syncthreads();
+    if (tid < 2 && sums[tid]) atomicAdd(counters + tid, (unsigned long long)sums[tid]);
+}
+
+constexpr int kPassCells = 1024;   // cells of one CTA of the two passes below: 4 per thread
+
+// Exclusive prefix of `mine` over the CTA of 256 threads, and the start of its range of `cursor`.
+__device__ __forceinline__ int reserve_range(int mine, unsigned long long* cursor, int& total, int64_t& base) {
+    __shared__ int warp_total[8];
+    __shared__ unsigned long long start;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int incl = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int u = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += u;
+    }
+    if (lane == 31) warp_total[warp] = incl;
+    __syncthreads();
+    int before = 0;
+    total = 0;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) {
+        if (w < warp) before += warp_total[w];
+        total += warp_total[w];
+    }
+    if (threadIdx.x == 0 && total) start = atomicAdd(cursor, (unsigned long long)total);
+    __syncthreads();
+    base = total ? (int64_t)start : 0;
+    return before + incl - mine;
+}
+
+// Four cells per thread read their request bytes; the requested edges of the CTA are listed in shared
+// memory and the list is worked off by all threads, so positions are computed without idle lanes
+// and leave as one contiguous run.
 __global__ void __launch_bounds__(256) mc_vertex_kernel(const float* __restrict__ sdfs, McLuts L,
                                                         const int32_t* __restrict__ grid_coords,
-                                                        const int32_t* __restrict__ cell_coords,
-                                                        int* __restrict__ edge_vertex,
+                                                        const int32_t* __restrict__ cell_coords, McEdges edges,
                                                         unsigned long long* __restrict__ cursor,
                                                         float* __restrict__ vertices, int64_t max_vertices,
                                                         float iso_value, int grid_dim) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const bool live = i < L.len;
-    int64_t grid_idx = 0, cell_idx = 0, self = 0;
-    if (live) {
-        grid_idx = L.grid_indices[i / L.cells];
-        cell_idx = i % L.cells;
-        self = grid_idx * L.cells + cell_idx;
-    }
-    const bool in_range = live && grid_idx >= 0 && grid_idx < L.n_emb;
+    __shared__ uint16_t list[3 * kPassCells];
+    const int64_t i0 = (int64_t)blockIdx.x * kPassCells;
+    uint32_t bits[4];
+    int64_t address[4];
+    int mine = 0;
 #pragma unroll
-    for (int d = 0; d < 3; ++d) {
-        const bool emit = in_range && edge_vertex[self * 3 + d] == kEdgeWanted;
-        const unsigned ballot = __ballot_sync(0xffffffffu, emit);
-        if (ballot == 0) continue;
-        const int leader = __ffs(ballot) - 1;
-        unsigned long long base = 0;
-        if ((int)(threadIdx.x & 31) == leader) base = atomicAdd(cursor, (unsigned long long)__popc(ballot));
-        base = __shfl_sync(0xffffffffu, base, leader);
-        if (!emit) continue;
-        const int64_t o = (int64_t)base + __popc(ballot & lanemask_lt());
-        edge_vertex[self * 3 + d] = (int)o;
+    for (int j = 0; j < 4; ++j) {
+        const int64_t i = i0 + 4 * threadIdx.x + j;
+        bits[j] = 0;
+        address[j] = 0;
+        if (i < L.len) {
+            int64_t pos, cell_idx;
+            L.split(i, pos, cell_idx);
+            const int64_t grid_idx = L.grid_indices[pos];
+            if (grid_idx >= 0 && grid_idx < L.n_emb) {
+                address[j] = grid_idx * L.cells + cell_idx;
+                bits[j] = edges.wanted[address[j]] & 7u;
+            }
+        }
+        mine += __popc(bits[j]);
+    }
+    int total;
+    int64_t base;
+    int at = reserve_range(mine, cursor, total, base);
+    if (total == 0) return;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        if (bits[j] == 0) continue;
+        edges.first_vertex[address[j]] = (int)(base + at);
+        edges.wanted[address[j]] = (uint8_t)(bits[j] | kHasVertices);
+#pragma unroll
+        for (int d = 0; d < 3; ++d)
+            if (bits[j] & (1u << d)) list[at++] = (uint16_t)((4 * threadIdx.x + j) * 4 + d);
+    }
+    __syncthreads();
+    for (int e = threadIdx.x; e < total; e += 256) {
+        const int d = list[e] & 3;
+        int64_t pos, cell_idx;
+        L.split(i0 + (list[e] >> 2), pos, cell_idx);
+        const int64_t grid_idx = L.grid_indices[pos], o = base + e;
         const int64_t nb = corner_address(L, grid_idx, cell_idx, 1 << d);
         if (o >= max_vertices || nb < 0) continue;  // cannot happen for edges a valid cube requested
-        const float self_iso = sdfs[self] - iso_value;
+        const float self_iso = sdfs[grid_idx * L.cells + cell_idx] - iso_value;
         const float nb_iso = sdfs[nb] - iso_value;
         const float ratio = self_iso / (self_iso - nb_iso);
 #pragma unroll
@@ -136,44 +332,64 @@ __global__ void __launch_bounds__(256) mc_vertex_kernel(const float* __restrict_
     }
 }
 
-__global__ void __launch_bounds__(256) mc_triangle_kernel(McLuts L, const uint8_t* __restrict__ codes,
-                                                          const int* __restrict__ edge_vertex,
+// The same for triangles: the CTA lists them, then a thread per corner looks its vertex up.
+__global__ void __launch_bounds__(256) mc_triangle_kernel(McLuts L, const uint8_t* __restrict__ codes, McEdges edges,
                                                           unsigned long long* __restrict__ cursor,
                                                           int32_t* __restrict__ triangles, int64_t max_triangles) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const int lane = threadIdx.x & 31;
-    const int code = i < L.len ? codes[i] : 0;
-    const int n = code ? (int)kMcTriCount[code] : 0;
-    // exclusive scan of the triangle counts over the warp, one atomic for the warp's total
-    int incl = n;
+    __shared__ uint16_t list[ASHB_MC_MAX_TRIS * kPassCells];
+    __shared__ uint8_t code_of[kPassCells];
+    const int64_t i0 = (int64_t)blockIdx.x * kPassCells;
+    int count[4];
+    int mine = 0;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int u = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += u;
+    for (int j = 0; j < 4; ++j) {
+        const int64_t i = i0 + 4 * threadIdx.x + j;
+        const int code = i < L.len ? codes[i] : 0;
+        count[j] = code ? (int)kMcTriCount[code] : 0;
+        code_of[4 * threadIdx.x + j] = (uint8_t)code;
+        mine += count[j];
     }
-    const int total = __shfl_sync(0xffffffffu, incl, 31);
+    int total;
+    int64_t base;
+    int at = reserve_range(mine, cursor, total, base);
     if (total == 0) return;
-    unsigned long long base = 0;
-    if (lane == 31) base = atomicAdd(cursor, (unsigned long long)total);
-    base = __shfl_sync(0xffffffffu, base, 31);
-    if (n == 0) return;
-    const int64_t grid_idx = L.grid_indices[i / L.cells];
-    const int64_t cell_idx = i % L.cells;
-    int64_t out = (int64_t)base + (incl - n);
-    for (int t = 0; t < n; ++t, ++out) {
-        if (out >= max_triangles) return;
 #pragma unroll
-        for (int v = 0; v < 3; ++v) {
-            const int e = kMcTris[code][3 * t + v];
-            const int64_t owner = corner_address(L, grid_idx, cell_idx, edge_lower_corner(e));
-            triangles[out * 3 + v] = owner >= 0 ? edge_vertex[owner * 3 + (e >> 2)] : -1;
+    for (int j = 0; j < 4; ++j)
+        for (int t = 0; t < count[j]; ++t) list[at++] = (uint16_t)((4 * threadIdx.x + j) * 8 + t);
+    __syncthreads();
+    for (int m = threadIdx.x; m < 3 * total; m += 256) {
+        const int t = m / 3, v = m - 3 * t;
+        if (base + t >= max_triangles) return;
+        const int local = list[t] >> 3;
+        const int e = kMcTris[code_of[local]][3 * (list[t] & 7) + v];
+        int64_t pos, cell_idx;
+        L.split(i0 + local, pos, cell_idx);
+        const int64_t owner = corner_address(L, L.grid_indices[pos], cell_idx, edge_lower_corner(e));
+        int id = -1;   // the owner's block is not listed
+        if (owner >= 0) {
+            const uint32_t bits = edges.wanted[owner];
+            if (bits & kHasVertices) id = edges.first_vertex[owner] + __popc(bits & ((1u << (e >> 2)) - 1));
         }
+        triangles[base * 3 + m] = id;
     }
 }
 
 }  // namespace ashb
 
 using namespace ashb;
+
+static McLuts mc_luts(const int64_t* grid_indices, const int64_t* g2g, const int64_t* c2c, const int64_t* c2g, int64_t cells,
+                      int64_t n_emb, int64_t num_grids) {
+    int shift = 0;
+    while ((1ll << shift) < cells) ++shift;
+    return McLuts{grid_indices, g2g, c2c, c2g, cells, n_emb, num_grids * cells, (1ll << shift) == cells ? shift : -1};
+}
+
+// Five bytes per cell and the word behind them, in the caller's twelve bytes per cell.
+static McEdges mc_edges(int32_t* scratch, int64_t n) {
+    uint8_t* wanted = reinterpret_cast<uint8_t*>(scratch + n);
+    return McEdges{scratch, wanted, reinterpret_cast<uint32_t*>(wanted + (n + 3) / 4 * 4)};
+}
 
 extern "C" {
 
@@ -193,11 +409,23 @@ int ashb_marching_cubes_count(const float* sdfs, const float* weights, const int
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     unsigned long long* counters = static_cast<unsigned long long*>(counters_dev);
     ASHB_CUDA_TRY(cudaMemsetAsync(counters, 0, 2 * sizeof(unsigned long long), st));
-    ASHB_CUDA_TRY(cudaMemsetAsync(edge_vertex, 0xFE, (size_t)n_emb * cells_per_grid * 3 * sizeof(int32_t), st));
-    const McLuts L{grid_indices, lut_grid_nb2grid_idx, lut_cell_nb2cell_idx, lut_cell_nb2grid_nb,
-                   cells_per_grid, n_emb, num_grids * cells_per_grid};
-    mc_classify_kernel<<<(unsigned)((L.len + 255) / 256), 256, 0, st>>>(sdfs, weights, L, codes, edge_vertex, counters,
-                                                                       iso_value, weight_thr);
+    const int64_t n = n_emb * cells_per_grid;
+    const McEdges edges = mc_edges(edge_vertex, n);
+    ASHB_CUDA_TRY(cudaMemsetAsync(edges.wanted, 0, (size_t)(n + 3) / 4 * 4 + sizeof(uint32_t), st));
+    const McLuts L = mc_luts(grid_indices, lut_grid_nb2grid_idx, lut_cell_nb2cell_idx, lut_cell_nb2grid_nb, cells_per_grid,
+                             n_emb, num_grids);
+    int G = 2;
+    while (G < kMaxFastEdge && (int64_t)G * G * G < cells_per_grid) ++G;
+    if ((int64_t)G * G * G != cells_per_grid) G = 0;
+    if (G) {
+        mc_check_tables_kernel<<<(unsigned)((cells_per_grid * 8 + 255) / 256), 256, 0, st>>>(L, edges, G);
+        ASHB_LAUNCH_CHECK();
+    }
+    // persistent: one resident set of CTAs shares out the tiles (27 each at 24,000 blocks)
+    const unsigned grid = (unsigned)std::min<int64_t>((L.len + 255) / 256, (int64_t)sm_count() * kClassifyCtas);
+    auto kernel = G == 8 ? mc_classify_kernel<8> : G == 4 ? mc_classify_kernel<4> : G == 16 ? mc_classify_kernel<16>
+                                                                                        : mc_classify_kernel<0>;
+    kernel<<<grid, 256, 0, st>>>(sdfs, weights, L, codes, edges, counters, iso_value, weight_thr, G, num_grids);
     ASHB_LAUNCH_CHECK();
     unsigned long long host[2] = {0, 0};
     ASHB_CUDA_TRY(cudaMemcpyAsync(host, counters, sizeof(host), cudaMemcpyDeviceToHost, st));
@@ -223,13 +451,14 @@ int ashb_marching_cubes_fill(const float* sdfs, const int64_t* grid_indices, con
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     unsigned long long* counters = static_cast<unsigned long long*>(counters_dev);
     ASHB_CUDA_TRY(cudaMemsetAsync(counters, 0, 2 * sizeof(unsigned long long), st));
-    const McLuts L{grid_indices, lut_grid_nb2grid_idx, lut_cell_nb2cell_idx, lut_cell_nb2grid_nb,
-                   cells_per_grid, n_emb, num_grids * cells_per_grid};
-    const unsigned grid = (unsigned)((L.len + 255) / 256);
-    mc_vertex_kernel<<<grid, 256, 0, st>>>(sdfs, L, grid_coords_table, cell_coords_table, edge_vertex, counters,
-                                           vertices, n_vertices, iso_value, grid_dim);
+    const McLuts L = mc_luts(grid_indices, lut_grid_nb2grid_idx, lut_cell_nb2cell_idx, lut_cell_nb2grid_nb, cells_per_grid,
+                             n_emb, num_grids);
+    const McEdges edges = mc_edges(edge_vertex, n_emb * cells_per_grid);
+    const unsigned grid = (unsigned)((L.len + kPassCells - 1) / kPassCells);
+    mc_vertex_kernel<<<grid, 256, 0, st>>>(sdfs, L, grid_coords_table, cell_coords_table, edges, counters, vertices,
+                                           n_vertices, iso_value, grid_dim);
     ASHB_LAUNCH_CHECK();
-    mc_triangle_kernel<<<grid, 256, 0, st>>>(L, codes, edge_vertex, counters + 1, triangles, n_triangles);
+    mc_triangle_kernel<<<grid, 256, 0, st>>>(L, codes, edges, counters + 1, triangles, n_triangles);
     ASHB_LAUNCH_CHECK();
     return ASHB_OK;
 }
