@@ -244,6 +244,7 @@ struct IntegrateFrame {
     int G, cells;
     float trunc;
     int sdf_ch, rgb_ch, w_ch;
+    int G_shift;   // log2(G), or -1
 };
 
 // One observation fused into every cell of block (gx, gy, gz), whose rows sit in `tile` (cells * D floats).
@@ -251,7 +252,12 @@ template <int D>
 __device__ __forceinline__ void integrate_cells(float* tile, int gx, int gy, int gz, const IntegrateFrame& f) {
     const int G = f.G;
     for (int c = threadIdx.x; c < f.cells; c += blockDim.x) {
-        const int cx = c % G, cy = (c / G) % G, cz = c / (G * G);
+        int cx, cy, cz;
+        if (f.G_shift >= 0) {   // three divisions would be a quarter of a cell's instructions
+            cx = c & (G - 1), cy = (c >> f.G_shift) & (G - 1), cz = c >> (2 * f.G_shift);
+        } else {
+            cx = c % G, cy = (c / G) % G, cz = c / (G * G);
+        }
         // cell_to_world: (block * G + cell) * cell_size (+ origin for bounded grids)
         const float px = __fadd_rn(__fmul_rn((float)(gx * G + cx), f.cell_size), f.origin.x);
         const float py = __fadd_rn(__fmul_rn((float)(gy * G + cy), f.cell_size), f.origin.y);
@@ -525,7 +531,7 @@ int ashb_tsdf_integrate(void* embeddings, int64_t n_emb, int G, int64_t D, const
     ASHB_REQUIRE(smem <= 200 * 1024, "block of %zu bytes does not fit in shared memory", smem);
     const IntegrateFrame frame{depth, color, H, W, cam, depth_max, (float)cell_size,
                                make_float3(origin[0], origin[1], origin[2]), G, cells, trunc, sdf_channel, rgb_channel,
-                               weight_channel};
+                               weight_channel, (G & (G - 1)) == 0 ? 31 - __builtin_clz((unsigned)G) : -1};
     // The copy-engine variant needs a work list, 16-byte aligned rows of a multiple of 16 bytes, and room
     // for two tiles per CTA; everything else takes the plain kernel.
     const bool bulk = touched_list != nullptr && smem % 16 == 0 && ((uintptr_t)embeddings & 15) == 0 && 2 * smem <= 96 * 1024;
