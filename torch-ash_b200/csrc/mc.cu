@@ -13,10 +13,10 @@
 //   vertices   per 1024 cells: requested edges get consecutive slots and positions
 //   triangles  per 1024 cells: triangles get consecutive slots, vertex ids looked up at the owners
 //
-// All three are bound by memory latency, not bytes: what they shed is work per CELL where only one
+// All three are bound by instructions and latency, not bytes: what they shed is work per CELL where only one
 // cell in twelve carries surface.  24,000 blocks of 8^3 on a B200: 444 + 114 + 107 us when every cell
 // read its eight corners through the tables, each warp bumped the shared counters and an edge took
-// four bytes of a 147 MB table that had to be filled, written and read.
+// four bytes of a 147 MB table that had to be filled, written and read; 130 + 39 + 57 us now.
 //
 // The triangulation table is this repository's own (mc_tables.h, derived by gen_mc_tables.py):
 // the reference's table is not reproduced, so which diagonal splits an ambiguous pattern, the
@@ -94,10 +94,11 @@ __global__ void __launch_bounds__(256) mc_check_tables_kernel(McLuts L, McEdges 
 }
 
 constexpr int kMaxTileBlocks = 32;
+constexpr int kTileTarget = 1024;   // cells
 constexpr int kMaxFastEdge = 16;
 constexpr int kClassifyCtas = 6;   // per SM: what 40 registers allow
 
-// A CTA walks tiles of max(1, 256 / G^3) blocks.  It stages one state byte per cell of the block AND of the
+// A CTA walks tiles of max(1, 1024 / G^3) blocks (five barriers a tile: 512 cells of G = 8 are too few).  It stages one state byte per cell of the block AND of the
 // layer that its upper neighbours add, (G + 1)^3 in all, so every value is read once (G = 8: 1.4 loads
 // of sdf and weight per cell instead of 8 of each behind 24 table reads); cubes then read bytes of
 // shared memory.  Requests for the block's own edges meet in shared memory and go out a word at a
@@ -110,8 +111,15 @@ __global__ void __launch_bounds__(256, kClassifyCtas) mc_classify_kernel(const f
                                                           uint8_t* __restrict__ codes, McEdges edges,
                                                           unsigned long long* __restrict__ counters, float iso_value,
                                                           float weight_thr, int G_arg, int64_t num_grids) {
-    __shared__ uint8_t state[(kMaxFastEdge + 1) * (kMaxFastEdge + 1) * (kMaxFastEdge + 1) + 15];
-    __shared__ uint32_t own[kMaxFastEdge * kMaxFastEdge * kMaxFastEdge / 4];
+    // largest tile: of kTileTarget cells, of a block with more, and for G not known here of any of either
+    constexpr int kTileCells = GT == 8 || GT == 4 ? kTileTarget : kMaxFastEdge * kMaxFastEdge * kMaxFastEdge;
+    constexpr int kHalo = (GT + 1) * (GT + 1) * (GT + 1);
+    __shared__ uint8_t state[GT == 8 ? 2 * kHalo : GT == 4 ? 16 * kHalo : (kMaxFastEdge + 1) * (kMaxFastEdge + 1) * (kMaxFastEdge + 1)];
+    // where a cell of a block's halo comes from: cell | neighbour << 9; 25 instructions otherwise
+    __shared__ uint16_t halo_cell[GT == 8 || GT == 4 ? kHalo : 1];
+    __shared__ uint32_t own[kTileCells / 4];
+    __shared__ uint32_t active[kTileCells];   // cells with surface: cell of the tile | code << 16
+    __shared__ int n_active;
     __shared__ int64_t rows[kMaxTileBlocks * 8];
     __shared__ uint16_t edge_mask[256];
     __shared__ uint8_t tri_count[256];
@@ -150,26 +158,48 @@ __global__ void __launch_bounds__(256, kClassifyCtas) mc_classify_kernel(const f
         }
     } else {
         const int H = G + 1, halo = H * H * H, cells = G * G * G;
-        const int per_tile = cells >= 256 ? 1 : min(256 / cells, kMaxTileBlocks);
+        const int per_tile = cells >= kTileTarget ? 1 : min(kTileTarget / cells, kMaxTileBlocks);
+        if (GT == 8 || GT == 4) {
+            for (int r = tid; r < halo; r += 256) {
+                const int x = r % H, y = r / H % H, z = r / (H * H);
+                halo_cell[r] = (uint16_t)((x % G + (y % G + z % G * G) * G) | ((x == G) | (y == G) << 1 | (z == G) << 2) << 9);
+            }
+            __syncthreads();
+        }
         const int64_t n_tiles = (num_grids + per_tile - 1) / per_tile;
+        // embedding row of one of a tile's blocks or of one of its upper neighbours, or -1
+        auto row_of = [&](int64_t tile) -> int64_t {
+            const int64_t at = tile * per_tile + (tid >> 3);
+            if (tid >= per_tile * 8 || at >= num_grids) return -1;
+            const int64_t g = L.grid_indices[at];
+            const int64_t nb = g >= 0 && g < L.n_emb ? L.g2g[g * 8 + (tid & 7)] : -1;
+            return nb < L.n_emb ? nb : -1;
+        };
+        int64_t row = row_of(blockIdx.x);
         for (int64_t tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
             const int64_t first = tile * per_tile;
-            const int blocks = (int)min((int64_t)per_tile, num_grids - first);
-            if (tid < blocks * 8) {
-                const int64_t g = L.grid_indices[first + (tid >> 3)];
-                const int64_t nb = g >= 0 && g < L.n_emb ? L.g2g[g * 8 + (tid & 7)] : -1;
-                rows[tid] = nb < L.n_emb ? nb : -1;
-            }
+            const int blocks = per_tile == 1 ? 1 : (int)min((int64_t)per_tile, num_grids - first);
+            if (tid < per_tile * 8) rows[tid] = row;
             for (int w = tid; w < (blocks * cells + 3) / 4; w += 256) own[w] = 0;
+            if (tid == 0) n_active = 0;
             __syncthreads();
+            row = row_of(tile + gridDim.x);   // two dependent loads that the rest of the tile covers
 #pragma unroll 3
             for (int h = tid; h < blocks * halo; h += 256) {
                 const int b = per_tile == 1 ? 0 : h / halo, r = h - b * halo;
-                const int x = r % H, y = r / H % H, z = r / (H * H);
-                const int64_t g = rows[b * 8 + ((x == G) | (y == G) << 1 | (z == G) << 2)];
+                int nb, at;
+                if (GT == 8 || GT == 4) {
+                    nb = halo_cell[r] >> 9;
+                    at = halo_cell[r] & 511;
+                } else {
+                    const int x = r % H, y = r / H % H, z = r / (H * H);
+                    nb = (x == G) | (y == G) << 1 | (z == G) << 2;
+                    at = (x == G ? 0 : x) + ((y == G ? 0 : y) + (z == G ? 0 : z) * G) * G;
+                }
+                const int64_t g = rows[b * 8 + nb];
                 uint8_t s = 0;   // bit 0: observed, bit 1: inside
                 if (g >= 0) {
-                    const int64_t a = g * cells + (x == G ? 0 : x) + ((y == G ? 0 : y) + (z == G ? 0 : z) * G) * G;
+                    const int64_t a = g * cells + at;
                     const float d = sdfs[a];
                     s = weights[a] >= weight_thr ? (d - iso_value < 0.f ? 3 : 1) : 0;
                 }
@@ -189,17 +219,24 @@ __global__ void __launch_bounds__(256, kClassifyCtas) mc_classify_kernel(const f
                 }
                 if (!seen || code == 255) code = 0;
                 codes[first * cells + c] = (uint8_t)code;
-                if (code == 0) continue;
-                n_triangles += tri_count[code];
-                const int mask = edge_mask[code];
+                if (code) active[atomicAdd(&n_active, 1)] = (uint32_t)c | code << 16;
+            }
+            __syncthreads();
+            // a thread per corner of a cube with surface, for the edges that leave it (none leave corner 7)
+            for (int i = tid; i < 7 * n_active; i += 256) {
+                const int which = i / 7, k = i - 7 * which;
+                const uint32_t entry = active[which];
+                const int c = (int)(entry & 0xFFFFu), mask = edge_mask[entry >> 16];
+                uint32_t bits = 0;
 #pragma unroll
-                for (int k = 0; k < 7; ++k) {   // the edges that leave corner k of the cube
-                    uint32_t bits = 0;
-#pragma unroll
-                    for (int e = 0; e < 12; ++e)
-                        if (edge_lower_corner(e) == k) bits |= (uint32_t)((mask >> e) & 1) << (e >> 2);
-                    if (bits == 0) continue;
-                    const int cx = x + (k & 1), cy = y + ((k >> 1) & 1), cz = z + (k >> 2);
+                for (int d = 0; d < 3; ++d) {
+                    const int e = d * 4 + (((k >> ((d + 1) % 3)) & 1) | ((k >> ((d + 2) % 3)) & 1) << 1);
+                    if (((k >> d) & 1) == 0) bits |= (uint32_t)((mask >> e) & 1) << d;
+                }
+                if (k == 0) n_triangles += tri_count[entry >> 16];
+                if (bits) {
+                    const int b = per_tile == 1 ? 0 : c / cells, cell = c - b * cells;
+                    const int cx = cell % G + (k & 1), cy = cell / G % G + ((k >> 1) & 1), cz = cell / (G * G) + (k >> 2);
                     const int nb = (cx == G) | (cy == G) << 1 | (cz == G) << 2;
                     const int at = (cx == G ? 0 : cx) + ((cy == G ? 0 : cy) + (cz == G ? 0 : cz) * G) * G;
                     if (nb == 0) {
@@ -421,7 +458,7 @@ int ashb_marching_cubes_count(const float* sdfs, const float* weights, const int
         mc_check_tables_kernel<<<(unsigned)((cells_per_grid * 8 + 255) / 256), 256, 0, st>>>(L, edges, G);
         ASHB_LAUNCH_CHECK();
     }
-    // persistent: one resident set of CTAs shares out the tiles (27 each at 24,000 blocks)
+    // persistent: one resident set of CTAs shares out the tiles (14 each at 24,000 blocks)
     const unsigned grid = (unsigned)std::min<int64_t>((L.len + 255) / 256, (int64_t)sm_count() * kClassifyCtas);
     auto kernel = G == 8 ? mc_classify_kernel<8> : G == 4 ? mc_classify_kernel<4> : G == 16 ? mc_classify_kernel<16>
                                                                                         : mc_classify_kernel<0>;
