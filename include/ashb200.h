@@ -541,6 +541,18 @@ int ashb_render_rays_backward(ashb_map* map, int interp, const float* embeddings
 int ashb_route_by_owner(const int32_t* keys, int64_t n, int key_dim, int world, int32_t* keys_out,
                         int64_t* perm_out, int64_t* counts_host, void* scratch_dev, void* stream);
 
+/* Around ashb_render_rays_* on tensors, one launch each.
+ *   _to_cells  ray origins [n][3] and the box's corners [3] (world) -> cells: (x - origin) * inv_cell, each step
+ *              rounded; bbox_cell receives min then max.  origin: HOST float[3] or null.
+ *   _split     the rows of ashb_render_rays_forward -> nine arrays: rgb [n][3], depth [n], normal [n][3], weight,
+ *              eikonal_l1, eikonal_l2, sample count, near, far [n].  `columns`: HOST array of device addresses.
+ *   _join      gradients of the first six of them (null: none; strides in elements, two each; HOST arrays) ->
+ *              grad_out rows of ashb_render_rays_backward. */
+int ashb_rays_to_cells(const float* ray_o_world, int64_t n_rays, const float* bbox_min, const float* bbox_max,
+                       const float* origin, float inv_cell, float* ray_o_cell, float* bbox_cell, void* stream);
+int ashb_render_split(const float* rows, float* const* columns, int64_t n_rays, void* stream);
+int ashb_render_join(const float* const* grads, const int64_t* strides, float* grad_rows, int64_t n_rays, void* stream);
+
 /* The same renderer with the samples of a ray evaluated in parallel: _intervals marches every ray
  * once (one thread per ray) and lists its intervals, float32 [n_rays][stride][2] (t0, t1 in cell
  * units), with counts int32 [n_rays] and near_far float32 [n_rays][2] (world units); intervals

@@ -31,3 +31,42 @@ def test_group_march_equals_thread_march(capacity, n, t_min, t_max, samples):
         assert torch.equal(thread[k], group[k]), k
     for k in ("depth", "weights"):
         torch.testing.assert_close(group[k], thread[k], rtol=2e-4, atol=2e-5)
+
+
+@pytest.mark.parametrize("cell_size", [0.02, 1.0 / 3.0, 7e-4])
+@pytest.mark.parametrize("n", [0, 1, 85, 1000])
+def test_rays_to_cells_rounds_as_the_tensor_expressions(cell_size, n):
+    import __ash
+
+    g = torch.Generator(device=DEV).manual_seed(n)
+    o = torch.randn(n, 3, device=DEV, generator=g)
+    lo, hi = torch.randn(2, 3, device=DEV, generator=g)
+    origin = [float(v) for v in torch.randn(3, generator=g, device=DEV)]
+    shift = torch.tensor(origin, device=DEV)
+    for got, x in zip(__ash.rays_to_cells(o, lo, hi, origin, cell_size), (o, lo, hi)):
+        assert torch.equal(got, (x - shift) / cell_size)
+
+
+@pytest.mark.parametrize("parallel", [False, True])
+def test_outputs_take_gradients_of_any_layout_and_may_be_changed_in_place(parallel):
+    from ash.render import render_rays
+    from test_raymarch_gpu import make_grid
+
+    grid = make_grid("bounded", 4, seed=5)
+    o, d = make_rays(grid, 300, 3, torch.zeros(3, device=DEV))
+    coef = torch.randn(3, 300, device=DEV).t()
+    grads = []
+    for dense in (False, True):
+        grid.embeddings.grad = None
+        beta = torch.tensor([0.03], device=DEV, requires_grad=True)
+        out = render_rays(grid, o, d, 0.05, 2.0, 48, beta, parallel_samples=parallel)
+        assert not any(out[k].requires_grad for k in ("n_samples", "near", "far"))
+        if dense:
+            (out["rgb"] * coef.contiguous() + out["weights"] * torch.ones_like(out["weights"])).sum().backward()
+        else:
+            out["rgb"].mul_(coef).add_(out["weights"])
+            out["rgb"].sum().backward()
+        grads.append((grid.embeddings.grad.clone(), beta.grad.clone()))
+    scale = float(grads[1][0].abs().max())
+    torch.testing.assert_close(grads[0][0], grads[1][0], rtol=1e-4, atol=1e-5 * scale)
+    torch.testing.assert_close(grads[0][1], grads[1][1], rtol=1e-4, atol=1e-6)

@@ -71,6 +71,9 @@ _lib.ashb_grid_query_backward.argtypes = [_vp, _int, _int, _vp, _vp, _vp, _c.c_d
                                           _i64, _i64, _i64, _vp]
 _lib.ashb_grid_query_backward_backward.argtypes = [_vp, _int, _int, _vp, _vp, _vp, _vp, _c.c_double, _vp, _int, _vp, _vp, _vp,
                                                    _vp, _int, _i64, _i64, _i64, _vp]
+_lib.ashb_rays_to_cells.argtypes = [_vp, _i64, _vp, _vp, _vp, _f32, _vp, _vp, _vp]
+_lib.ashb_render_split.argtypes = [_vp, _vp, _i64, _vp]
+_lib.ashb_render_join.argtypes = [_vp, _vp, _vp, _i64, _vp]
 _lib.ashb_conv_forward_tiled.argtypes = [_vp, _vp, _vp, _vp, _vp, _int, _i64, _i64, _int, _int, _i64, _vp]
 _lib.ashb_conv_forward_separable.argtypes = [_vp, _vp, _vp, _vp, _vp, _int, _i64, _i64, _int, _int, _i64, _vp]
 _lib.ashb_filter_separable_inplace.argtypes = [_vp] * 6 + [_i64, _int, _int, _i64, _vp]
@@ -1136,8 +1139,7 @@ def render_rays_forward(hashmap, embeddings, nb_lut, cell_size, origin, ray_o_wo
                                    bbox_min_cell, bbox_max_cell, t_min_cell, t_max_cell, max_samples_per_ray,
                                    skip_missed, beta, interpolation)
     out = torch.empty((n, 16), dtype=torch.float32, device=emb.device)
-    with torch.cuda.device(emb.device):
-        _check(_lib.ashb_render_rays_forward(*args, out.data_ptr(), n, _stream(emb.device)))
+    _check(_lib.ashb_render_rays_forward(*args, out.data_ptr(), n, _stream(emb.device)))
     return out
 
 
@@ -1160,9 +1162,8 @@ def render_rays_backward(hashmap, embeddings, nb_lut, cell_size, origin, ray_o_w
         if not (ge.is_cuda and ge.is_contiguous() and ge.shape == emb.shape and ge.dtype == emb.dtype):
             raise RuntimeError("grad_embeddings_out must be a contiguous CUDA tensor shaped like embeddings")
     gb = torch.zeros(1, dtype=torch.float32, device=emb.device)
-    with torch.cuda.device(emb.device):
-        _check(_lib.ashb_render_rays_backward(*args, out.data_ptr(), go.data_ptr(), ge.data_ptr(), gb.data_ptr(), n,
-                                              _stream(emb.device)))
+    _check(_lib.ashb_render_rays_backward(*args, out.data_ptr(), go.data_ptr(), ge.data_ptr(), gb.data_ptr(), n,
+                                          _stream(emb.device)))
     return ge, gb
 
 
@@ -1305,11 +1306,10 @@ def render_rays_intervals(hashmap, embeddings, nb_lut, cell_size, origin, ray_o_
     intervals = torch.empty((n, stride, 2), dtype=torch.float32, device=dev)
     counts = torch.empty(n, dtype=torch.int32, device=dev)
     near_far = torch.empty((n, 2), dtype=torch.float32, device=dev)
-    with torch.cuda.device(dev):
-        _check(_lib.ashb_render_rays_intervals(*args, oc.data_ptr(), d.data_ptr(), lo.data_ptr(), hi.data_ptr(),
-                                               float(t_min_cell), float(t_max_cell), int(max_samples_per_ray),
-                                               int(bool(skip_missed)), intervals.data_ptr(), counts.data_ptr(),
-                                               near_far.data_ptr(), stride, n, _stream(dev)))
+    _check(_lib.ashb_render_rays_intervals(*args, oc.data_ptr(), d.data_ptr(), lo.data_ptr(), hi.data_ptr(),
+                                           float(t_min_cell), float(t_max_cell), int(max_samples_per_ray),
+                                           int(bool(skip_missed)), intervals.data_ptr(), counts.data_ptr(),
+                                           near_far.data_ptr(), stride, n, _stream(dev)))
     return intervals, counts, near_far
 
 
@@ -1322,10 +1322,9 @@ def render_intervals_forward(hashmap, embeddings, nb_lut, cell_size, origin, ray
     b = _cuda(beta, "beta", torch.float32).view(-1)
     n, dev = ow.shape[0], ow.device
     out = torch.empty((n, 16), dtype=torch.float32, device=dev)
-    with torch.cuda.device(dev):
-        _check(_lib.ashb_render_intervals_forward(*args, ow.data_ptr(), d.data_ptr(), b.data_ptr(), intervals.data_ptr(),
-                                                  counts.data_ptr(), near_far.data_ptr(), intervals.shape[1],
-                                                  out.data_ptr(), n, _stream(dev)))
+    _check(_lib.ashb_render_intervals_forward(*args, ow.data_ptr(), d.data_ptr(), b.data_ptr(), intervals.data_ptr(),
+                                              counts.data_ptr(), near_far.data_ptr(), intervals.shape[1],
+                                              out.data_ptr(), n, _stream(dev)))
     return out
 
 
@@ -1349,11 +1348,57 @@ def render_intervals_backward(hashmap, embeddings, nb_lut, cell_size, origin, ra
         if not (ge.is_cuda and ge.is_contiguous() and ge.shape == emb.shape and ge.dtype == emb.dtype):
             raise RuntimeError("grad_embeddings_out must be a contiguous CUDA tensor shaped like embeddings")
     gb = torch.zeros(1, dtype=torch.float32, device=dev)
-    with torch.cuda.device(dev):
-        _check(_lib.ashb_render_intervals_backward(*args, ow.data_ptr(), d.data_ptr(), b.data_ptr(), intervals.data_ptr(),
-                                                   counts.data_ptr(), intervals.shape[1], out.data_ptr(), go.data_ptr(),
-                                                   ge.data_ptr(), gb.data_ptr(), n, _stream(dev)))
+    _check(_lib.ashb_render_intervals_backward(*args, ow.data_ptr(), d.data_ptr(), b.data_ptr(), intervals.data_ptr(),
+                                               counts.data_ptr(), intervals.shape[1], out.data_ptr(), go.data_ptr(),
+                                               ge.data_ptr(), gb.data_ptr(), n, _stream(dev)))
     return ge, gb
+
+
+def rays_to_cells(ray_o_world, bbox_min, bbox_max, origin, cell_size):
+    """``(x - origin) / cell_size`` of the ray origins and of the box's corners in one launch: (origins (n, 3),
+    min (3,), max (3,)), rounded as those tensor expressions are."""
+    o = _cuda(ray_o_world, "ray_o_world", torch.float32)
+    lo, hi = _cuda(bbox_min, "bbox_min", torch.float32), _cuda(bbox_max, "bbox_max", torch.float32)
+    if o.dim() != 2 or o.shape[1] != 3 or lo.numel() != 3 or hi.numel() != 3:
+        raise RuntimeError("ray origins must be (n_rays, 3) and the box's corners (3,)")
+    o_cell = torch.empty_like(o)
+    box = torch.empty((2, 3), dtype=torch.float32, device=o.device)
+    inv = 1.0 / float(cell_size)   # in double, rounded once when passed: what dividing a tensor by a number multiplies by
+    with torch.cuda.device(o.device):
+        _check(_lib.ashb_rays_to_cells(o.data_ptr(), o.shape[0], lo.data_ptr(), hi.data_ptr(), _host_floats(origin, 3), inv,
+                                       o_cell.data_ptr(), box.data_ptr(), _stream(o.device)))
+    return o_cell, box[0], box[1]
+
+
+_RENDER_WIDTHS = (3, 1, 3, 1, 1, 1, 1, 1, 1)
+
+
+def render_split(rows):
+    """The columns of the renderer's (n, 16) rows as nine tensors of their own: rgb, depth, normal, weight, the two
+    eikonal sums, sample count, near, far."""
+    n = rows.shape[0]
+    columns = [torch.empty((n, w), dtype=torch.float32, device=rows.device) for w in _RENDER_WIDTHS]
+    with torch.cuda.device(rows.device):
+        _check(_lib.ashb_render_split(rows.data_ptr(), (_vp * 9)(*[c.data_ptr() for c in columns]), n, _stream(rows.device)))
+    return columns
+
+
+def render_join(grads, rows):
+    """Gradients of the first six of those columns (None: none), of any strides, as rows like ``rows``."""
+    n, out = rows.shape[0], torch.empty_like(rows)
+    pointers, strides, keep = (_vp * 6)(), (_i64 * 12)(), []
+    for k, g in enumerate(grads):
+        if g is None:
+            continue
+        g = g if g.is_cuda and g.dtype == torch.float32 else g.to(rows)
+        if g.shape != (n, _RENDER_WIDTHS[k]):
+            raise RuntimeError("gradient of another shape than its output")
+        keep.append(g)
+        pointers[k] = g.data_ptr()
+        strides[2 * k], strides[2 * k + 1] = g.stride()
+    with torch.cuda.device(rows.device):
+        _check(_lib.ashb_render_join(pointers, strides, out.data_ptr(), n, _stream(rows.device)))
+    return out
 
 
 # ---- table sharded over the ranks, queries routed to the owners -----------------------------------

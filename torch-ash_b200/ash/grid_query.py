@@ -113,10 +113,13 @@ class FusedGridQuery(torch.autograd.Function):
         ctx.save_for_backward(embeddings, x, block_idx)
         ctx.geom = geom
         ctx.mark_non_differentiable(masks)
+        ctx.set_materialize_grads(False)   # or each backward pass fills a tensor of zeros for the masks
         return y, masks
 
     @staticmethod
     def backward(ctx, z, _grad_masks):
+        if z is None:
+            return None, None, None
         embeddings, x, block_idx = ctx.saved_tensors
         # positions that need no gradient spare the backward its eight embedding-row reads
         need_grad_x = bool(ctx.needs_input_grad[1])

@@ -86,39 +86,47 @@ class SDFToDensity(nn.Module):
         return (1 / beta) * (0.5 + 0.5 * sdf.sign() * torch.expm1(-sdf.abs() / beta))
 
 
+def _render_rows(embeddings, beta, geom, rays, parallel_samples):
+    """The kernels' (n, 16) rows, and the list of intervals that a backward pass can reuse (or None)."""
+    if not parallel_samples:
+        return backend.render_rays_forward(geom[0], embeddings, *geom[1:4], *rays, beta, geom[4]), None
+    o_world, o_cell, d = rays[0], rays[1], rays[2]
+    intervals, counts, near_far = backend.render_rays_intervals(
+        geom[0], embeddings, *geom[1:4], o_cell, d, *rays[3:], geom[4])
+    rows = backend.render_intervals_forward(geom[0], embeddings, *geom[1:4], o_world, d, beta, intervals, counts, near_far,
+                                            geom[4])
+    return rows, (intervals, counts)
+
+
 class _RenderRays(torch.autograd.Function):
     """One launch forward, one launch backward for the whole ray -> pixel composition -- or, with
     ``parallel_samples``, a marching launch that lists every ray's intervals followed by a
-    warp-per-ray evaluation (and a backward that reuses the list)."""
+    warp-per-ray evaluation (and a backward that reuses the list).  The outputs are tensors of their own:
+    as slices of the kernels' rows each of them would cost autograd a zero-fill, a copy and a sum."""
 
     @staticmethod
     def forward(ctx, embeddings, beta, geom, rays, parallel_samples):
-        ctx.listed = None
-        if parallel_samples:
-            o_world, o_cell, d = rays[0], rays[1], rays[2]
-            intervals, counts, near_far = backend.render_rays_intervals(
-                geom[0], embeddings, *geom[1:4], o_cell, d, *rays[3:], geom[4])
-            rows = backend.render_intervals_forward(geom[0], embeddings, *geom[1:4], o_world, d, beta, intervals,
-                                                    counts, near_far, geom[4])
-            ctx.listed = (intervals, counts)
-        else:
-            rows = backend.render_rays_forward(geom[0], embeddings, *geom[1:4], *rays, beta, geom[4])
+        rows, ctx.listed = _render_rows(embeddings, beta, geom, rays, parallel_samples)
         ctx.save_for_backward(embeddings, beta, rows)
         ctx.geom, ctx.rays = geom, rays
-        return rows
+        ctx.set_materialize_grads(False)
+        columns = backend.render_split(rows)
+        ctx.mark_non_differentiable(*columns[6:])
+        return tuple(columns)
 
     @staticmethod
-    def backward(ctx, grad_rows):
+    def backward(ctx, *grads):
         embeddings, beta, rows = ctx.saved_tensors
         geom, rays = ctx.geom, ctx.rays
+        grad_rows = backend.render_join(grads[:6], rows)
         grad_buffer = geom[5]
         if ctx.listed is not None:
             grad_embeddings, grad_beta = backend.render_intervals_backward(
-                geom[0], embeddings, *geom[1:4], rays[0], rays[2], beta, *ctx.listed, rows, grad_rows.contiguous(),
+                geom[0], embeddings, *geom[1:4], rays[0], rays[2], beta, *ctx.listed, rows, grad_rows,
                 geom[4], grad_embeddings_out=grad_buffer)
         else:
             grad_embeddings, grad_beta = backend.render_rays_backward(
-                geom[0], embeddings, *geom[1:4], *rays, beta, rows, grad_rows.contiguous(), geom[4],
+                geom[0], embeddings, *geom[1:4], *rays, beta, rows, grad_rows, geom[4],
                 grad_embeddings_out=grad_buffer)
         if grad_buffer is not None or not ctx.needs_input_grad[0]:
             grad_embeddings = None
@@ -163,14 +171,17 @@ def render_rays(grid, rays_o: torch.Tensor, rays_d: torch.Tensor, t_min: float, 
             grid.embeddings.grad = torch.zeros_like(grid.embeddings)
         grad_buffer = grid.embeddings.grad
     with torch.no_grad():
-        bbox_min, bbox_max = grid.get_bbox()
-        rays = (rays_o.contiguous(), grid.transform_world_to_cell(rays_o).contiguous(), rays_d.contiguous(),
-                grid.transform_world_to_cell(bbox_min).contiguous(), grid.transform_world_to_cell(bbox_max).contiguous(),
-                t_min / grid.cell_size, t_max / grid.cell_size, int(max_samples_per_ray), bool(skip_rays_without_hit))
+        rays_o, (bbox_min, bbox_max) = rays_o.contiguous(), grid.get_bbox()
+        o_cell, lo_cell, hi_cell = backend.rays_to_cells(rays_o, bbox_min, bbox_max, origin, cell_size)
+        rays = (rays_o, o_cell, rays_d.contiguous(), lo_cell, hi_cell, t_min / grid.cell_size, t_max / grid.cell_size,
+                int(max_samples_per_ray), bool(skip_rays_without_hit))
     geom = (grid.engine.backend, grid._neighbor_lut32(), cell_size, origin, interpolation, grad_buffer)
     if parallel_samples is None:
         parallel_samples = rays_o.shape[0] <= 32768
-    rows = _RenderRays.apply(grid.embeddings, beta.to(torch.float32), geom, rays, bool(parallel_samples))
-    return {"rgb": rows[:, 0:3], "depth": rows[:, 3:4], "normal": rows[:, 4:7], "weights": rows[:, 7:8],
-            "eikonal_l1": rows[:, 8:9], "eikonal_l2": rows[:, 9:10], "n_samples": rows[:, 10:11].detach(),
-            "near": rows[:, 11:12].detach(), "far": rows[:, 12:13].detach()}
+    beta = beta.to(torch.float32)
+    if torch.is_grad_enabled() and (grid.embeddings.requires_grad or beta.requires_grad):
+        columns = _RenderRays.apply(grid.embeddings, beta, geom, rays, bool(parallel_samples))
+    else:
+        rows, _ = _render_rows(grid.embeddings, beta, geom, rays, bool(parallel_samples))
+        columns = [rows[:, a:b] for a, b in ((0, 3), (3, 4), (4, 7), (7, 8), (8, 9), (9, 10), (10, 11), (11, 12), (12, 13))]
+    return dict(zip(("rgb", "depth", "normal", "weights", "eikonal_l1", "eikonal_l2", "n_samples", "near", "far"), columns))

@@ -521,6 +521,63 @@ __global__ void __launch_bounds__(256) render_intervals_backward_kernel(
     if (lane == 0 && gbeta != 0.f) atomicAdd(grad_beta, gbeta);
 }
 
+// ---- around the renderer: one launch where tensor expressions took several -------------------------
+struct Origin { float v[3]; };
+
+// World -> cell of the ray origins and of the box's two corners (entries n and n + 1), rounded as
+// (x - origin) / cell_size is on a tensor: a difference, then a product with the float reciprocal.
+__global__ void __launch_bounds__(256) rays_to_cells_kernel(const float* __restrict__ o, const float* __restrict__ lo,
+                                                            const float* __restrict__ hi, Origin origin, float inv_cell,
+                                                            float* __restrict__ o_cell, float* __restrict__ box_cell,
+                                                            int64_t n) {
+    const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
+    if (i >= 3 * n + 6) return;
+    const int64_t at = i - 3 * n;
+    const float x = at < 0 ? o[i] : at < 3 ? lo[at] : hi[at - 3];
+    const float v = __fmul_rn(__fsub_rn(x, origin.v[i % 3]), inv_cell);
+    if (at < 0) o_cell[i] = v;
+    else box_cell[at] = v;
+}
+
+// The first 13 columns of the renderer's rows as nine tensors, and the gradients of the first six of them as rows.
+constexpr int kColumns = 9;
+struct RenderColumns { float* p[kColumns]; };
+struct RenderGradients { const float* p[6]; long long stride[6][2]; };   // null: no gradient
+
+__device__ __forceinline__ int column_of(int c, int& within) {   // widths 3 1 3 1 1 1 1 1 1
+    within = c < 3 ? c : c >= 4 && c < 7 ? c - 4 : 0;
+    return c < 3 ? 0 : c == 3 ? 1 : c < 7 ? 2 : c - 4;
+}
+
+// A thread per ray: four wide loads, and every store instruction of a warp writes one stretch.
+__global__ void __launch_bounds__(256) render_split_kernel(const float4* __restrict__ rows, RenderColumns out, int64_t n) {
+    const int64_t ray = (int64_t)blockIdx.x * 256 + threadIdx.x;
+    if (ray >= n) return;
+    float v[kRayOut];
+#pragma unroll
+    for (int j = 0; j < kRayOut / 4; ++j) *reinterpret_cast<float4*>(v + 4 * j) = rows[ray * (kRayOut / 4) + j];
+#pragma unroll
+    for (int c = 0; c < 13; ++c) {
+        int within;
+        const int k = column_of(c, within);
+        out.p[k][ray * (k == 0 || k == 2 ? 3 : 1) + within] = v[c];
+    }
+}
+
+__global__ void __launch_bounds__(256) render_join_kernel(RenderGradients in, float* __restrict__ rows, int64_t n) {
+    const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
+    const int c = (int)(i & (kRayOut - 1));
+    const int64_t ray = i / kRayOut;
+    if (ray >= n) return;
+    float v = 0.f;
+    if (c < 10) {
+        int within;
+        const int k = column_of(c, within);
+        if (in.p[k]) v = in.p[k][ray * in.stride[k][0] + within * in.stride[k][1]];
+    }
+    rows[i] = v;
+}
+
 }  // namespace ashb
 
 using namespace ashb;
@@ -688,6 +745,49 @@ int ashb_render_intervals_backward(ashb_map* map, int interp, const float* embed
         render_intervals_backward_kernel<false><<<grid, 256, 0, st>>>(g, ray_o_world, ray_d, beta, iv, counts,
                                                                       (int)stride, out, grad_out, grad_embeddings,
                                                                       grad_beta, n_rays);
+    ASHB_LAUNCH_CHECK();
+    return ASHB_OK;
+}
+
+int ashb_rays_to_cells(const float* ray_o_world, int64_t n_rays, const float* bbox_min, const float* bbox_max,
+                       const float* origin, float inv_cell, float* ray_o_cell, float* bbox_cell, void* stream) {
+    ASHB_REQUIRE(n_rays >= 0 && bbox_min && bbox_max && bbox_cell, "bad ray count or null buffer");
+    ASHB_REQUIRE(n_rays == 0 || (ray_o_world && ray_o_cell), "null buffer");
+    Origin org{};
+    for (int k = 0; k < 3; ++k) org.v[k] = origin ? origin[k] : 0.f;
+    rays_to_cells_kernel<<<(unsigned)((3 * n_rays + 6 + 255) / 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+            ray_o_world, bbox_min, bbox_max, org, inv_cell, ray_o_cell, bbox_cell, n_rays);
+    ASHB_LAUNCH_CHECK();
+    return ASHB_OK;
+}
+
+int ashb_render_split(const float* rows, float* const* columns, int64_t n_rays, void* stream) {
+    ASHB_REQUIRE(n_rays >= 0 && columns != nullptr, "bad ray count or null table");
+    if (n_rays == 0) return ASHB_OK;
+    RenderColumns out{};
+    for (int k = 0; k < kColumns; ++k) {
+        ASHB_REQUIRE(columns[k] != nullptr, "null buffer");
+        out.p[k] = columns[k];
+    }
+    ASHB_REQUIRE(rows != nullptr && ((uintptr_t)rows & 15) == 0, "null or misaligned rows");
+    render_split_kernel<<<(unsigned)((n_rays + 255) / 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+            reinterpret_cast<const float4*>(rows), out, n_rays);
+    ASHB_LAUNCH_CHECK();
+    return ASHB_OK;
+}
+
+int ashb_render_join(const float* const* grads, const int64_t* strides, float* grad_rows, int64_t n_rays, void* stream) {
+    ASHB_REQUIRE(n_rays >= 0 && grads != nullptr && strides != nullptr, "bad ray count or null table");
+    if (n_rays == 0) return ASHB_OK;
+    ASHB_REQUIRE(grad_rows != nullptr, "null buffer");
+    RenderGradients in{};
+    for (int k = 0; k < 6; ++k) {
+        in.p[k] = grads[k];
+        in.stride[k][0] = strides[2 * k];
+        in.stride[k][1] = strides[2 * k + 1];
+    }
+    render_join_kernel<<<(unsigned)((n_rays * kRayOut + 255) / 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+            in, grad_rows, n_rays);
     ASHB_LAUNCH_CHECK();
     return ASHB_OK;
 }
