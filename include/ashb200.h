@@ -89,9 +89,18 @@ int ashb_map_status_async(ashb_map* map, uint32_t* status_out_host, void* stream
 int ashb_map_find(ashb_map* map, const int32_t* keys_dev, int64_t n, int64_t* indices_dev,
                   uint8_t* masks_dev, void* stream);
 
+/* The masks of ashb_map_find alone. */
+int ashb_map_contains(ashb_map* map, const int32_t* keys_dev, int64_t n, uint8_t* masks_dev, void* stream);
+
 /* Replaces insert_kernel (keys) + insert_keys (ash/src/hashmap_gpu.cuh:212-247).
  * Insert-if-absent; each new key takes heap[counter++]. */
 int ashb_map_insert_keys(ashb_map* map, const int32_t* keys_dev, int64_t n, void* stream);
+
+/* The same for a large batch into a table far beyond L2, its keys first sorted by the part of the table they
+ * belong to.  _workspace: bytes of device scratch (16-byte aligned) that this takes, 0 where it does not apply. */
+int64_t ashb_map_insert_workspace(ashb_map* map, int64_t n);
+int ashb_map_insert_keys_sorted(ashb_map* map, const int32_t* keys_dev, int64_t n, void* workspace,
+                                int64_t workspace_bytes, void* stream);
 
 /* Replaces insert_kernel (values) + insert + ValueContext
  * (ash/src/hashmap_gpu.cuh:23-114, :250-313).  For each NEW key i with index

@@ -39,7 +39,11 @@ _lib.ashb_map_size.argtypes = [_vp, _vp, _c.POINTER(_i64)]
 _lib.ashb_map_status.argtypes = [_vp, _vp, _c.POINTER(_c.c_uint32)]
 _lib.ashb_map_status_async.argtypes = [_vp, _vp, _vp]
 _lib.ashb_map_find.argtypes = [_vp, _vp, _i64, _vp, _vp, _vp]
+_lib.ashb_map_contains.argtypes = [_vp, _vp, _i64, _vp, _vp]
 _lib.ashb_map_insert_keys.argtypes = [_vp, _vp, _i64, _vp]
+_lib.ashb_map_insert_workspace.argtypes = [_vp, _i64]
+_lib.ashb_map_insert_workspace.restype = _i64
+_lib.ashb_map_insert_keys_sorted.argtypes = [_vp, _vp, _i64, _vp, _i64, _vp]
 _lib.ashb_map_insert_values.argtypes = [_vp, _vp, _i64, _int, _vp, _vp, _vp, _vp]
 _lib.ashb_map_erase.argtypes = [_vp, _vp, _i64, _vp]
 _lib.ashb_map_items.argtypes = [_vp, _vp, _vp, _i64, _c.POINTER(_i64), _vp]
@@ -263,8 +267,25 @@ class HashMap:
         _check(_lib.ashb_map_find(self._h, keys.data_ptr(), n, indices.data_ptr(), masks.data_ptr(), _stream(self._device)))
         return indices, masks
 
+    def contains(self, keys: torch.Tensor) -> torch.Tensor:
+        """The masks of ``find`` alone (not in the reference)."""
+        keys = self._keys(keys)
+        masks = torch.empty(keys.shape[0], dtype=torch.bool, device=self._device)
+        _check(_lib.ashb_map_contains(self._h, keys.data_ptr(), keys.shape[0], masks.data_ptr(), _stream(self._device)))
+        return masks
+
     def insert_keys(self, keys: torch.Tensor) -> None:
         keys = self._keys(keys)
+        nbytes = _lib.ashb_map_insert_workspace(self._h, keys.shape[0])
+        if nbytes:
+            try:
+                workspace = torch.empty(nbytes, dtype=torch.uint8, device=self._device)
+            except torch.cuda.OutOfMemoryError:   # then in the batch's own order
+                workspace = None
+            if workspace is not None:
+                _check(_lib.ashb_map_insert_keys_sorted(self._h, keys.data_ptr(), keys.shape[0], workspace.data_ptr(), nbytes,
+                                                        _stream(self._device)))
+                return
         _check(_lib.ashb_map_insert_keys(self._h, keys.data_ptr(), keys.shape[0], _stream(self._device)))
 
     def insert(self, keys: torch.Tensor, values: dict, external_values: dict) -> None:

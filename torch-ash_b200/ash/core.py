@@ -139,6 +139,15 @@ class ASHEngine(nn.Module):
             )
         return self.backend.find(k)
 
+    def contains(self, keys: torch.Tensor) -> torch.Tensor:
+        """The masks of ``find`` without its indices."""
+        if not hasattr(self.backend, "contains"):
+            return self.find(keys)[1]
+        k = self._prepare(keys)
+        if k is None:
+            return torch.empty((0,), dtype=torch.bool, device=self.device)
+        return self.backend.contains(k)
+
     def insert_keys(self, keys: torch.Tensor) -> None:
         """Insert-if-absent without values; each new key takes the next free index."""
         k = self._prepare(keys)

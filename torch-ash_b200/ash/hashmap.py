@@ -123,7 +123,7 @@ class HashSet(ASHModule):
         self.engine.insert_keys(keys)
 
     def find(self, keys: torch.Tensor) -> torch.Tensor:
-        return self.engine.find(keys)[1]
+        return self.engine.contains(keys)
 
     def erase(self, keys: torch.Tensor) -> None:
         self.engine.erase(keys)

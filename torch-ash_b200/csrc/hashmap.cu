@@ -65,10 +65,10 @@ __global__ void __launch_bounds__(256) find_kernel(Table t, const int32_t* __res
         }
     }
     if constexpr (FILTER) {
-        __stcs(indices + i, found >= 0 ? (int64_t)found : 0);
+        if (indices) __stcs(indices + i, found >= 0 ? (int64_t)found : 0);
         __stcs(masks + i, (uint8_t)(found >= 0));
     } else {
-        indices[i] = found >= 0 ? (int64_t)found : 0;
+        if (indices) indices[i] = found >= 0 ? (int64_t)found : 0;
         masks[i] = (uint8_t)(found >= 0);
     }
 }
@@ -117,7 +117,7 @@ __global__ void __launch_bounds__(256) find_coop_kernel(Table16 t, const int32_t
         }
     }
     if (live && sub == 0) {
-        indices[q] = found >= 0 ? (int64_t)found : 0;
+        if (indices) indices[q] = found >= 0 ? (int64_t)found : 0;
         masks[q] = (uint8_t)(found >= 0);
     }
 }
@@ -174,6 +174,114 @@ __global__ void __launch_bounds__(256) insert_kernel(Table t, const int32_t* __r
         copy_row(vctx.src[j] + i * vctx.row_bytes[j], vctx.dst[j] + (long long)idx * vctx.row_bytes[j],
                  vctx.row_bytes[j], vctx.word[j]);
     publish_index(t, slot, idx);
+}
+
+// ---- insert of a large batch into a large table, window by window ----------------------------------
+// A batch of several keys per 128-byte line of the table, inserted in its own order, fetches a line from
+// DRAM for every key of it and writes it back for most.  Sorted first into windows of the table that stay
+// in L2 (2^kWindowShift of them, 32 MB), each line comes and goes once: two streams over the keys (count 0.10,
+// sort 0.38 ms) buy that.  50M keys, half of them twice, into 2 GB: 2.29 -> 2.01 ms.
+constexpr uint32_t kWindowShift = 21;        // slots per window
+constexpr int kMaxWindows = 256;
+constexpr int kSortKeys = 2048;              // keys of a CTA: 8 per thread
+
+// Inside a window the rest of a line is wanted too: fetched whole.
+struct Table16Lines : Table16 {
+    __device__ __forceinline__ Entry read_fresh(uint32_t s) const {
+        uint4 u;
+        asm volatile("ld.global.cg.L2::128B.v4.u32 {%0,%1,%2,%3}, [%4];"
+                     : "=r"(u.x), "=r"(u.y), "=r"(u.z), "=r"(u.w)
+                     : "l"(slots + s)
+                     : "memory");
+        return unpack(u);
+    }
+};
+
+template <int DIM>
+__device__ __forceinline__ int window_of(const int32_t* __restrict__ keys, int64_t i, uint32_t mask, int* k) {
+    int k3;
+    load_key<DIM>(keys, i, k[0], k[1], k[2], k3);
+    return (int)((hash_key(k[0], k[1], k[2], 0) & mask) >> kWindowShift);
+}
+
+template <int DIM>
+__global__ void __launch_bounds__(256) window_count_kernel(uint32_t mask, const int32_t* __restrict__ keys, int64_t n,
+                                                           uint32_t* __restrict__ count) {
+    __shared__ uint32_t mine[kMaxWindows];
+    mine[threadIdx.x] = 0;
+    __syncthreads();
+    for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < n; i += (int64_t)gridDim.x * 256) {
+        int k[3];
+        atomicAdd(mine + window_of<DIM>(keys, i, mask, k), 1u);
+    }
+    __syncthreads();
+    if (mine[threadIdx.x]) atomicAdd(count + threadIdx.x, mine[threadIdx.x]);
+}
+
+// Exclusive prefix over the CTA's 256 threads.
+__device__ __forceinline__ uint32_t prefix_256(uint32_t v) {
+    __shared__ uint32_t warp_total[8];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint32_t incl = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t u = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += u;
+    }
+    if (lane == 31) warp_total[warp] = incl;
+    __syncthreads();
+    uint32_t before = 0;
+    for (int w = 0; w < warp; ++w) before += warp_total[w];
+    return before + incl - v;
+}
+
+__global__ void __launch_bounds__(256) window_start_kernel(const uint32_t* __restrict__ count, uint32_t* __restrict__ cursor) {
+    cursor[threadIdx.x] = prefix_256(count[threadIdx.x]);
+}
+
+template <int DIM>
+__global__ void __launch_bounds__(256) window_sort_kernel(uint32_t mask, const int32_t* __restrict__ keys, int64_t n,
+                                                          uint32_t* __restrict__ cursor, int32_t* __restrict__ sorted) {
+    constexpr int kEach = kSortKeys / 256;
+    __shared__ uint32_t count[kMaxWindows], local[kMaxWindows];
+    __shared__ int64_t shift_to[kMaxWindows];   // place in the sorted batch less place in the tile
+    __shared__ int32_t stage[kSortKeys * DIM];
+    __shared__ uint8_t window[kSortKeys];
+    const int64_t first = (int64_t)blockIdx.x * kSortKeys;
+    count[threadIdx.x] = 0;
+    __syncthreads();
+    int k[kEach][3], w[kEach];
+    uint32_t rank[kEach];
+#pragma unroll
+    for (int j = 0; j < kEach; ++j) {
+        const int64_t i = first + j * 256 + threadIdx.x;
+        w[j] = -1;
+        if (i < n) {
+            w[j] = window_of<DIM>(keys, i, mask, k[j]);
+            rank[j] = atomicAdd(count + w[j], 1u);
+        }
+    }
+    __syncthreads();
+    const uint32_t at = prefix_256(count[threadIdx.x]);
+    local[threadIdx.x] = at;
+    if (count[threadIdx.x])
+        shift_to[threadIdx.x] = (int64_t)atomicAdd(cursor + threadIdx.x, count[threadIdx.x]) - (int64_t)at;
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < kEach; ++j) {
+        if (w[j] < 0) continue;
+        const uint32_t place = local[w[j]] + rank[j];
+        window[place] = (uint8_t)w[j];
+#pragma unroll
+        for (int d = 0; d < DIM; ++d) stage[place * DIM + d] = k[j][d];
+    }
+    __syncthreads();
+    const int have = (int)min((int64_t)kSortKeys, n - first);
+    // word by word: a window's keys are a contiguous run here and there
+    for (int e = threadIdx.x; e < have * DIM; e += 256) {
+        const int place = e / DIM;
+        sorted[(shift_to[window[place]] + place) * DIM + (e - place * DIM)] = stage[e];
+    }
 }
 
 // ---- erase -----------------------------------------------------------------------
@@ -500,12 +608,12 @@ int ashb_map_status_async(ashb_map* m, uint32_t* status_out_host, void* stream) 
     return ASHB_OK;
 }
 
-int ashb_map_find(ashb_map* m, const int32_t* keys, int64_t n, int64_t* indices, uint8_t* masks,
-                  void* stream) {
+// indices null: only the masks are wanted (an eighth of what a lookup writes; 0.985 -> 0.956 ms for 50M keys in 2 GB)
+static int find_impl(ashb_map* m, const int32_t* keys, int64_t n, int64_t* indices, uint8_t* masks, void* stream) {
     ASHB_MAP_PROLOGUE(m);
     ASHB_REQUIRE(n >= 0, "negative count");
     if (n == 0) return ASHB_OK;
-    ASHB_REQUIRE(keys && indices && masks, "null buffer");
+    ASHB_REQUIRE(keys && masks, "null buffer");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (g_find_cooperative && m->key_dim <= 3) {
         const Table16 t = table16_of(m);
@@ -529,6 +637,16 @@ int ashb_map_find(ashb_map* m, const int32_t* keys, int64_t n, int64_t* indices,
     }
     ASHB_LAUNCH_CHECK();
     return ASHB_OK;
+}
+
+int ashb_map_find(ashb_map* m, const int32_t* keys, int64_t n, int64_t* indices, uint8_t* masks,
+                  void* stream) {
+    ASHB_REQUIRE(n <= 0 || indices != nullptr, "null buffer");
+    return find_impl(m, keys, n, indices, masks, stream);
+}
+
+int ashb_map_contains(ashb_map* m, const int32_t* keys, int64_t n, uint8_t* masks, void* stream) {
+    return find_impl(m, keys, n, nullptr, masks, stream);
 }
 
 int ashb_set_find_cooperative(int enable) {
@@ -558,6 +676,49 @@ int ashb_map_insert_keys(ashb_map* m, const int32_t* keys, int64_t n, void* stre
     ValueCtx v;
     std::memset(&v, 0, sizeof(v));
     return insert_impl(m, keys, n, v, stream);
+}
+
+// Worth it for tables of at least twice L2 (126 MB) and a key or more per line; beyond kMaxWindows the sorted runs get
+// short.
+static bool sorts_by_window(const ashb_map* m, int64_t n) {
+    return m->key_dim <= 3 && m->n_slots >= (uint64_t)8 << kWindowShift &&
+           m->n_slots <= (uint64_t)kMaxWindows << kWindowShift && (uint64_t)n >= m->n_slots / 8 && n < (int64_t)1 << 32;
+}
+
+int64_t ashb_map_insert_workspace(ashb_map* m, int64_t n) {
+    if (m == nullptr || m->slots == nullptr || n < 0 || !sorts_by_window(m, n)) return 0;
+    return 2 * kMaxWindows * (int64_t)sizeof(uint32_t) + n * m->key_dim * (int64_t)sizeof(int32_t);
+}
+
+int ashb_map_insert_keys_sorted(ashb_map* m, const int32_t* keys, int64_t n, void* workspace, int64_t workspace_bytes,
+                                void* stream) {
+    ASHB_MAP_PROLOGUE(m);
+    const int64_t need = ashb_map_insert_workspace(m, n);
+    ASHB_REQUIRE(need > 0, "not for this table and batch: ashb_map_insert_workspace says 0");
+    ASHB_REQUIRE(keys && workspace && ((uintptr_t)workspace & 15) == 0 && workspace_bytes >= need, "null or small workspace");
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    uint32_t* count = static_cast<uint32_t*>(workspace);
+    uint32_t* cursor = count + kMaxWindows;
+    int32_t* sorted = reinterpret_cast<int32_t*>(cursor + kMaxWindows);
+    const uint32_t mask = (uint32_t)(m->n_slots - 1);
+    Table16Lines t{table16_of(m)};
+    ValueCtx none;
+    std::memset(&none, 0, sizeof(none));
+    ASHB_CUDA_TRY(cudaMemsetAsync(count, 0, kMaxWindows * sizeof(uint32_t), st));
+    const unsigned tiles = blocks_for(n, kSortKeys), counters = wave_grid(n, 256, 8), grid = blocks_for(n, 256);
+#define ASHB_SORTED_INSERT(DIM)                                                                                       \
+    window_count_kernel<DIM><<<counters, 256, 0, st>>>(mask, keys, n, count);                                          \
+    window_start_kernel<<<1, 256, 0, st>>>(count, cursor);                                                            \
+    window_sort_kernel<DIM><<<tiles, 256, 0, st>>>(mask, keys, n, cursor, sorted);                                     \
+    insert_kernel<Table16Lines, DIM><<<grid, 256, 0, st>>>(t, sorted, n, m->heap, m->counter, (int32_t)m->capacity, none)
+    switch (m->key_dim) {
+        case 1: ASHB_SORTED_INSERT(1); break;
+        case 2: ASHB_SORTED_INSERT(2); break;
+        default: ASHB_SORTED_INSERT(3); break;
+    }
+#undef ASHB_SORTED_INSERT
+    ASHB_LAUNCH_CHECK();
+    return ASHB_OK;
 }
 
 int ashb_map_insert_values(ashb_map* m, const int32_t* keys, int64_t n, int n_values,
