@@ -89,6 +89,12 @@ int ashb_map_status_async(ashb_map* map, uint32_t* status_out_host, void* stream
 int ashb_map_find(ashb_map* map, const int32_t* keys_dev, int64_t n, int64_t* indices_dev,
                   uint8_t* masks_dev, void* stream);
 
+/* ashb_map_find, and the value rows of the keys: row i of dst_dev[j] (row_bytes[j] bytes) becomes row indices_dev[i]
+ * of src_dev[j], so row 0 for a miss.  n_values <= 16; src_dev / dst_dev / row_bytes are HOST arrays. */
+int ashb_map_find_values(ashb_map* map, const int32_t* keys_dev, int64_t n, int64_t* indices_dev, uint8_t* masks_dev,
+                         int n_values, const void* const* src_dev, void* const* dst_dev, const int64_t* row_bytes,
+                         void* stream);
+
 /* The masks of ashb_map_find alone. */
 int ashb_map_contains(ashb_map* map, const int32_t* keys_dev, int64_t n, uint8_t* masks_dev, void* stream);
 

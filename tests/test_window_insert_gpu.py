@@ -73,3 +73,50 @@ def test_contains_is_the_masks_of_find(capacity, dim):
             assert torch.equal(m.find(keys), m.engine.find(keys)[1])
         finally:
             __ash.set_find_cooperative(False)
+
+
+@pytest.mark.parametrize("capacity", [700, 3_000_000])      # without and with the occupancy bits asked first
+@pytest.mark.parametrize("dim", [1, 3, 4])
+def test_find_with_values_is_find_and_indexing(capacity, dim):
+    import ash
+
+    m = ash.HashMap(dim, {"a": 1, "b": 3, "c": 16, "wide": 40}, capacity, DEV)
+    g = torch.Generator(device=DEV).manual_seed(dim)
+    keys = torch.randint(-9, 9, (701, dim), generator=g, device=DEV, dtype=torch.int32)
+    values = {k: torch.randn(701, w, generator=g, device=DEV) for k, w in m.value_dims.items()}
+    m.insert(keys[:600].contiguous(), {k: v[:600].contiguous() for k, v in values.items()})
+    for n in (701, 1, 0):
+        if n == 0:
+            with pytest.warns(UserWarning):
+                masks, idx, got = m.find(keys[:0], return_values=True)
+        else:
+            masks, idx, got = m.find(keys[:n], return_values=True)
+        assert got.keys() == values.keys() and got["b"].shape == (n, 3)
+        ref_idx, ref_masks = (idx, masks) if n == 0 else m.engine.find(keys[:n])
+        assert torch.equal(idx, ref_idx) and torch.equal(masks, ref_masks)
+        for k, v in m.values.items():
+            assert torch.equal(got[k], v[ref_idx]), k
+    backend = m.engine.backend
+    odd = {"bytes": torch.randint(0, 255, (capacity, 3), device=DEV, dtype=torch.uint8), "d": torch.randn(capacity, 2, device=DEV).double(),
+           "flat": torch.arange(capacity, device=DEV, dtype=torch.int16)}
+    idx, masks, got = backend.find_values(keys, odd)
+    for k, v in odd.items():
+        assert got[k].dtype == v.dtype and torch.equal(got[k], v[idx]), k
+    assert backend.find_values(keys, {"wide": m.values["wide"]}) is None
+    assert backend.find_values(keys, {"p": torch.zeros(capacity, 1, device=DEV, requires_grad=True)}) is None
+
+
+@pytest.mark.parametrize("capacity", [1, 5, 1000, 1_000_000, 3_000_000])
+@pytest.mark.parametrize("dim", [2, 4])
+def test_clear_leaves_an_empty_map(capacity, dim):
+    import ash
+
+    m = ash.HashSet(dim, capacity, DEV)
+    n = min(capacity, 2000)
+    keys = torch.arange(n * dim, device=DEV, dtype=torch.int32).view(n, dim)
+    for _ in range(2):
+        m.insert(keys)
+        assert m.size() == n and bool(m.find(keys).all())
+        m.clear()
+        assert m.size() == 0 and not bool(m.find(keys).any()) and m.keys().shape[0] == 0
+        assert torch.equal(m.engine._heap, torch.arange(capacity, device=DEV, dtype=torch.int32))

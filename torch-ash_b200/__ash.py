@@ -39,6 +39,7 @@ _lib.ashb_map_size.argtypes = [_vp, _vp, _c.POINTER(_i64)]
 _lib.ashb_map_status.argtypes = [_vp, _vp, _c.POINTER(_c.c_uint32)]
 _lib.ashb_map_status_async.argtypes = [_vp, _vp, _vp]
 _lib.ashb_map_find.argtypes = [_vp, _vp, _i64, _vp, _vp, _vp]
+_lib.ashb_map_find_values.argtypes = [_vp, _vp, _i64, _vp, _vp, _int, _vp, _vp, _vp, _vp]
 _lib.ashb_map_contains.argtypes = [_vp, _vp, _i64, _vp, _vp]
 _lib.ashb_map_insert_keys.argtypes = [_vp, _vp, _i64, _vp]
 _lib.ashb_map_insert_workspace.argtypes = [_vp, _i64]
@@ -266,6 +267,29 @@ class HashMap:
         masks = torch.empty(n, dtype=torch.bool, device=self._device)
         _check(_lib.ashb_map_find(self._h, keys.data_ptr(), n, indices.data_ptr(), masks.data_ptr(), _stream(self._device)))
         return indices, masks
+
+    def find_values(self, keys: torch.Tensor, tables: dict):
+        """``(indices, masks, {name: tables[name][indices]})`` in one launch (not in the reference), or None where the
+        gathers are better left to indexing: wide rows, which a warp reads side by side, more tables than a launch
+        takes, and tables that autograd records."""
+        if len(tables) > 16:
+            return None
+        for v in tables.values():
+            if not (v.device == self._device and v.is_contiguous() and v.dim() >= 1 and 0 < v.numel() and v.shape[0] == self._capacity
+                    and v.numel() // v.shape[0] * v.element_size() <= 64) or (v.requires_grad and torch.is_grad_enabled()):
+                return None
+        keys = self._keys(keys)
+        n, k = keys.shape[0], len(tables)
+        indices = torch.empty(n, dtype=torch.int64, device=self._device)
+        masks = torch.empty(n, dtype=torch.bool, device=self._device)
+        out = {name: torch.empty((n, *v.shape[1:]), dtype=v.dtype, device=self._device) for name, v in tables.items()}
+        src, dst, row = (_vp * max(k, 1))(), (_vp * max(k, 1))(), (_i64 * max(k, 1))()
+        for j, (name, v) in enumerate(tables.items()):
+            src[j], dst[j] = v.data_ptr(), out[name].data_ptr()
+            row[j] = v.numel() // v.shape[0] * v.element_size()
+        _check(_lib.ashb_map_find_values(self._h, keys.data_ptr(), n, indices.data_ptr(), masks.data_ptr(), k, src, dst, row,
+                                         _stream(self._device)))
+        return indices, masks, out
 
     def contains(self, keys: torch.Tensor) -> torch.Tensor:
         """The masks of ``find`` alone (not in the reference)."""

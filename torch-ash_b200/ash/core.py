@@ -139,6 +139,15 @@ class ASHEngine(nn.Module):
             )
         return self.backend.find(k)
 
+    def find_values(self, keys: torch.Tensor, tables: Dict[str, torch.Tensor]):
+        """``(indices, masks, {name: tables[name][indices]})``."""
+        if keys.shape[0] > 0 and hasattr(self.backend, "find_values"):
+            found = self.backend.find_values(self._prepare(keys), tables)
+            if found is not None:
+                return found
+        indices, masks = self.find(keys)
+        return indices, masks, {name: v[indices] for name, v in tables.items()}
+
     def contains(self, keys: torch.Tensor) -> torch.Tensor:
         """The masks of ``find`` without its indices."""
         if not hasattr(self.backend, "contains"):

@@ -70,12 +70,15 @@ class HashMap(ASHModule):
     def find(self, keys: torch.Tensor, return_indices: bool = True, return_values: bool = False):
         """(masks[, indices][, values]) -- masks first, as ash/hashmap.py:72-95."""
         assert return_indices or return_values, "Must return at least one of indices or values"
-        indices, masks = self.engine.find(keys)
+        if return_values:
+            indices, masks, values = self.engine.find_values(keys, self.values)
+        else:
+            indices, masks = self.engine.find(keys)
         ans = (masks,)
         if return_indices:
             ans += (indices,)
         if return_values:
-            ans += (self._gather(indices),)
+            ans += (self.reinterpret_value_dict(values),)
         return ans
 
     def erase(self, keys: torch.Tensor) -> None:

@@ -27,14 +27,49 @@
 
 namespace ashb {
 
+// ---- value rows ------------------------------------------------------------------
+struct ValueCtx {
+    int n;
+    const char* src[kMaxValues];
+    char* dst[kMaxValues];
+    long long row_bytes[kMaxValues];
+    int word[kMaxValues];  // widest power-of-two copy word (<= 16) both sides allow
+};
+
+__device__ __forceinline__ void copy_row(const char* __restrict__ src, char* __restrict__ dst,
+                                         long long bytes, int word) {
+    switch (word) {
+        case 16:
+            for (long long b = 0; b < bytes; b += 16)
+                *reinterpret_cast<int4*>(dst + b) = *reinterpret_cast<const int4*>(src + b);
+            break;
+        case 8:
+            for (long long b = 0; b < bytes; b += 8)
+                *reinterpret_cast<int2*>(dst + b) = *reinterpret_cast<const int2*>(src + b);
+            break;
+        case 4:
+            for (long long b = 0; b < bytes; b += 4)
+                *reinterpret_cast<int*>(dst + b) = *reinterpret_cast<const int*>(src + b);
+            break;
+        case 2:
+            for (long long b = 0; b < bytes; b += 2)
+                *reinterpret_cast<short*>(dst + b) = *reinterpret_cast<const short*>(src + b);
+            break;
+        default:
+            for (long long b = 0; b < bytes; ++b) dst[b] = src[b];
+    }
+}
+
 // ---- find ----------------------------------------------------------------------
 // FILTER (16-byte slots only): the one-bit-per-slot occupancy map is consulted first.  A key whose
 // home slot never held anything is absent, and the map (1/128 of the table) sits in L2 when the
 // table itself is far beyond it, so such a miss costs no DRAM access at all.
-template <class Table, int DIM, bool FILTER = false>
+// GATHER: the value rows of the keys are copied out too (row 0 for a miss, as indexing with its index 0 does): one
+// launch where a gather per value followed, and the indices need not be read back.
+template <class Table, int DIM, bool FILTER, bool GATHER>
 __global__ void __launch_bounds__(256) find_kernel(Table t, const int32_t* __restrict__ keys, int64_t n,
                                                    int64_t* __restrict__ indices,
-                                                   uint8_t* __restrict__ masks) {
+                                                   uint8_t* __restrict__ masks, ValueCtx vctx) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     int k0, k1, k2, k3;
@@ -70,6 +105,11 @@ __global__ void __launch_bounds__(256) find_kernel(Table t, const int32_t* __res
     } else {
         if (indices) indices[i] = found >= 0 ? (int64_t)found : 0;
         masks[i] = (uint8_t)(found >= 0);
+    }
+    if constexpr (GATHER) {
+        for (int j = 0; j < vctx.n; ++j)
+            copy_row(vctx.src[j] + max(found, 0) * vctx.row_bytes[j], vctx.dst[j] + i * vctx.row_bytes[j], vctx.row_bytes[j],
+                     vctx.word[j]);
     }
 }
 
@@ -123,38 +163,6 @@ __global__ void __launch_bounds__(256) find_coop_kernel(Table16 t, const int32_t
 }
 
 // ---- insert ----------------------------------------------------------------------
-struct ValueCtx {
-    int n;
-    const char* src[kMaxValues];
-    char* dst[kMaxValues];
-    long long row_bytes[kMaxValues];
-    int word[kMaxValues];  // widest power-of-two copy word (<= 16) both sides allow
-};
-
-__device__ __forceinline__ void copy_row(const char* __restrict__ src, char* __restrict__ dst,
-                                         long long bytes, int word) {
-    switch (word) {
-        case 16:
-            for (long long b = 0; b < bytes; b += 16)
-                *reinterpret_cast<int4*>(dst + b) = *reinterpret_cast<const int4*>(src + b);
-            break;
-        case 8:
-            for (long long b = 0; b < bytes; b += 8)
-                *reinterpret_cast<int2*>(dst + b) = *reinterpret_cast<const int2*>(src + b);
-            break;
-        case 4:
-            for (long long b = 0; b < bytes; b += 4)
-                *reinterpret_cast<int*>(dst + b) = *reinterpret_cast<const int*>(src + b);
-            break;
-        case 2:
-            for (long long b = 0; b < bytes; b += 2)
-                *reinterpret_cast<short*>(dst + b) = *reinterpret_cast<const short*>(src + b);
-            break;
-        default:
-            for (long long b = 0; b < bytes; ++b) dst[b] = src[b];
-    }
-}
-
 template <class Table, int DIM>
 __global__ void __launch_bounds__(256) insert_kernel(Table t, const int32_t* __restrict__ keys, int64_t n,
                                                      int32_t* __restrict__ heap, int32_t* counter,
@@ -374,6 +382,18 @@ __global__ void __launch_bounds__(256) rehash_kernel(Table dst, Table src) {
 
 __global__ void set_counter_kernel(int32_t* counter, int32_t v) { *counter = v; }
 
+// A small map emptied by one launch instead of three fills and the one below (kFilterMinBytes is the line: beyond it a
+// fill runs at memory speed).
+__global__ void __launch_bounds__(256) clear_map_kernel(uint4* __restrict__ slots, int64_t n_slot16, uint32_t* __restrict__ occupied,
+                                                        int64_t n_occupied, int32_t* __restrict__ heap, int64_t capacity,
+                                                        int32_t* counter) {
+    const int64_t first = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, step = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t i = first; i < n_slot16; i += step) slots[i] = make_uint4(~0u, ~0u, ~0u, ~0u);
+    for (int64_t i = first; i < n_occupied; i += step) occupied[i] = 0u;
+    for (int64_t i = first; i < capacity; i += step) heap[i] = (int32_t)i;
+    if (first == 0) *counter = 0;
+}
+
 __global__ void reset_heap_kernel(int32_t* __restrict__ heap, int64_t capacity) {
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < capacity;
          i += (int64_t)gridDim.x * blockDim.x)
@@ -498,6 +518,49 @@ constexpr size_t kFilterMinBytes = (size_t)64 << 20;
 
 static size_t occupied_bytes(uint64_t n_slots) { return (size_t)(n_slots / 8 < 4 ? 4 : n_slots / 8); }
 
+// The widest copy word that source, destination and row length allow.
+static int value_ctx(int n_values, const void* const* src, void* const* dst, const int64_t* row_bytes, ValueCtx* out) {
+    ASHB_REQUIRE(n_values >= 0 && n_values <= kMaxValues, "n_values %d not in 0..%d", n_values, kMaxValues);
+    ASHB_REQUIRE(n_values == 0 || (src && dst && row_bytes), "null value tables");
+    std::memset(out, 0, sizeof(*out));
+    out->n = n_values;
+    for (int j = 0; j < n_values; ++j) {
+        ASHB_REQUIRE(src[j] && dst[j] && row_bytes[j] > 0, "value %d: null pointer or empty row", j);
+        out->src[j] = static_cast<const char*>(src[j]);
+        out->dst[j] = static_cast<char*>(dst[j]);
+        out->row_bytes[j] = row_bytes[j];
+        int w = 16;
+        const uintptr_t bits = (uintptr_t)src[j] | (uintptr_t)dst[j] | (uintptr_t)row_bytes[j];
+        while (w > 1 && (bits & (uintptr_t)(w - 1))) w >>= 1;
+        out->word[j] = w;
+    }
+    return ASHB_OK;
+}
+
+template <bool GATHER>
+static void launch_find(ashb_map* m, const int32_t* keys, int64_t n, int64_t* indices, uint8_t* masks, const ValueCtx& v,
+                        cudaStream_t st) {
+    const unsigned grid = blocks_for(n, 256);
+    const Table16 t = table16_of(m);
+    if (m->key_dim == 4) {
+        const Table32 t4{static_cast<Slot32*>(m->slots), (uint32_t)(m->n_slots - 1), m->status};
+        find_kernel<Table32, 4, false, GATHER><<<grid, 256, 0, st>>>(t4, keys, n, indices, masks, v);
+    } else if (m->occupied != nullptr &&
+               (g_find_filter > 0 || (g_find_filter < 0 && m->n_slots * m->slot_bytes >= kFilterMinBytes))) {
+        switch (m->key_dim) {
+            case 1: find_kernel<Table16, 1, true, GATHER><<<grid, 256, 0, st>>>(t, keys, n, indices, masks, v); break;
+            case 2: find_kernel<Table16, 2, true, GATHER><<<grid, 256, 0, st>>>(t, keys, n, indices, masks, v); break;
+            default: find_kernel<Table16, 3, true, GATHER><<<grid, 256, 0, st>>>(t, keys, n, indices, masks, v); break;
+        }
+    } else {
+        switch (m->key_dim) {
+            case 1: find_kernel<Table16, 1, false, GATHER><<<grid, 256, 0, st>>>(t, keys, n, indices, masks, v); break;
+            case 2: find_kernel<Table16, 2, false, GATHER><<<grid, 256, 0, st>>>(t, keys, n, indices, masks, v); break;
+            default: find_kernel<Table16, 3, false, GATHER><<<grid, 256, 0, st>>>(t, keys, n, indices, masks, v); break;
+        }
+    }
+}
+
 extern "C" {
 
 int ashb_map_create(int key_dim, int64_t capacity, int32_t* heap_dev, int device, ashb_map** out) {
@@ -568,6 +631,14 @@ int ashb_map_destroy(ashb_map* m) {
 int ashb_map_clear(ashb_map* m, void* stream) {
     ASHB_MAP_PROLOGUE(m);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
+    if (m->n_slots * m->slot_bytes < kFilterMinBytes) {
+        const int64_t n_slot16 = (int64_t)(m->n_slots * m->slot_bytes / 16);
+        clear_map_kernel<<<wave_grid(n_slot16, 256, 8), 256, 0, st>>>(
+                static_cast<uint4*>(m->slots), n_slot16, m->occupied,
+                m->occupied ? (int64_t)(occupied_bytes(m->n_slots) / 4) : 0, m->heap, m->capacity, m->counter);
+        ASHB_LAUNCH_CHECK();
+        return ASHB_OK;
+    }
     ASHB_CUDA_TRY(cudaMemsetAsync(m->slots, 0xFF, m->n_slots * m->slot_bytes, st));
     if (m->occupied) ASHB_CUDA_TRY(cudaMemsetAsync(m->occupied, 0, occupied_bytes(m->n_slots), st));
     ASHB_CUDA_TRY(cudaMemsetAsync(m->counter, 0, sizeof(int32_t), st));
@@ -623,17 +694,10 @@ static int find_impl(ashb_map* m, const int32_t* keys, int64_t n, int64_t* indic
             case 2: find_coop_kernel<2><<<grid, 256, 0, st>>>(t, keys, n, indices, masks); break;
             default: find_coop_kernel<3><<<grid, 256, 0, st>>>(t, keys, n, indices, masks); break;
         }
-    } else if (m->occupied != nullptr &&
-               (g_find_filter > 0 || (g_find_filter < 0 && m->n_slots * m->slot_bytes >= kFilterMinBytes))) {
-        const Table16 t = table16_of(m);
-        const unsigned grid = blocks_for(n, 256);
-        switch (m->key_dim) {
-            case 1: find_kernel<Table16, 1, true><<<grid, 256, 0, st>>>(t, keys, n, indices, masks); break;
-            case 2: find_kernel<Table16, 2, true><<<grid, 256, 0, st>>>(t, keys, n, indices, masks); break;
-            default: find_kernel<Table16, 3, true><<<grid, 256, 0, st>>>(t, keys, n, indices, masks); break;
-        }
     } else {
-        ASHB_DIM_LAUNCH(find_kernel, m, blocks_for(n, 256), 256, st, keys, n, indices, masks);
+        ValueCtx none;
+        std::memset(&none, 0, sizeof(none));
+        launch_find<false>(m, keys, n, indices, masks, none, st);
     }
     ASHB_LAUNCH_CHECK();
     return ASHB_OK;
@@ -647,6 +711,19 @@ int ashb_map_find(ashb_map* m, const int32_t* keys, int64_t n, int64_t* indices,
 
 int ashb_map_contains(ashb_map* m, const int32_t* keys, int64_t n, uint8_t* masks, void* stream) {
     return find_impl(m, keys, n, nullptr, masks, stream);
+}
+
+int ashb_map_find_values(ashb_map* m, const int32_t* keys, int64_t n, int64_t* indices, uint8_t* masks, int n_values,
+                         const void* const* src, void* const* dst, const int64_t* row_bytes, void* stream) {
+    ASHB_MAP_PROLOGUE(m);
+    ASHB_REQUIRE(n >= 0, "negative count");
+    if (n == 0) return ASHB_OK;
+    ASHB_REQUIRE(keys && indices && masks, "null buffer");
+    ValueCtx v;
+    if (int rc = value_ctx(n_values, src, dst, row_bytes, &v)) return rc;
+    launch_find<true>(m, keys, n, indices, masks, v, static_cast<cudaStream_t>(stream));
+    ASHB_LAUNCH_CHECK();
+    return ASHB_OK;
 }
 
 int ashb_set_find_cooperative(int enable) {
@@ -724,21 +801,8 @@ int ashb_map_insert_keys_sorted(ashb_map* m, const int32_t* keys, int64_t n, voi
 int ashb_map_insert_values(ashb_map* m, const int32_t* keys, int64_t n, int n_values,
                            const void* const* src, void* const* dst, const int64_t* row_bytes,
                            void* stream) {
-    ASHB_REQUIRE(n_values >= 0 && n_values <= kMaxValues, "n_values %d not in 0..%d", n_values, kMaxValues);
-    ASHB_REQUIRE(n_values == 0 || (src && dst && row_bytes), "null value tables");
     ValueCtx v;
-    std::memset(&v, 0, sizeof(v));
-    v.n = n_values;
-    for (int j = 0; j < n_values; ++j) {
-        ASHB_REQUIRE(src[j] && dst[j] && row_bytes[j] > 0, "value %d: null pointer or empty row", j);
-        v.src[j] = static_cast<const char*>(src[j]);
-        v.dst[j] = static_cast<char*>(dst[j]);
-        v.row_bytes[j] = row_bytes[j];
-        int w = 16;
-        const uintptr_t bits = (uintptr_t)src[j] | (uintptr_t)dst[j] | (uintptr_t)row_bytes[j];
-        while (w > 1 && (bits & (uintptr_t)(w - 1))) w >>= 1;
-        v.word[j] = w;
-    }
+    if (int rc = value_ctx(n_values, src, dst, row_bytes, &v)) return rc;
     return insert_impl(m, keys, n, v, stream);
 }
 
