@@ -179,8 +179,13 @@ def set_find_cooperative(enable: bool) -> None:
     _check(_lib.ashb_set_find_cooperative(int(bool(enable))))
 
 
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
 def _stream(device: torch.device) -> int:
-    return torch.cuda.current_stream(device).cuda_stream
+    if _raw_stream is None or device.index is None:
+        return torch.cuda.current_stream(device).cuda_stream
+    return _raw_stream(device.index)   # without building a Stream object: several per cent of a small call
 
 
 def _cuda(t: torch.Tensor, name: str, dtype=None) -> torch.Tensor:

@@ -27,6 +27,13 @@ def _host_matrix(m) -> np.ndarray:
     return np.asarray(m, dtype=np.float64)
 
 
+def _scale_depth_(datum) -> None:
+    """``datum.depth *= datum.depth_scale``, without a launch where the depth is in metres already."""
+    scale = datum.depth_scale
+    if not (type(scale) in (int, float) and scale == 1 and datum.depth.is_floating_point()):
+        datum.depth *= scale
+
+
 class TSDFFusion:
     def __init__(self, grid: Union[UnBoundedSparseDenseGrid, BoundedSparseDenseGrid], dilation: int):
         assert grid.embedding_dim >= 5, "embeddings must hold sdf(1) + rgb(3) + weight(1)"
@@ -57,7 +64,7 @@ class TSDFFusion:
         world -> camera, rgb (H, W, 3); as demo/rgbd_fusion.py:199-254 (``datum.depth`` is scaled to
         metres in place there too).  ``counter``: optional int64 device tensor incremented by the
         number of blocks fused."""
-        datum.depth *= datum.depth_scale
+        _scale_depth_(datum)
         depth = datum.depth
         K = _host_matrix(datum.intrinsic)
         E = _host_matrix(datum.extrinsic)
@@ -118,7 +125,7 @@ class TSDFFusion:
             return
         depths, colors = [], []
         for f in frames:
-            f.depth *= f.depth_scale
+            _scale_depth_(f)
             depths.append(f.depth if f.depth.dtype == torch.float32 and f.depth.is_contiguous() else f.depth.float().contiguous())
             colors.append(f.rgb if f.rgb.dtype == torch.float32 and f.rgb.is_contiguous() else f.rgb.float().contiguous())
         K = np.stack([_host_matrix(f.intrinsic) for f in frames])

@@ -71,6 +71,7 @@ class SparseDenseGrid(ASHModule):
         self.grad_mode = "dense"
         self._lut32 = None
         self._lut32_source = None
+        self._gaussian_window = None   # ((size, sigma, channels, device), factors) of the last gaussian_filter_
         self._own_transform = self.transform_world_to_cell
 
     def _allocate_embeddings(self) -> torch.Tensor:
@@ -344,10 +345,16 @@ class SparseDenseGrid(ASHModule):
         emb = self.embeddings
         if (self.separable_gaussian and self.tiled_convolution and emb.is_cuda and emb.dtype == torch.float32
                 and 1 <= radius <= self.grid_dim and hasattr(backend, "filter_separable_")):
-            k1 = self._gaussian_weights_1d(size, sigma)
-            k1 = k1 / k1.sum()                       # (k1 (x) k1 (x) k1) / sum = product of the normalised factors
-            w1 = torch.from_numpy(k1).float().view(1, size, 1).repeat(3, 1, channels).contiguous()
-            backend.filter_separable_(emb.data, w1.to(emb.device), self.engine.backend, self.grid_dim, radius)
+            # the window of the last call is kept: laying it out costs a host copy that waits for the device
+            window = (size, sigma, channels, emb.device)
+            if self._gaussian_window is None or self._gaussian_window[0] != window:
+                k1 = self._gaussian_weights_1d(size, sigma)
+                k1 = k1 / k1.sum()                   # (k1 (x) k1 (x) k1) / sum = product of the normalised factors
+                w1 = torch.from_numpy(k1).float().view(1, size, 1).repeat(3, 1, channels).contiguous()
+                self._gaussian_window = (window, w1.to(emb.device))
+            w1 = self._gaussian_window[1]
+            w1.record_stream(torch.cuda.current_stream(emb.device))   # it may be replaced while another stream reads it
+            backend.filter_separable_(emb.data, w1, self.engine.backend, self.grid_dim, radius)
             return
         weights = self._gaussian_weights(size, sigma).view(size, size, size, 1).repeat(1, 1, 1, channels)
         self.embeddings.copy_(self.convolution(self.embeddings, weights.to(self.embeddings.device)))
