@@ -7,54 +7,63 @@ pytestmark = pytest.mark.gpu
 DEV = torch.device("cuda:0")
 
 
-def _unique(keys):
-    return torch.unique(keys, dim=0)
+def _packed(keys):
+    p = torch.zeros(keys.shape[0], dtype=torch.int64, device=DEV)
+    for d in range(keys.shape[1]):
+        p = p * 2**20 + keys[:, d].long() + 2**19 if keys.shape[1] > 1 else keys[:, 0].long()
+    return p
 
 
-@pytest.mark.parametrize("dim,n,spread", [(3, 2_100_001, 2**18), (2, 2_097_152, 2**12), (1, 3_000_001, 2**30), (3, 4_000_000, 40)])
+CAPACITY = 16_777_217     # 2^26 slots: the smallest table that is sorted for, from a key per line on
+
+
+@pytest.mark.parametrize("dim,n,spread", [(3, 8_388_609, 2**18), (2, 8_388_608, 2**12), (1, 12_000_001, 2**30), (3, 9_000_000, 40)])
 def test_sorted_insert(dim, n, spread):
     import __ash
     import ash
 
-    m = ash.HashSet(dim, 5_000_000, DEV)      # 2^24 slots: the smallest table that is sorted for
+    m = ash.HashSet(dim, CAPACITY, DEV)
     ws = __ash._lib.ashb_map_insert_workspace
     h = m.engine.backend._h
-    assert ws(h, n) > 0 and ws(h, 2_097_151) == 0
+    assert ws(h, n) > 0 and ws(h, 8_388_607) == 0
     g = torch.Generator(device=DEV).manual_seed(n)
     keys = torch.randint(-spread, spread, (n, dim), generator=g, device=DEV, dtype=torch.int32)
     keys[n // 2:n // 2 + 1000] = keys[:1000]                   # some twice, and (spread 40) all many times over
     present = keys[: n // 10].contiguous()
     m.insert(present)                                         # a small batch: in its own order
-    first = dict(zip(("masks", "rows"), m.engine.find(present)[::-1]))
+    rows_before, masks_before = m.engine.find(present)
     m.insert(keys)
-    want = _unique(keys)
+    order = torch.sort(_packed(keys), stable=True)
+    firsts = torch.ones(n, dtype=torch.bool, device=DEV)
+    firsts[1:] = order.values[1:] != order.values[:-1]
+    want = keys[order.indices[firsts]].contiguous()           # each distinct key once
     got, rows = m.engine.items()
-    assert torch.equal(_unique(got), want) and got.shape == want.shape
+    assert torch.equal(torch.sort(_packed(got)).values, _packed(want))
     assert torch.equal(torch.sort(rows).values, torch.arange(want.shape[0], device=DEV))
     rows_now, masks = m.engine.find(present)
-    assert bool(masks.all()) and bool(first["masks"].all()) and torch.equal(rows_now, first["rows"])   # kept their rows
+    assert bool(masks.all()) and bool(masks_before.all()) and torch.equal(rows_now, rows_before)   # kept their rows
     assert bool(m.find(keys).all())
-    absent = keys.clone()
-    absent[:, 0] += 2 * spread if spread < 2**20 else 0
     if spread < 2**20:
+        absent = keys.clone()
+        absent[:, 0] += 2 * spread
         assert not bool(m.find(absent).any())
     m.erase(want[::2].contiguous())
     mask = m.find(want)
     assert not bool(mask[::2].any()) and bool(mask[1::2].all())
     m.insert(keys)                                            # over tombstones
     got, rows = m.engine.items()
-    assert got.shape == want.shape and torch.unique(rows).numel() == want.shape[0]
+    assert torch.equal(torch.sort(_packed(got)).values, _packed(want)) and torch.unique(rows).numel() == want.shape[0]
 
 
 def test_sorted_insert_beyond_capacity_reports_and_keeps_what_fits():
     import ash
 
-    m = ash.HashSet(3, 4_300_000, DEV)
+    m = ash.HashSet(3, CAPACITY, DEV)
     g = torch.Generator(device=DEV).manual_seed(3)
-    keys = torch.randint(-2**18, 2**18, (5_000_000, 3), generator=g, device=DEV, dtype=torch.int32)
+    keys = torch.randint(-2**18, 2**18, (18_000_000, 3), generator=g, device=DEV, dtype=torch.int32)
     with pytest.warns(UserWarning):
         m.insert(keys)
-    assert m.size() == 4_300_000 and int(m.find(keys).sum()) >= 4_300_000
+    assert m.size() == CAPACITY and int(m.find(keys).sum()) >= CAPACITY
 
 
 @pytest.mark.parametrize("capacity", [1000, 5_000_000])

@@ -187,9 +187,12 @@ __global__ void __launch_bounds__(256) insert_kernel(Table t, const int32_t* __r
 // ---- insert of a large batch into a large table, window by window ----------------------------------
 // A batch of several keys per 128-byte line of the table, inserted in its own order, fetches a line from
 // DRAM for every key of it and writes it back for most.  Sorted first into windows of the table that stay
-// in L2 (2^kWindowShift of them, 32 MB), each line comes and goes once: two streams over the keys (count 0.10,
-// sort 0.38 ms) buy that.  50M keys, half of them twice, into 2 GB: 2.29 -> 2.01 ms.
-constexpr uint32_t kWindowShift = 21;        // slots per window
+// in L2 (2^kWindowShift of them, 64 MB), each line comes and goes once: two streams over the keys (count 0.10,
+// sort 0.38 ms) buy that.  50M keys, half of them twice, into 2 GB: 2.29 -> 1.94 ms.  The insertion itself then
+// takes 1.46 ms (16 MB windows: 1.58, 32 MB: 1.52 -- more keys after the same line at once; fetching 64 bytes
+// instead of the line: 0.1 more; four keys of a thread in flight: 1.47): what is left is a 16-byte compare-and-swap,
+// an occupancy bit and a store per new key.
+constexpr uint32_t kWindowShift = 22;        // slots per window
 constexpr int kMaxWindows = 256;
 constexpr int kSortKeys = 2048;              // keys of a CTA: 8 per thread
 
@@ -755,10 +758,11 @@ int ashb_map_insert_keys(ashb_map* m, const int32_t* keys, int64_t n, void* stre
     return insert_impl(m, keys, n, v, stream);
 }
 
-// Worth it for tables of at least twice L2 (126 MB) and a key or more per line; beyond kMaxWindows the sorted runs get
-// short.
+// Worth it for tables of 1 GB and more and a key or more per line: 8.4M to 50M keys into 1 and 2 GB take 0.76 to 0.86 of
+// the time, but into 512 MB 1.06 to 0.90 and into 256 MB 1.08 to 1.35, because part of those stays in L2 (126 MB)
+// as it is.  Beyond kMaxWindows the sorted runs get short.
 static bool sorts_by_window(const ashb_map* m, int64_t n) {
-    return m->key_dim <= 3 && m->n_slots >= (uint64_t)8 << kWindowShift &&
+    return m->key_dim <= 3 && m->n_slots >= (uint64_t)1 << 26 &&
            m->n_slots <= (uint64_t)kMaxWindows << kWindowShift && (uint64_t)n >= m->n_slots / 8 && n < (int64_t)1 << 32;
 }
 

@@ -508,12 +508,13 @@ int ashb_grid_spatial_init(ashb_map* m, const float* points, int64_t n, double c
     return ASHB_OK;
 }
 
-int ashb_tsdf_integrate(void* embeddings, int64_t n_emb, int G, int64_t D, const int32_t* grid_coords,
-                        const uint32_t* touched, uint32_t stamp, const float* depth, const float* color, int H,
-                        int W, const float* intrinsic, const float* world_to_cam, float depth_max,
-                        double cell_size, const float* origin, float trunc, int sdf_channel, int rgb_channel,
-                        int weight_channel, unsigned long long* n_integrated_dev, const int32_t* touched_list,
-                        const int32_t* touched_count, void* stream) {
+// ctas_per_sm: most CTAs of a work list's pass that an SM takes.
+static int integrate_impl(void* embeddings, int64_t n_emb, int G, int64_t D, const int32_t* grid_coords,
+                          const uint32_t* touched, uint32_t stamp, const float* depth, const float* color, int H,
+                          int W, const float* intrinsic, const float* world_to_cam, float depth_max,
+                          double cell_size, const float* origin, float trunc, int sdf_channel, int rgb_channel,
+                          int weight_channel, unsigned long long* n_integrated_dev, const int32_t* touched_list,
+                          const int32_t* touched_count, int ctas_per_sm, void* stream) {
     ASHB_REQUIRE((touched_list == nullptr) == (touched_count == nullptr), "pass both the list and its counter, or neither");
     ASHB_REQUIRE(embeddings && grid_coords && touched && depth && color && intrinsic && world_to_cam && origin,
                  "null buffer");
@@ -537,10 +538,6 @@ int ashb_tsdf_integrate(void* embeddings, int64_t n_emb, int G, int64_t D, const
     const bool bulk = touched_list != nullptr && smem % 16 == 0 && ((uintptr_t)embeddings & 15) == 0 && 2 * smem <= 96 * 1024;
     // with a work list: exactly the CTAs that are resident at once walk it (more would queue behind them
     // as a partly filled second wave); without: one CTA per row
-    // The pass is bound by arithmetic (seven IEEE divisions per cell), which half of an SM's thread slots
-    // already saturate; the other half is left to the allocation pass of the NEXT frame, which runs
-    // beside it on a second stream when a sequence is fused (ashb_tsdf_fuse_frames).
-    constexpr int kIntegrateCtasPerSm = 4;
 #define ASHB_TSDF_LAUNCH(DD)                                                                               \
     case DD: {                                                                                             \
         const size_t dyn = bulk ? 2 * smem : smem;                                                         \
@@ -549,7 +546,7 @@ int ashb_tsdf_integrate(void* embeddings, int64_t n_emb, int G, int64_t D, const
             ASHB_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn)); \
         int per_sm = 0;                                                                                    \
         ASHB_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, 256, dyn));               \
-        if (per_sm > kIntegrateCtasPerSm) per_sm = kIntegrateCtasPerSm;                                    \
+        if (per_sm > ctas_per_sm) per_sm = ctas_per_sm;                                                    \
         const int64_t resident = (int64_t)sm_count() * (per_sm > 0 ? per_sm : 1);                          \
         const unsigned launch_ctas = touched_list ? (unsigned)(n_emb < resident ? n_emb : resident) : (unsigned)n_emb; \
         if (bulk)                                                                                          \
@@ -577,6 +574,23 @@ int ashb_tsdf_integrate(void* embeddings, int64_t n_emb, int G, int64_t D, const
 #undef ASHB_TSDF_LAUNCH
     ASHB_LAUNCH_CHECK();
     return ASHB_OK;
+}
+
+// The pass is bound by arithmetic (seven IEEE divisions per cell).  A frame on its own takes all of an SM's thread
+// slots (3,500 blocks: 23.7 us, 26.4 with half of them); where a sequence is fused the allocation pass of the NEXT
+// frame runs beside it on a second stream (ashb_tsdf_fuse_frames) and needs the other half (100 frames: 4.02 ms,
+// 4.26 with all).
+constexpr int kIntegrateCtasAlone = 8, kIntegrateCtasPaired = 4;
+
+int ashb_tsdf_integrate(void* embeddings, int64_t n_emb, int G, int64_t D, const int32_t* grid_coords,
+                        const uint32_t* touched, uint32_t stamp, const float* depth, const float* color, int H,
+                        int W, const float* intrinsic, const float* world_to_cam, float depth_max,
+                        double cell_size, const float* origin, float trunc, int sdf_channel, int rgb_channel,
+                        int weight_channel, unsigned long long* n_integrated_dev, const int32_t* touched_list,
+                        const int32_t* touched_count, void* stream) {
+    return integrate_impl(embeddings, n_emb, G, D, grid_coords, touched, stamp, depth, color, H, W, intrinsic,
+                          world_to_cam, depth_max, cell_size, origin, trunc, sdf_channel, rgb_channel, weight_channel,
+                          n_integrated_dev, touched_list, touched_count, kIntegrateCtasAlone, stream);
 }
 
 // Device address of g_tsdf_static_scratch on the current device.  In host code the array's
@@ -688,10 +702,11 @@ int ashb_tsdf_fuse_frames(ashb_map* m, void* embeddings, int64_t n_emb, int G, i
             return rc;
         ASHB_CUDA_TRY(cudaEventRecord(p->touched[b], p->side));
         ASHB_CUDA_TRY(cudaStreamWaitEvent(st, p->touched[b], 0));
-        if (int rc = ashb_tsdf_integrate(embeddings, n_emb, G, D, grid_coords, touched, first_stamp + (uint32_t)f,
+        if (int rc = integrate_impl(embeddings, n_emb, G, D, grid_coords, touched, first_stamp + (uint32_t)f,
                                          depths[f], colors[f], H, W, intrinsics + 9 * f, world_to_cams + 12 * f,
                                          depth_max, cell_size, origin, trunc, sdf_channel, rgb_channel, weight_channel,
-                                         n_integrated_dev, touched_list + (int64_t)b * n_emb, touched_count + b, st))
+                                         n_integrated_dev, touched_list + (int64_t)b * n_emb, touched_count + b,
+                                    kIntegrateCtasPaired, st))
             return rc;
         ASHB_CUDA_TRY(cudaEventRecord(p->integrated[b], st));
     }
