@@ -346,7 +346,7 @@ class SparseDenseGrid(ASHModule):
         if (self.separable_gaussian and self.tiled_convolution and emb.is_cuda and emb.dtype == torch.float32
                 and 1 <= radius <= self.grid_dim and hasattr(backend, "filter_separable_")):
             # the window of the last call is kept: laying it out costs a host copy that waits for the device
-            window = (size, sigma, channels, emb.device)
+            window = (size, float(sigma), channels, emb.device)
             if self._gaussian_window is None or self._gaussian_window[0] != window:
                 k1 = self._gaussian_weights_1d(size, sigma)
                 k1 = k1 / k1.sum()                   # (k1 (x) k1 (x) k1) / sum = product of the normalised factors
