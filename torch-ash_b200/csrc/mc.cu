@@ -98,13 +98,14 @@ constexpr int kTileTarget = 1024;   // cells
 constexpr int kMaxFastEdge = 16;
 constexpr int kClassifyCtas = 6;   // per SM: what 40 registers allow
 
-// A CTA walks tiles of max(1, 1024 / G^3) blocks (five barriers a tile: 512 cells of G = 8 are too few).  It stages one state byte per cell of the block AND of the
-// layer that its upper neighbours add, (G + 1)^3 in all, so every value is read once (G = 8: 1.4 loads
-// of sdf and weight per cell instead of 8 of each behind 24 table reads); cubes then read bytes of
-// shared memory.  Requests for the block's own edges meet in shared memory and go out a word at a
-// time; the two counters see one atomic per CTA.  GT: the block edge where it is known when compiling
-// (the halo's divisions), 0 otherwise.  Cell tables that are not the usual ones (odd_tables), and edges
-// beyond kMaxFastEdge (G = 0), take the corners from the tables.
+// A CTA walks tiles of max(1, 1024 / G^3) blocks (a tile has five barriers: the 512 cells of one block of
+// G = 8 are too few).  It stages one state byte per cell of a block AND of the layer that its upper
+// neighbours add, (G + 1)^3 in all, so every value is read once (G = 8: 1.4 loads of sdf and weight per
+// cell instead of 8 of each behind 24 table reads); cubes then read bytes of shared memory.  Requests for
+// the block's own edges meet in shared memory and go out a word at a time; the two counters see one
+// atomic per CTA.  GT: the block edge where it is known when compiling (the halo's divisions), 0
+// otherwise.  Cell tables that are not the usual ones (odd_tables), and edges beyond kMaxFastEdge
+// (G = 0), take the corners from the tables.
 template <int GT>
 __global__ void __launch_bounds__(256, kClassifyCtas) mc_classify_kernel(const float* __restrict__ sdfs,
                                                           const float* __restrict__ weights, McLuts L,
