@@ -354,6 +354,13 @@ class SparseDenseGrid(ASHModule):
                 self._gaussian_window = (window, w1.to(emb.device))
             w1 = self._gaussian_window[1]
             w1.record_stream(torch.cuda.current_stream(emb.device))   # it may be replaced while another stream reads it
+            if emb.is_inference():   # copy_ knows where such a tensor may be written
+                _, lut_g2g = self.construct_grid_neighbor_lut(1, bidirectional=True)
+                _, _, grid_indices, _ = self.items()
+                emb.copy_(backend.convolution_forward_separable(emb.data, w1, grid_indices, lut_g2g, self.grid_dim, radius))
+                return
+            # a forward pass may have saved the table: autograd has to hear of a write that it does not see
+            torch.autograd.graph.increment_version(emb)
             backend.filter_separable_(emb.data, w1, self.engine.backend, self.grid_dim, radius)
             return
         weights = self._gaussian_weights(size, sigma).view(size, size, size, 1).repeat(1, 1, 1, channels)
