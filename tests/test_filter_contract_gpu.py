@@ -42,3 +42,14 @@ def test_render_backward_after_the_filter_is_refused():
     grid.gaussian_filter_(3, 1.0)
     with pytest.raises(RuntimeError, match="modified by an inplace operation"):
         out["rgb"].sum().backward()
+
+
+@pytest.mark.parametrize("rows", [12, 40])
+def test_table_of_another_row_count_is_refused(rows):
+    """Rows of a shard are not the map's indices."""
+    grid = _grid(n=20, spare=5)
+    grid.embeddings = torch.nn.Parameter(torch.randn(rows, 64, 2, device=DEV))
+    before = grid.embeddings.detach().clone()
+    with pytest.raises(RuntimeError):
+        grid.gaussian_filter_(3, 1.0)
+    assert torch.equal(grid.embeddings.detach(), before)

@@ -942,6 +942,8 @@ def filter_separable_(values, weights_1d, hashmap, grid_dim, radius):
     n_emb, cells, D = v.shape
     if v.data_ptr() != values.data_ptr() or cells != int(grid_dim) ** 3 or w.shape != (3, 2 * int(radius) + 1, D):
         raise RuntimeError("filter_separable_: values must be contiguous and shaped for (grid_dim, radius)")
+    if n_emb != hashmap._capacity or v.device != hashmap.device():   # a shard's rows are not the map's indices
+        raise RuntimeError("filter_separable_: values must hold a row for every index of the map, on its device")
     dev = v.device
     scratch = torch.empty_like(v)
     lut = torch.empty((n_emb, 27), dtype=torch.int64, device=dev)
