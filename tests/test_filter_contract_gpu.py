@@ -53,3 +53,14 @@ def test_table_of_another_row_count_is_refused(rows):
     with pytest.raises(RuntimeError):
         grid.gaussian_filter_(3, 1.0)
     assert torch.equal(grid.embeddings.detach(), before)
+
+
+def test_other_strides_are_filtered_too():
+    grid = _grid()
+    start = grid.embeddings.detach().clone()
+    grid.gaussian_filter_(5, 1.5)
+    want = grid.embeddings.detach().clone()
+    grid.embeddings = torch.nn.Parameter(start.permute(2, 0, 1).contiguous().permute(1, 2, 0))
+    assert not grid.embeddings.is_contiguous()
+    grid.gaussian_filter_(5, 1.5)
+    assert torch.equal(grid.embeddings.detach(), want)

@@ -354,9 +354,9 @@ class SparseDenseGrid(ASHModule):
                 self._gaussian_window = (window, w1.to(emb.device))
             w1 = self._gaussian_window[1]
             w1.record_stream(torch.cuda.current_stream(emb.device))   # it may be replaced while another stream reads it
-            # through a copy: an inference tensor (copy_ knows where it may be written) and a shard of a split table,
-            # whose rows are not the map's indices (refused there)
-            if emb.is_inference() or emb.shape[0] != self.num_embeddings:
+            # through a copy: an inference tensor (copy_ knows where it may be written), a shard of a split table,
+            # whose rows are not the map's indices (refused there), and strides that the kernels do not take
+            if emb.is_inference() or emb.shape[0] != self.num_embeddings or not emb.is_contiguous():
                 _, lut_g2g = self.construct_grid_neighbor_lut(1, bidirectional=True)
                 _, _, grid_indices, _ = self.items()
                 emb.copy_(backend.convolution_forward_separable(emb.data, w1, grid_indices, lut_g2g, self.grid_dim, radius))
