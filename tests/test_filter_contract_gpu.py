@@ -64,3 +64,19 @@ def test_other_strides_are_filtered_too():
     assert not grid.embeddings.is_contiguous()
     grid.gaussian_filter_(5, 1.5)
     assert torch.equal(grid.embeddings.detach(), want)
+
+
+@pytest.mark.parametrize("call", [lambda g: g.gaussian_filter_(3, 1.0)])
+def test_capture_is_refused(call):
+    """A graph would hold the address of factors that a later call replaces."""
+    grid = _grid()
+    call(grid)
+    before = grid.embeddings.detach().clone()
+    graph = torch.cuda.CUDAGraph()
+    with pytest.raises(RuntimeError, match="captur"):
+        with torch.cuda.graph(graph):
+            call(grid)
+    del graph
+    torch.cuda.synchronize()
+    assert torch.equal(grid.embeddings.detach(), before)
+    call(grid)

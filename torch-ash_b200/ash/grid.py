@@ -345,6 +345,8 @@ class SparseDenseGrid(ASHModule):
         emb = self.embeddings
         if (self.separable_gaussian and self.tiled_convolution and emb.is_cuda and emb.dtype == torch.float32
                 and 1 <= radius <= self.grid_dim and hasattr(backend, "filter_separable_")):
+            if torch.cuda.is_current_stream_capturing():
+                raise RuntimeError("gaussian_filter_ in stream capture: a later call may free the factors that the graph reads")
             # the window of the last call is kept: laying it out costs a host copy that waits for the device
             window = (size, float(sigma), channels, emb.device)
             if self._gaussian_window is None or self._gaussian_window[0] != window:
