@@ -66,9 +66,38 @@ def test_other_strides_are_filtered_too():
     assert torch.equal(grid.embeddings.detach(), want)
 
 
-@pytest.mark.parametrize("call", [lambda g: g.gaussian_filter_(3, 1.0)])
+def _overflow(grid):
+    keys = torch.arange(30, dtype=torch.int32, device=DEV).view(-1, 1).repeat(1, 3)
+    grid.engine.backend.insert_keys(keys)        # as native insertions do: past the host's own bound
+
+
+@pytest.mark.parametrize("call", [lambda g: g.gaussian_filter_(3, 1.0), lambda g: g.construct_grid_neighbor_lut(1, True)])
+def test_dropped_keys_are_reported(call):
+    grid = _grid()
+    _overflow(grid)
+    with pytest.warns(UserWarning, match="capacity"):
+        call(grid)
+
+
+def test_a_table_in_error_is_left_unfiltered():
+    grid = _grid()
+    keys, index = grid.engine.items()
+    keys[1] = keys[0]
+    import __ash
+
+    h = grid.engine.backend
+    rc = __ash._lib.ashb_map_load_states(h._h, keys.data_ptr(), index.data_ptr(), keys.shape[0], h._heap.data_ptr(),
+                                         torch.cuda.current_stream().cuda_stream)
+    assert rc == 0
+    before = grid.embeddings.detach().clone()
+    with pytest.raises(RuntimeError, match="status"):
+        grid.gaussian_filter_(3, 1.0)
+    assert torch.equal(grid.embeddings.detach(), before)
+
+
+@pytest.mark.parametrize("call", [lambda g: g.gaussian_filter_(3, 1.0), lambda g: g.construct_grid_neighbor_lut(1, True)])
 def test_capture_is_refused(call):
-    """A graph would hold the address of factors that a later call replaces."""
+    """The call reads the map's status, and a graph would hold the address of factors that a later call replaces."""
     grid = _grid()
     call(grid)
     before = grid.embeddings.detach().clone()

@@ -934,26 +934,33 @@ def convolution_forward_separable(inputs, weights_1d, grid_indices, lut_grid_nb2
     return out
 
 
-def filter_separable_(values, weights_1d, hashmap, grid_dim, radius):
-    """``values`` (num_embeddings, G^3, D) float32, filtered in place over the active blocks of ``hashmap`` with the x, y and
-    z factors ``weights_1d`` (3, 2R+1, D); rows of inactive indices become zero.  No host synchronisation."""
+def grid_active_rows(hashmap):
+    """(rows int32 (capacity + 1,), lut int64 (capacity, 27)): the active indices of ``hashmap`` in no particular order
+    with their number in the last element, and the two-sided block window of radius 1, as ``filter_separable_`` takes
+    them.  No host synchronisation."""
+    n_emb, dev = hashmap._capacity, hashmap.device()
+    lut = torch.empty((n_emb, 27), dtype=torch.int64, device=dev)
+    rows = torch.empty(n_emb + 1, dtype=torch.int32, device=dev)
+    _check(_lib.ashb_grid_build_window_lut(hashmap._h, 1, 1, lut.data_ptr(), None, n_emb, rows.data_ptr(),
+                                           rows[n_emb:].data_ptr(), _stream(dev)))
+    return rows, lut
+
+
+def filter_separable_(values, weights_1d, rows, lut, grid_dim, radius):
+    """``values`` (num_embeddings, G^3, D) float32, filtered in place over the active blocks that ``grid_active_rows``
+    found, with the x, y and z factors ``weights_1d`` (3, 2R+1, D); the other rows become zero.  No host synchronisation."""
     v = _cuda(values, "values", torch.float32)
     w = _cuda(weights_1d, "weights_1d", torch.float32)
     n_emb, cells, D = v.shape
     if v.data_ptr() != values.data_ptr() or cells != int(grid_dim) ** 3 or w.shape != (3, 2 * int(radius) + 1, D):
         raise RuntimeError("filter_separable_: values must be contiguous and shaped for (grid_dim, radius)")
-    if n_emb != hashmap._capacity or v.device != hashmap.device():   # a shard's rows are not the map's indices
+    if rows.shape != (n_emb + 1,) or lut.shape != (n_emb, 27) or v.device != lut.device:   # a shard's rows are not the map's indices
         raise RuntimeError("filter_separable_: values must hold a row for every index of the map, on its device")
-    dev = v.device
     scratch = torch.empty_like(v)
-    lut = torch.empty((n_emb, 27), dtype=torch.int64, device=dev)
-    rows = torch.empty(n_emb + 1, dtype=torch.int32, device=dev)
-    count = rows[n_emb:]
-    st = _stream(dev)
-    with torch.cuda.device(dev):
-        _check(_lib.ashb_grid_build_window_lut(hashmap._h, 1, 1, lut.data_ptr(), None, n_emb, rows.data_ptr(), count.data_ptr(), st))
-        _check(_lib.ashb_filter_separable_inplace(v.data_ptr(), scratch.data_ptr(), w.data_ptr(), rows.data_ptr(), count.data_ptr(),
-                                                  lut.data_ptr(), n_emb, int(grid_dim), int(radius), D, st))
+    with torch.cuda.device(v.device):
+        _check(_lib.ashb_filter_separable_inplace(v.data_ptr(), scratch.data_ptr(), w.data_ptr(), rows.data_ptr(),
+                                                  rows[n_emb:].data_ptr(), lut.data_ptr(), n_emb, int(grid_dim), int(radius), D,
+                                                  _stream(v.device)))
 
 
 def grid_spatial_init(hashmap, points, cell_size, origin, grid_dim, dilation, bidirectional, grid_coords, touched,

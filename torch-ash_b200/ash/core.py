@@ -7,6 +7,7 @@ out.  Class, method, argument and state_dict key names follow ash/core.py:39-371
 so that code and checkpoints written for the reference keep working.
 """
 import warnings
+from contextlib import contextmanager
 from typing import Dict, Optional, Tuple, Union
 
 import torch
@@ -117,9 +118,28 @@ class ASHEngine(nn.Module):
         (ash/core.py:206-211); a probe or wait that gave up (the key was NOT stored) -> error.  Called
         where the host synchronises with the device anyway (a batch that could overflow, size(),
         items(), state_dict()), so that no such bit stays unseen."""
-        if not hasattr(self.backend, "status"):
+        if hasattr(self.backend, "status"):
+            self._tell_status(self.backend.status(), what)
+
+    @contextmanager
+    def _status_reported(self, what: str):
+        """``_report_status`` around work that needs no host read itself: the word is copied out ahead of it, and
+        once the work is enqueued the host waits for the copy, not for the work."""
+        if not hasattr(self.backend, "status_async"):
+            self._report_status(what)
+            yield
             return
-        st = self.backend.status()
+        if torch.cuda.is_current_stream_capturing():
+            raise RuntimeError("the status of the hash map is read by the host, which stream capture does not allow")
+        word = torch.empty(1, dtype=torch.int32, pin_memory=True)
+        copied = self.backend.status_async(word)
+        try:
+            yield
+        finally:
+            copied.synchronize()
+            self._tell_status(int(word.item()), what)
+
+    def _tell_status(self, st: int, what: str) -> None:
         if st & backend.STATUS_CAPACITY:
             warnings.warn(
                 f"{what} exceeds the hash map capacity {self.capacity}; the keys beyond "

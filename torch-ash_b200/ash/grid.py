@@ -363,9 +363,11 @@ class SparseDenseGrid(ASHModule):
                 _, _, grid_indices, _ = self.items()
                 emb.copy_(backend.convolution_forward_separable(emb.data, w1, grid_indices, lut_g2g, self.grid_dim, radius))
                 return
+            with self.engine._status_reported("An earlier insertion"):
+                rows, lut_g2g = backend.grid_active_rows(self.engine.backend)
             # a forward pass may have saved the table: autograd has to hear of a write that it does not see
             torch.autograd.graph.increment_version(emb)
-            backend.filter_separable_(emb.data, w1, self.engine.backend, self.grid_dim, radius)
+            backend.filter_separable_(emb.data, w1, rows, lut_g2g, self.grid_dim, radius)
             return
         weights = self._gaussian_weights(size, sigma).view(size, size, size, 1).repeat(1, 1, 1, channels)
         self.embeddings.copy_(self.convolution(self.embeddings, weights.to(self.embeddings.device)))
@@ -422,8 +424,9 @@ class SparseDenseGrid(ASHModule):
         (num_embeddings, K) int64)``; rows of inactive blocks and absent neighbours hold -1
         (ash/grid.py:566-617)."""
         if self.device.type == "cuda" and hasattr(backend, "grid_build_window_lut"):
-            # one table scan in which a warp probes a block's window; no enumeration, no host read
-            return backend.grid_build_window_lut(self.engine.backend, self.num_embeddings, radius, bidirectional)
+            # one table scan in which a warp probes a block's window; no enumeration
+            with self.engine._status_reported("An earlier insertion"):
+                return backend.grid_build_window_lut(self.engine.backend, self.num_embeddings, radius, bidirectional)
         coords, indices = self.engine.items()
         offsets, _ = enumerate_neighbor_coord_offsets(self.in_dim, radius, bidirectional, self.device)
         K = offsets.shape[0]
