@@ -109,3 +109,34 @@ def test_capture_is_refused(call):
     torch.cuda.synchronize()
     assert torch.equal(grid.embeddings.detach(), before)
     call(grid)
+
+
+def test_window_kept_by_another_thread_is_not_used():
+    """Another thread's window may take the place of this call's at any time."""
+    grid, alone = _grid(seed=4), _grid(seed=4)
+    alone.gaussian_filter_(3, 1.0)
+    ours = alone._gaussian_window
+    other = _grid(seed=4)
+    other.gaussian_filter_(3, 2.0)
+    theirs, start = other._gaussian_window, grid.embeddings.detach().clone()
+    for looks in range(4):
+        class Raced(ash.SparseDenseGrid):
+            seen = 0
+
+            @property
+            def _gaussian_window(self):
+                Raced.seen += 1
+                return ours if Raced.seen <= looks else theirs
+
+            @_gaussian_window.setter
+            def _gaussian_window(self, value):
+                pass
+
+        grid.embeddings.data.copy_(start)
+        grid.__class__ = Raced
+        grid.gaussian_filter_(3, 1.0)
+        grid.__class__ = ash.SparseDenseGrid
+        want = grid.embeddings.detach().clone()
+        grid.embeddings.data.copy_(start)
+        grid.gaussian_filter_(3, 1.0)
+        assert torch.equal(want, grid.embeddings.detach()), looks

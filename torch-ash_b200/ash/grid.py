@@ -349,12 +349,13 @@ class SparseDenseGrid(ASHModule):
                 raise RuntimeError("gaussian_filter_ in stream capture: a later call may free the factors that the graph reads")
             # the window of the last call is kept: laying it out costs a host copy that waits for the device
             window = (size, float(sigma), channels, emb.device)
-            if self._gaussian_window is None or self._gaussian_window[0] != window:
+            kept = self._gaussian_window             # read once: another thread may put its own there
+            if kept is None or kept[0] != window:
                 k1 = self._gaussian_weights_1d(size, sigma)
                 k1 = k1 / k1.sum()                   # (k1 (x) k1 (x) k1) / sum = product of the normalised factors
                 w1 = torch.from_numpy(k1).float().view(1, size, 1).repeat(3, 1, channels).contiguous()
-                self._gaussian_window = (window, w1.to(emb.device))
-            w1 = self._gaussian_window[1]
+                kept = self._gaussian_window = (window, w1.to(emb.device))
+            w1 = kept[1]
             w1.record_stream(torch.cuda.current_stream(emb.device))   # it may be replaced while another stream reads it
             # through a copy: an inference tensor (copy_ knows where it may be written), a shard of a split table,
             # whose rows are not the map's indices (refused there), and strides that the kernels do not take
