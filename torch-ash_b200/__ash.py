@@ -17,6 +17,7 @@ import os
 import warnings
 
 import torch
+import torch.autograd.forward_ad as _forward_ad
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 _LIB_PATH = os.path.join(_HERE, "libashb200.so")
@@ -179,6 +180,13 @@ def set_find_cooperative(enable: bool) -> None:
     _check(_lib.ashb_set_find_cooperative(int(bool(enable))))
 
 
+def transforms_open() -> bool:
+    """Whether a forward-mode level or a torch.func transform is open: tensors may then carry tangents or batch
+    dimensions that a kernel called with their addresses would drop.  True where torch does not say."""
+    return getattr(_forward_ad, "_current_level", 0) >= 0 or _functorch_active()
+
+
+_functorch_active = getattr(torch._C, "_are_functorch_transforms_active", lambda: True)
 _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
 
 

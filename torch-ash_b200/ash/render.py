@@ -179,7 +179,8 @@ def render_rays(grid, rays_o: torch.Tensor, rays_d: torch.Tensor, t_min: float, 
     if parallel_samples is None:
         parallel_samples = rays_o.shape[0] <= 32768
     beta = beta.to(torch.float32)
-    if torch.is_grad_enabled() and (grid.embeddings.requires_grad or beta.requires_grad):
+    # the autograd function also refuses tangents, which it has no rule for
+    if (torch.is_grad_enabled() and (grid.embeddings.requires_grad or beta.requires_grad)) or backend.transforms_open():
         columns = _RenderRays.apply(grid.embeddings, beta, geom, rays, bool(parallel_samples))
     else:
         rows, _ = _render_rows(grid.embeddings, beta, geom, rays, bool(parallel_samples))
