@@ -284,10 +284,13 @@ class HashMap:
     def find_values(self, keys: torch.Tensor, tables: dict):
         """``(indices, masks, {name: tables[name][indices]})`` in one launch (not in the reference), or None where the
         gathers are better left to indexing: wide rows, which a warp reads side by side, more tables than a launch
-        takes, and tables that autograd records."""
-        if len(tables) > 16:
+        takes, tables that autograd records, and those whose values are more than their bytes (tangents, batch
+        dimensions, conjugate and negative views, subclasses)."""
+        if len(tables) > 16 or transforms_open():
             return None
         for v in tables.values():
+            if type(v) not in (torch.Tensor, torch.nn.Parameter) or v.is_conj() or v.is_neg():
+                return None
             if not (v.device == self._device and v.is_contiguous() and v.dim() >= 1 and 0 < v.numel() and v.shape[0] == self._capacity
                     and v.numel() // v.shape[0] * v.element_size() <= 64) or (v.requires_grad and torch.is_grad_enabled()):
                 return None
