@@ -59,3 +59,23 @@ def test_a_list_of_some_blocks():
     assert mesh[0].shape[0] == ref[0].shape[0]
     # vertices owned by a block outside the list are not placed: their id is -1 on both sides
     np.testing.assert_array_equal(np.sort((mesh[0] < 0).sum(1).cpu().numpy()), np.sort((ref[0] < 0).sum(1)))
+
+
+@pytest.mark.parametrize("G", [3, 8])
+def test_a_block_listed_twice(G):
+    """Its triangles come twice, its vertices once: every id points at a vertex that was placed."""
+    import __ash
+    import mesh_checks
+    import numpy as np
+
+    grid, sdf, w = _noisy_grid(G, 3, 0)
+    _, idx = grid.engine.items()
+    rest = (grid.grid_coords, grid.lut_grid_nb2grid_idx, grid.cell_coords, grid.lut_cell_nb2cell_idx,
+            grid.lut_cell_nb2grid_nb, G, 0.0, 1.0)
+    tris, verts = [t.cpu().numpy() for t in __ash.marching_cubes(sdf, w, idx, *rest)]
+    tris2, verts2 = [t.cpu().numpy() for t in __ash.marching_cubes(sdf, w, torch.cat([idx, idx]), *rest)]
+    assert verts2.shape == verts.shape and tris2.shape[0] == 2 * tris.shape[0]
+    assert tris2.min() >= 0 and tris2.max() < verts.shape[0]
+    np.testing.assert_array_equal(verts2[np.lexsort(verts2.T[::-1])], verts[np.lexsort(verts.T[::-1])])
+    np.testing.assert_array_equal(mesh_checks.canonical_triangle_rows(verts2, tris2),
+                                  np.repeat(mesh_checks.canonical_triangle_rows(verts, tris), 2, axis=0))

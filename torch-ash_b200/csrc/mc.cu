@@ -82,6 +82,12 @@ __device__ __forceinline__ int request_edges(uint8_t* wanted, int64_t a, uint32_
     return __popc(bits & ~(old >> at));
 }
 
+// Marks the vertices of the cell at flat address `a` as placed; returns whether they were.
+__device__ __forceinline__ bool claimed(uint8_t* wanted, int64_t a) {
+    const int at = (int)(a & 3) * 8;
+    return (atomicOr(reinterpret_cast<uint32_t*>(wanted + (a - (a & 3))), kHasVertices << at) >> at) & kHasVertices;
+}
+
 // Raises odd_tables unless corner k of cell (x, y, z) is, in both cell tables, the cell at + k's offsets.
 __global__ void __launch_bounds__(256) mc_check_tables_kernel(McLuts L, McEdges edges, int G) {
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
@@ -336,6 +342,8 @@ __global__ void __launch_bounds__(256) mc_vertex_kernel(const float* __restrict_
                 bits[j] = edges.wanted[address[j]] & 7u;
             }
         }
+        // a block may be listed twice: whichever listing comes first places the cell's vertices
+        if (bits[j] && claimed(edges.wanted, address[j])) bits[j] = 0;
         mine += __popc(bits[j]);
     }
     int total;
@@ -346,7 +354,6 @@ __global__ void __launch_bounds__(256) mc_vertex_kernel(const float* __restrict_
     for (int j = 0; j < 4; ++j) {
         if (bits[j] == 0) continue;
         edges.first_vertex[address[j]] = (int)(base + at);
-        edges.wanted[address[j]] = (uint8_t)(bits[j] | kHasVertices);
 #pragma unroll
         for (int d = 0; d < 3; ++d)
             if (bits[j] & (1u << d)) list[at++] = (uint16_t)((4 * threadIdx.x + j) * 4 + d);
