@@ -206,7 +206,7 @@ int ashb_query_backward_backward(int dtype, int interp, const void* grad_grad_of
 int ashb_grid_build_neighbor_lut(ashb_map* map, int32_t* nb_lut, int32_t* grid_coords, int64_t n_emb,
                                  void* stream);
 
-/* The block window of any radius, one-sided (offsets 0..radius) or two-sided (-radius..radius), as the
+/* The block window of a radius of 0 to 64, one-sided (offsets 0..radius) or two-sided (-radius..radius), as the
  * int64 table lut [n_emb][window^3] of SparseDenseGrid.construct_grid_neighbor_lut (ash/grid.py:566-617):
  * x fastest, -1 for absent neighbours and in the rows of inactive indices; grid_coords as above.  list
  * int32 [n_emb] and list_count (both or neither) receive the active rows in no particular order. */

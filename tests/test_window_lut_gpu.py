@@ -30,3 +30,20 @@ def test_window_table_equals_dictionary(n, capacity, radius, bidirectional):
         want_coords[i] = torch.tensor([x, y, z])
         want_lut[i] = torch.tensor([rows.get((x + dx, y + dy, z + dz), -1) for dz, dy, dx in itertools.product(steps, repeat=3)])
     assert torch.equal(coords.cpu(), want_coords) and torch.equal(lut.cpu(), want_lut)
+
+
+@pytest.mark.parametrize("radius", [64, 65, 70])
+def test_wide_one_sided_windows(radius):
+    grid = ash.SparseDenseGrid(3, 4, 1, 2, DEV)
+    keys = [(0, 0, 0), (radius, 0, 3), (70, 70, 70), (-radius, 1, -2)]
+    grid.engine.insert_keys(torch.tensor(keys, dtype=torch.int32, device=DEV))
+    coords, lut = grid.construct_grid_neighbor_lut(radius, False)
+    keys, index = grid.engine.items()
+    S = radius + 1
+    want = torch.full((4, S**3), -1, dtype=torch.int64)
+    for a, i in zip(keys.tolist(), index.tolist()):
+        for b, j in zip(keys.tolist(), index.tolist()):
+            dx, dy, dz = (q - p for p, q in zip(a, b))
+            if all(0 <= d <= radius for d in (dx, dy, dz)):
+                want[i, dx + S * (dy + S * dz)] = j
+    assert torch.equal(lut.cpu(), want) and torch.equal(coords[index], keys)

@@ -424,8 +424,8 @@ class SparseDenseGrid(ASHModule):
         """Per-block tables ``(grid_coords (num_embeddings, 3) int32, lut_grid_nb2grid_idx
         (num_embeddings, K) int64)``; rows of inactive blocks and absent neighbours hold -1
         (ash/grid.py:566-617)."""
-        if self.device.type == "cuda" and hasattr(backend, "grid_build_window_lut"):
-            # one table scan in which a warp probes a block's window; no enumeration
+        if self.device.type == "cuda" and 0 <= radius <= 64 and hasattr(backend, "grid_build_window_lut"):
+            # one table scan in which a warp probes a block's window; no enumeration (64: as far as the kernel goes)
             with self.engine._status_reported("An earlier insertion"):
                 return backend.grid_build_window_lut(self.engine.backend, self.num_embeddings, radius, bidirectional)
         coords, indices = self.engine.items()
