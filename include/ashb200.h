@@ -569,7 +569,7 @@ int ashb_render_split(const float* rows, float* const* columns, int64_t n_rays, 
 int ashb_render_join(const float* const* grads, const int64_t* strides, float* grad_rows, int64_t n_rays, void* stream);
 
 /* The same renderer with the samples of a ray evaluated in parallel: _intervals marches every ray
- * once (one thread per ray) and lists its intervals, float32 [n_rays][stride][2] (t0, t1 in cell
+ * once (a group of eight lanes per ray) and lists its intervals, float32 [n_rays][stride][2] (t0, t1 in cell
  * units), with counts int32 [n_rays] and near_far float32 [n_rays][2] (world units); intervals
  * beyond `stride` are dropped and ASHB_STATUS_CAPACITY is set in the map's status word (stride =
  * max_samples_per_ray + 2 always suffices).  _forward / _backward then spend one WARP per ray on

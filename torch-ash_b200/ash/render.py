@@ -149,9 +149,12 @@ def render_rays(grid, rays_o: torch.Tensor, rays_d: torch.Tensor, t_min: float, 
     ``parallel_samples``: a marching launch lists every ray's intervals ((max_samples_per_ray + 2) x
     8 bytes per ray) and a warp per ray evaluates them 32 at a time; the backward reuses the list.
     Same results up to floating-point summation order.  It shortens the dependent chain of a ray, which
-    is what bounds small batches (8192 rays: forward 0.14 against 0.19 ms, backward 0.04 against
-    0.17 ms), and wastes lanes on large ones (262144 rays: 0.98 + 1.14 against 0.82 + 0.74 ms);
-    ``None`` picks it for batches of up to 32768 rays.
+    is what bounds small batches, and wastes lanes on large ones; ``None`` picks it for batches of up to
+    32768 rays.  Whole calls against the one-launch form, without a gradient, for the rays of a view and
+    for rays in random directions: 8192 rays 102 against 185 and 104 against 227 us, 32768 rays 162
+    against 184 and 165 against 238, 65536 rays 250 against 183 and 263 against 263, 262144 rays 799
+    against 324 and 854 against 632; with the backward pass 417 against 464 and 404 against 551 at 32768,
+    551 against 476 and 560 against 608 at 65536.
 
     Returns a dict of per-ray tensors: ``rgb`` (n, 3), ``depth`` (n, 1) = sum of weight * t_mid,
     ``normal`` (n, 3), ``weights`` (n, 1), ``eikonal_l1`` / ``eikonal_l2`` (n, 1) = sums over the

@@ -1,11 +1,12 @@
 // Triangle mesh of the iso-surface over the sparse-dense structure (sm_100a): marching cubes
-// in three launches and ONE host read.  Stages and validity rules follow ash/src/grid.cu:607-946:
+// in four launches and ONE host read.  Stages and validity rules follow ash/src/grid.cu:607-946:
 // a cube sits at every cell of a listed block whose own weight and the weights of its 8 corners
 // (the cell and its +x/+y/+z neighbours through the lookup tables) reach the threshold and whose
 // neighbour blocks all exist; corner c is inside when sdf - iso < 0; every cut edge of a valid
 // cube gets one vertex, owned by the cell at the edge's lower corner, placed by linear
 // interpolation; triangles index those vertices.
 //
+//   check      whether the cell tables are the usual ones, which classify then need not read
 //   classify   per tile of blocks: corner pattern -> codes[]; each cut edge is requested at its owner
 //              as one bit of a byte per cell, so the number of distinct vertices is counted in the
 //              same pass, as is the number of triangles
@@ -13,7 +14,7 @@
 //   vertices   per 1024 cells: requested edges get consecutive slots and positions
 //   triangles  per 1024 cells: triangles get consecutive slots, vertex ids looked up at the owners
 //
-// All three are bound by instructions and latency, not bytes: what they shed is work per CELL where only one
+// The last three are bound by instructions and latency, not bytes: what they shed is work per CELL where only one
 // cell in twelve carries surface.  24,000 blocks of 8^3 on a B200: 444 + 114 + 107 us when every cell
 // read its eight corners through the tables, each warp bumped the shared counters and an edge took
 // four bytes of a 147 MB table that had to be filled, written and read; 130 + 39 + 57 us now.
