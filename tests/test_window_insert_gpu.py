@@ -129,3 +129,20 @@ def test_clear_leaves_an_empty_map(capacity, dim):
         m.clear()
         assert m.size() == 0 and not bool(m.find(keys).any()) and m.keys().shape[0] == 0
         assert torch.equal(m.engine._heap, torch.arange(capacity, device=DEV, dtype=torch.int32))
+
+
+def test_rows_of_many_small_words_are_left_to_indexing():
+    import ash
+
+    m = ash.HashMap(3, 1, 500, DEV)
+    keys = torch.randint(-9, 9, (300, 3), device=DEV, dtype=torch.int32)
+    m.engine.insert_keys(keys)
+    find, bytes_of = m.engine.backend.find_values, lambda w: torch.randint(0, 255, (500, w), device=DEV, dtype=torch.uint8)
+    unaligned = bytes_of(32).view(-1).new_zeros(500 * 32 + 1)[1:].view(500, 32)
+    for table, gathers in ((bytes_of(15), True), (bytes_of(17), False), (bytes_of(32), True), (bytes_of(30), True), (bytes_of(34), False),
+                           (bytes_of(60), True), (bytes_of(64), True), (bytes_of(68), False), (unaligned, False)):
+        found = find(keys, {"t": table})
+        assert (found is not None) == gathers, table.shape
+        m.values["default"] = table
+        _, rows, got = m.find(keys, return_values=True)
+        assert torch.equal(got, table[rows])

@@ -283,26 +283,30 @@ class HashMap:
 
     def find_values(self, keys: torch.Tensor, tables: dict):
         """``(indices, masks, {name: tables[name][indices]})`` in one launch (not in the reference), or None where the
-        gathers are better left to indexing: wide rows, which a warp reads side by side, more tables than a launch
+        gathers are better left to indexing: wide rows and rows of many small words, more tables than a launch
         takes, tables that autograd records, and those whose values are more than their bytes (tangents, batch
         dimensions, conjugate and negative views, subclasses)."""
         if len(tables) > 16 or transforms_open():
             return None
+        recorded, rows = torch.is_grad_enabled(), []
         for v in tables.values():
-            if type(v) not in (torch.Tensor, torch.nn.Parameter) or v.is_conj() or v.is_neg():
+            if type(v) not in (torch.Tensor, torch.nn.Parameter) or v.is_conj() or v.is_neg() or not v.is_contiguous() \
+                    or v.device != self._device or (recorded and v.requires_grad) or v.shape[:1] != (self._capacity,):
                 return None
-            if not (v.device == self._device and v.is_contiguous() and v.dim() >= 1 and 0 < v.numel() and v.shape[0] == self._capacity
-                    and v.numel() // v.shape[0] * v.element_size() <= 64) or (v.requires_grad and torch.is_grad_enabled()):
+            # a thread copies a row in the widest words that its length and address allow: 15 of them 39 against 45 us for
+            # 100k keys and 1.28 against 1.86 ms for 16M, 31 of them 54 against 50 us, 63 of them 6.2 against 5.4 ms
+            nbytes, at = v.nbytes // self._capacity, v.data_ptr()
+            if not 0 < nbytes <= 64 or nbytes > 16 * min(16, nbytes & -nbytes, at & -at):
                 return None
+            rows.append((at, nbytes))
         keys = self._keys(keys)
         n, k = keys.shape[0], len(tables)
         indices = torch.empty(n, dtype=torch.int64, device=self._device)
         masks = torch.empty(n, dtype=torch.bool, device=self._device)
         out = {name: torch.empty((n, *v.shape[1:]), dtype=v.dtype, device=self._device) for name, v in tables.items()}
         src, dst, row = (_vp * max(k, 1))(), (_vp * max(k, 1))(), (_i64 * max(k, 1))()
-        for j, (name, v) in enumerate(tables.items()):
-            src[j], dst[j] = v.data_ptr(), out[name].data_ptr()
-            row[j] = v.numel() // v.shape[0] * v.element_size()
+        for j, (to, (at, nbytes)) in enumerate(zip(out.values(), rows)):
+            src[j], dst[j], row[j] = at, to.data_ptr(), nbytes
         _check(_lib.ashb_map_find_values(self._h, keys.data_ptr(), n, indices.data_ptr(), masks.data_ptr(), k, src, dst, row,
                                          _stream(self._device)))
         return indices, masks, out
