@@ -140,3 +140,46 @@ def test_window_kept_by_another_thread_is_not_used():
         grid.embeddings.data.copy_(start)
         grid.gaussian_filter_(3, 1.0)
         assert torch.equal(want, grid.embeddings.detach()), looks
+
+
+@pytest.mark.parametrize("G,size,D,side,spare", [(4, 3, 1, 28, 100), (8, 7, 4, 17, 3000), (16, 7, 4, 11, 1), (5, 5, 13, 11, 200),
+                                                 (3, 3, 1, 20, 0)])
+def test_more_blocks_than_ctas(G, size, D, side, spare):
+    """Beyond eight waves of CTAs each takes a second block (and a second row to copy back): the same bits as with a CTA per
+    block, and zeros in the spare rows."""
+    import __ash as native
+
+    n = side**3
+    cells = torch.arange(n, device=DEV)
+    cells = cells[cells % 7 != 3]                                   # holes in the lattice
+    grid = ash.SparseDenseGrid(3, len(cells) + spare, D, G, DEV)
+    grid.engine.insert_keys(torch.stack([cells % side, cells // side % side, cells // side**2], 1).int())
+    grid.embeddings.data.normal_(generator=torch.Generator(device=DEV).manual_seed(G))
+    _, lut = grid.construct_grid_neighbor_lut(1, bidirectional=True)
+    _, index = grid.engine.items()
+    start = grid.embeddings.detach().clone()
+    grid.gaussian_filter_(size, 1.5)
+    want = native.convolution_forward_separable(start, grid._gaussian_window[1], index.view(-1, 1), lut, G, size // 2)
+    assert torch.equal(grid.embeddings.detach(), want)
+    rest = torch.ones(len(cells) + spare, dtype=torch.bool, device=DEV)
+    rest[index] = False
+    assert int(rest.sum()) == spare and not bool(want[rest].any())
+
+
+def test_windows_replaced_on_another_stream():
+    grid = _grid(D=16, seed=5)
+    start = grid.embeddings.detach().clone()
+    for _ in range(20):
+        grid.gaussian_filter_(3, 1.0)
+        grid.gaussian_filter_(5, 2.0)
+    want = grid.embeddings.detach().clone()
+    grid.embeddings.data.copy_(start)
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        for _ in range(20):
+            grid.gaussian_filter_(3, 1.0)
+            grid.gaussian_filter_(5, 2.0)
+            torch.full((3, 3, 16), 7.0, device=DEV), torch.full((3, 5, 16), 7.0, device=DEV)   # into what was given back
+    side.synchronize()
+    assert torch.equal(grid.embeddings.detach(), want)

@@ -74,9 +74,11 @@ def test_fused_equals_split_sequence(kind, G, D, interp):
     torch.testing.assert_close(ge2_f, ge2_s, rtol=2e-4, atol=1e-5 * max(1.0, float(ge2_s.abs().max())))
 
 
-def test_native_neighbor_table_equals_python_construction():
+def test_native_neighbor_table_equals_python_construction(monkeypatch):
     grid, _ = _make("plain", 8, 2, seed=5)
-    coords_py, lut_py = grid.construct_grid_neighbor_lut(1, False)  # items + find(8n) + scatter, ash/grid.py:566-617
+    with monkeypatch.context() as patch:
+        patch.delattr("__ash.grid_build_window_lut")
+        coords_py, lut_py = grid.construct_grid_neighbor_lut(1, False)  # items + find(8n) + scatter, ash/grid.py:566-617
     grid.construct_grid_neighbor_lut_(1, False)                      # native table scan
     assert torch.equal(grid.lut_grid_nb2grid_idx, lut_py)
     assert torch.equal(grid.grid_coords, coords_py)

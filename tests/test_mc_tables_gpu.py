@@ -79,3 +79,10 @@ def test_a_block_listed_twice(G):
     np.testing.assert_array_equal(verts2[np.lexsort(verts2.T[::-1])], verts[np.lexsort(verts.T[::-1])])
     np.testing.assert_array_equal(mesh_checks.canonical_triangle_rows(verts2, tris2),
                                   np.repeat(mesh_checks.canonical_triangle_rows(verts, tris), 2, axis=0))
+
+
+@pytest.mark.parametrize("G,side", [(4, 26), (6, 17), (8, 14), (16, 11), (17, 4)])
+def test_more_tiles_than_ctas(G, side):
+    """Six CTAs per SM share out the tiles (beyond the staged edge: 256 cells at a time), so each takes more than one."""
+    grid, sdf, w = _noisy_grid(G, side, 1)
+    _compare_with_oracle(grid, sdf + 2.5, w, 0.0, 1.0)

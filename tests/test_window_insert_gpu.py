@@ -146,3 +146,33 @@ def test_rows_of_many_small_words_are_left_to_indexing():
         m.values["default"] = table
         _, rows, got = m.find(keys, return_values=True)
         assert torch.equal(got, table[rows])
+
+
+@pytest.mark.parametrize("route", ["no memory", "side stream"])
+def test_sorted_insert_without_its_workspace_and_on_a_side_stream(route, monkeypatch):
+    import ash
+
+    m = ash.HashSet(3, CAPACITY, DEV)
+    g = torch.Generator(device=DEV).manual_seed(11)
+    keys = torch.randint(-2**18, 2**18, (8_500_000, 3), generator=g, device=DEV, dtype=torch.int32)
+    want = torch.unique(_packed(keys))
+    empty, refused = torch.empty, []
+
+    def no_workspace(*args, **kwargs):
+        if route == "no memory" and kwargs.get("dtype") is torch.uint8:
+            refused.append(args)
+            raise torch.cuda.OutOfMemoryError("no room for the workspace")
+        return empty(*args, **kwargs)
+
+    side = torch.cuda.Stream() if route == "side stream" else torch.cuda.current_stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side), monkeypatch.context() as patch:
+        patch.setattr(torch, "empty", no_workspace)
+        m.insert(keys)
+        # the workspace's memory goes to whoever asks next on this stream, after the insertion
+        empty(sum(keys.shape) * 12, dtype=torch.uint8, device=DEV).fill_(255)
+    side.synchronize()
+    assert len(refused) == (route == "no memory")
+    got, rows = m.engine.items()
+    assert torch.equal(torch.sort(_packed(got)).values, want)
+    assert torch.equal(torch.sort(rows).values, torch.arange(want.shape[0], device=DEV))
