@@ -103,7 +103,8 @@ int ashb_map_contains(ashb_map* map, const int32_t* keys_dev, int64_t n, uint8_t
 int ashb_map_insert_keys(ashb_map* map, const int32_t* keys_dev, int64_t n, void* stream);
 
 /* The same for a large batch into a table far beyond L2, its keys first sorted by the part of the table they
- * belong to.  _workspace: bytes of device scratch (16-byte aligned) that this takes, 0 where it does not apply. */
+ * belong to (unless a sample of them shows that most repeat: then in their own order).  _workspace: bytes of device
+ * scratch (16-byte aligned) that this takes, 0 where it does not apply. */
 int64_t ashb_map_insert_workspace(ashb_map* map, int64_t n);
 int ashb_map_insert_keys_sorted(ashb_map* map, const int32_t* keys_dev, int64_t n, void* workspace,
                                 int64_t workspace_bytes, void* stream);

@@ -131,6 +131,39 @@ def test_clear_leaves_an_empty_map(capacity, dim):
         assert torch.equal(m.engine._heap, torch.arange(capacity, device=DEV, dtype=torch.int32))
 
 
+@pytest.mark.parametrize("batch,sorts", [("distinct", True), ("half of them twice", True), ("one key", False), ("runs of twelve", False),
+                                         ("few in any order", False)])
+@pytest.mark.parametrize("dim", [1, 2, 3])
+def test_batches_of_repeats_go_in_their_own_order(batch, sorts, dim):
+    """The window counts at the workspace's head stay zero where the sample finds too few distinct keys."""
+    import __ash
+    import ash
+
+    n = 9_000_001
+    m = ash.HashSet(dim, CAPACITY, DEV)
+    g = torch.Generator(device=DEV).manual_seed(dim)
+    span = {1: 2**30, 2: 2**19, 3: 2**18}[dim]
+    keys = torch.randint(-span, span, (n, dim), generator=g, device=DEV, dtype=torch.int32)
+    if batch == "half of them twice":
+        keys[n // 2:] = keys[torch.randint(n // 2, (n - n // 2,), generator=g, device=DEV)]
+        keys = keys[torch.randperm(n, generator=g, device=DEV)]
+    elif batch == "one key":
+        keys[:] = keys[0]
+    elif batch == "runs of twelve":
+        keys = keys[torch.arange(n, device=DEV) // 12]
+    elif batch == "few in any order":
+        keys = keys[torch.randint(100_000, (n,), generator=g, device=DEV)]
+    keys = keys.contiguous()
+    h, stream = m.engine.backend._h, torch.cuda.current_stream().cuda_stream
+    workspace = torch.empty(__ash._lib.ashb_map_insert_workspace(h, n) // 4, dtype=torch.int32, device=DEV)
+    assert __ash._lib.ashb_map_insert_keys_sorted(h, keys.data_ptr(), n, workspace.data_ptr(), workspace.numel() * 4, stream) == 0
+    assert int(workspace[:256].sum()) == (n if sorts else 0)
+    got, rows = m.engine.items()
+    want = torch.unique(_packed(keys))
+    assert torch.equal(torch.sort(_packed(got)).values, want)
+    assert torch.equal(torch.sort(rows).values, torch.arange(want.shape[0], device=DEV))
+
+
 def test_rows_of_many_small_words_are_left_to_indexing():
     import ash
 

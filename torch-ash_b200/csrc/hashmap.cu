@@ -20,6 +20,7 @@
 // Semantics follow ash/src/hashmap_gpu.cuh (find :164-178, insert-if-absent +
 // heap pop :212-232, value copy by the winner :250-283, erase + heap push
 // :317-336, clear :355-358, items :377-405, load_states :408-450).
+#include <algorithm>
 #include <cstring>
 #include <new>
 
@@ -196,9 +197,50 @@ constexpr uint32_t kWindowShift = 22;        // slots per window
 constexpr int kMaxWindows = 256;
 constexpr int kSortKeys = 2048;              // keys of a CTA: 8 per thread
 
+// That pays while the batch has many distinct keys.  Where most of them repeat, or repeats stand side by side,
+// their lines stay in L2 as it is and the two streams come on top (50M keys of 1M distinct in order: 0.93 -> 1.40 ms, of
+// one: 0.50 -> 1.06), so a sample is asked first: 64 runs of 256 keys, and how many of their s = 16,384 keys another
+// key of the sample repeats.  With D distinct keys in random order that is s^2 / 2 D; the line lies at
+// D = slots / 16, half a distinct key per 128-byte line, where both ways take about the same time (4M distinct among 16M
+// keys into 1 GB: 0.55 ms in their order, 0.57 sorted; among 50M into 2 GB: 1.30 and 1.23; all distinct: 1.01 and 0.81,
+// 3.56 and 2.40).
+constexpr int kSampleRuns = 64;
+constexpr uint32_t kSampleSlots = 1u << 15;
+
+struct BatchSample {
+    const uint32_t* repeats;
+    uint32_t most;
+    __device__ __forceinline__ bool sorts() const { return *repeats <= most; }
+};
+
+// A CTA per run.  Asking and not sorting costs 15 to 25 us of the 300 us and more that such a batch takes (all runs by one
+// CTA with its set in shared memory: 45 us); repeats side by side are inserted 6 to 13 % faster than by insert_kernel.
+template <int DIM>
+__global__ void __launch_bounds__(256) batch_sample_kernel(const int32_t* __restrict__ keys, int64_t n, uint32_t* seen,
+                                                           uint32_t* repeats) {
+    int k0, k1, k2, k3;
+    load_key<DIM>(keys, n / kSampleRuns * blockIdx.x + threadIdx.x, k0, k1, k2, k3);
+    // two hashes of the key: the place and the word; what falls together in both counts as a repeat
+    const uint32_t word = hash_key(k2, k0, k1, 1) | 1u;
+    const unsigned peers = __match_any_sync(0xffffffffu, word);
+    bool repeat = (int)(threadIdx.x & 31) != __ffs(peers) - 1;
+    uint32_t s = hash_key(k0, k1, k2, 0) & (kSampleSlots - 1);
+    for (int probe = 0; probe < 64 && !repeat; ++probe) {
+        uint32_t old = __ldcg(seen + s);
+        if (old == 0u) old = atomicCAS(seen + s, 0u, word);
+        if (old == 0u) break;
+        repeat = old == word;
+        s = (s + 1) & (kSampleSlots - 1);
+    }
+    const int n_repeats = __syncthreads_count(repeat);
+    if (threadIdx.x == 0 && n_repeats) atomicAdd(repeats, (uint32_t)n_repeats);
+}
+
 // Inside a window the rest of a line is wanted too: fetched whole.
 struct Table16Lines : Table16 {
+    bool whole_lines;
     __device__ __forceinline__ Entry read_fresh(uint32_t s) const {
+        if (!whole_lines) return Table16::read_fresh(s);
         uint4 u;
         asm volatile("ld.global.cg.L2::128B.v4.u32 {%0,%1,%2,%3}, [%4];"
                      : "=r"(u.x), "=r"(u.y), "=r"(u.z), "=r"(u.w)
@@ -216,9 +258,10 @@ __device__ __forceinline__ int window_of(const int32_t* __restrict__ keys, int64
 }
 
 template <int DIM>
-__global__ void __launch_bounds__(256) window_count_kernel(uint32_t mask, const int32_t* __restrict__ keys, int64_t n,
-                                                           uint32_t* __restrict__ count) {
+__global__ void __launch_bounds__(256) window_count_kernel(BatchSample sample, uint32_t mask, const int32_t* __restrict__ keys,
+                                                           int64_t n, uint32_t* __restrict__ count) {
     __shared__ uint32_t mine[kMaxWindows];
+    if (!sample.sorts()) return;
     mine[threadIdx.x] = 0;
     __syncthreads();
     for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < n; i += (int64_t)gridDim.x * 256) {
@@ -246,53 +289,71 @@ __device__ __forceinline__ uint32_t prefix_256(uint32_t v) {
     return before + incl - v;
 }
 
-__global__ void __launch_bounds__(256) window_start_kernel(const uint32_t* __restrict__ count, uint32_t* __restrict__ cursor) {
-    cursor[threadIdx.x] = prefix_256(count[threadIdx.x]);
-}
-
 template <int DIM>
-__global__ void __launch_bounds__(256) window_sort_kernel(uint32_t mask, const int32_t* __restrict__ keys, int64_t n,
+__global__ void __launch_bounds__(256) window_sort_kernel(BatchSample sample, uint32_t mask, const int32_t* __restrict__ keys,
+                                                          int64_t n, const uint32_t* __restrict__ counted,
                                                           uint32_t* __restrict__ cursor, int32_t* __restrict__ sorted) {
     constexpr int kEach = kSortKeys / 256;
     __shared__ uint32_t count[kMaxWindows], local[kMaxWindows];
     __shared__ int64_t shift_to[kMaxWindows];   // place in the sorted batch less place in the tile
     __shared__ int32_t stage[kSortKeys * DIM];
     __shared__ uint8_t window[kSortKeys];
-    const int64_t first = (int64_t)blockIdx.x * kSortKeys;
-    count[threadIdx.x] = 0;
-    __syncthreads();
-    int k[kEach][3], w[kEach];
-    uint32_t rank[kEach];
+    if (!sample.sorts()) return;
+    const uint32_t start = prefix_256(counted[threadIdx.x]);   // of the thread's window in the sorted batch
+    for (int64_t first = (int64_t)blockIdx.x * kSortKeys; first < n; first += (int64_t)gridDim.x * kSortKeys) {
+        count[threadIdx.x] = 0;
+        __syncthreads();
+        int k[kEach][3], w[kEach];
+        uint32_t rank[kEach];
 #pragma unroll
-    for (int j = 0; j < kEach; ++j) {
-        const int64_t i = first + j * 256 + threadIdx.x;
-        w[j] = -1;
-        if (i < n) {
-            w[j] = window_of<DIM>(keys, i, mask, k[j]);
-            rank[j] = atomicAdd(count + w[j], 1u);
+        for (int j = 0; j < kEach; ++j) {
+            const int64_t i = first + j * 256 + threadIdx.x;
+            w[j] = -1;
+            if (i < n) {
+                w[j] = window_of<DIM>(keys, i, mask, k[j]);
+                rank[j] = atomicAdd(count + w[j], 1u);
+            }
         }
-    }
-    __syncthreads();
-    const uint32_t at = prefix_256(count[threadIdx.x]);
-    local[threadIdx.x] = at;
-    if (count[threadIdx.x])
-        shift_to[threadIdx.x] = (int64_t)atomicAdd(cursor + threadIdx.x, count[threadIdx.x]) - (int64_t)at;
-    __syncthreads();
+        __syncthreads();
+        const uint32_t at = prefix_256(count[threadIdx.x]);
+        local[threadIdx.x] = at;
+        if (count[threadIdx.x])
+            shift_to[threadIdx.x] = (int64_t)start + (int64_t)atomicAdd(cursor + threadIdx.x, count[threadIdx.x]) - (int64_t)at;
+        __syncthreads();
 #pragma unroll
-    for (int j = 0; j < kEach; ++j) {
-        if (w[j] < 0) continue;
-        const uint32_t place = local[w[j]] + rank[j];
-        window[place] = (uint8_t)w[j];
+        for (int j = 0; j < kEach; ++j) {
+            if (w[j] < 0) continue;
+            const uint32_t place = local[w[j]] + rank[j];
+            window[place] = (uint8_t)w[j];
 #pragma unroll
-        for (int d = 0; d < DIM; ++d) stage[place * DIM + d] = k[j][d];
+            for (int d = 0; d < DIM; ++d) stage[place * DIM + d] = k[j][d];
+        }
+        __syncthreads();
+        const int have = (int)min((int64_t)kSortKeys, n - first);
+        // word by word: a window's keys are a contiguous run here and there
+        for (int e = threadIdx.x; e < have * DIM; e += 256) {
+            const int place = e / DIM;
+            sorted[(shift_to[window[place]] + place) * DIM + (e - place * DIM)] = stage[e];
+        }
+        __syncthreads();   // the tile is used again
     }
-    __syncthreads();
-    const int have = (int)min((int64_t)kSortKeys, n - first);
-    // word by word: a window's keys are a contiguous run here and there
-    for (int e = threadIdx.x; e < have * DIM; e += 256) {
-        const int place = e / DIM;
-        sorted[(shift_to[window[place]] + place) * DIM + (e - place * DIM)] = stage[e];
+}
+
+template <int DIM>
+__global__ void __launch_bounds__(256) insert_sorted_kernel(Table16Lines t, BatchSample sample, const int32_t* __restrict__ batch,
+                                                            const int32_t* __restrict__ sorted, int64_t n,
+                                                            int32_t* __restrict__ heap, int32_t* counter, int32_t capacity) {
+    const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
+    t.whole_lines = sample.sorts();
+    int64_t slot = -1;
+    if (i < n) {
+        int k0, k1, k2, k3;
+        load_key<DIM>(t.whole_lines ? sorted : batch, i, k0, k1, k2, k3);
+        bool present = false;
+        slot = emplace(t, k0, k1, k2, k3, kPending, &present);
     }
+    const int idx = pop_index_for_slot_cta(t, slot, heap, counter, capacity);
+    if (idx >= 0) publish_index(t, slot, idx);
 }
 
 // ---- erase -----------------------------------------------------------------------
@@ -766,9 +827,13 @@ static bool sorts_by_window(const ashb_map* m, int64_t n) {
            m->n_slots <= (uint64_t)kMaxWindows << kWindowShift && (uint64_t)n >= m->n_slots / 8 && n < (int64_t)1 << 32;
 }
 
+// Words of the workspace before the sorted keys: window counts, the windows' cursors, repeats in the sample (padded to
+// 16 bytes) and the sample's set, all zeroed.
+constexpr int64_t kWorkspaceHead = 2 * kMaxWindows + 4 + kSampleSlots;
+
 int64_t ashb_map_insert_workspace(ashb_map* m, int64_t n) {
     if (m == nullptr || m->slots == nullptr || n < 0 || !sorts_by_window(m, n)) return 0;
-    return 2 * kMaxWindows * (int64_t)sizeof(uint32_t) + n * m->key_dim * (int64_t)sizeof(int32_t);
+    return (kWorkspaceHead + n * m->key_dim) * (int64_t)sizeof(int32_t);
 }
 
 int ashb_map_insert_keys_sorted(ashb_map* m, const int32_t* keys, int64_t n, void* workspace, int64_t workspace_bytes,
@@ -779,19 +844,21 @@ int ashb_map_insert_keys_sorted(ashb_map* m, const int32_t* keys, int64_t n, voi
     ASHB_REQUIRE(keys && workspace && ((uintptr_t)workspace & 15) == 0 && workspace_bytes >= need, "null or small workspace");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     uint32_t* count = static_cast<uint32_t*>(workspace);
-    uint32_t* cursor = count + kMaxWindows;
-    int32_t* sorted = reinterpret_cast<int32_t*>(cursor + kMaxWindows);
+    uint32_t *cursor = count + kMaxWindows, *repeats = cursor + kMaxWindows;
+    uint32_t* seen = repeats + 4;
+    int32_t* sorted = reinterpret_cast<int32_t*>(seen + kSampleSlots);
     const uint32_t mask = (uint32_t)(m->n_slots - 1);
-    Table16Lines t{table16_of(m)};
-    ValueCtx none;
-    std::memset(&none, 0, sizeof(none));
-    ASHB_CUDA_TRY(cudaMemsetAsync(count, 0, kMaxWindows * sizeof(uint32_t), st));
-    const unsigned tiles = blocks_for(n, kSortKeys), counters = wave_grid(n, 256, 8), grid = blocks_for(n, 256);
+    const uint64_t s = kSampleRuns * 256ull;
+    const BatchSample sample{repeats, (uint32_t)(8 * s * s / m->n_slots)};
+    const Table16Lines t{table16_of(m), true};
+    ASHB_CUDA_TRY(cudaMemsetAsync(workspace, 0, kWorkspaceHead * sizeof(uint32_t), st));
+    const unsigned tiles = std::min(blocks_for(n, kSortKeys), (unsigned)sm_count() * 4u);   // as many as fit: 62 registers
+    const unsigned counters = (unsigned)sm_count() * 8u, grid = blocks_for(n, 256);
 #define ASHB_SORTED_INSERT(DIM)                                                                                       \
-    window_count_kernel<DIM><<<counters, 256, 0, st>>>(mask, keys, n, count);                                          \
-    window_start_kernel<<<1, 256, 0, st>>>(count, cursor);                                                            \
-    window_sort_kernel<DIM><<<tiles, 256, 0, st>>>(mask, keys, n, cursor, sorted);                                     \
-    insert_kernel<Table16Lines, DIM><<<grid, 256, 0, st>>>(t, sorted, n, m->heap, m->counter, (int32_t)m->capacity, none)
+    batch_sample_kernel<DIM><<<kSampleRuns, 256, 0, st>>>(keys, n, seen, repeats);                                     \
+    window_count_kernel<DIM><<<counters, 256, 0, st>>>(sample, mask, keys, n, count);                                  \
+    window_sort_kernel<DIM><<<tiles, 256, 0, st>>>(sample, mask, keys, n, count, cursor, sorted);                      \
+    insert_sorted_kernel<DIM><<<grid, 256, 0, st>>>(t, sample, keys, sorted, n, m->heap, m->counter, (int32_t)m->capacity)
     switch (m->key_dim) {
         case 1: ASHB_SORTED_INSERT(1); break;
         case 2: ASHB_SORTED_INSERT(2); break;
