@@ -11,8 +11,8 @@
 //              as one bit of a byte per cell, so the number of distinct vertices is counted in the
 //              same pass, as is the number of triangles
 //   (host reads the two counts and allocates)
-//   vertices   per 1024 cells: requested edges get consecutive slots and positions
-//   triangles  per 1024 cells: triangles get consecutive slots, vertex ids looked up at the owners
+//   vertices   per 1024 cells (256 in short lists): requested edges get consecutive slots and positions
+//   triangles  likewise: triangles get consecutive slots, vertex ids looked up at the owners
 //
 // The last three are bound by instructions and latency, not bytes: what they shed is work per CELL where only one
 // cell in twelve carries surface.  24,000 blocks of 8^3 on a B200: 444 + 114 + 107 us when every cell
@@ -83,10 +83,14 @@ __device__ __forceinline__ int request_edges(uint8_t* wanted, int64_t a, uint32_
     return __popc(bits & ~(old >> at));
 }
 
-// Marks the vertices of the cell at flat address `a` as placed; returns whether they were.
-__device__ __forceinline__ bool claimed(uint8_t* wanted, int64_t a) {
-    const int at = (int)(a & 3) * 8;
-    return (atomicOr(reinterpret_cast<uint32_t*>(wanted + (a - (a & 3))), kHasVertices << at) >> at) & kHasVertices;
+// Marks the vertices of the requested cells among the four at flat address `a` (a multiple of 4) as placed; returns the
+// requests (bits 0..2 of each byte) that this call marked first: a block may be listed twice.
+__device__ __forceinline__ uint32_t claim_vertices(uint8_t* wanted, int64_t a, uint32_t cells) {
+    uint32_t* word = reinterpret_cast<uint32_t*>(wanted + a);
+    const uint32_t want = *word & 0x07070707u & cells;
+    if (want == 0u) return 0u;
+    const uint32_t marks = ((want | want >> 1 | want >> 2) & 0x01010101u) << 3;
+    return want & ~((atomicOr(word, marks) >> 3 & 0x01010101u) * 7u);
 }
 
 // Raises odd_tables unless corner k of cell (x, y, z) is, in both cell tables, the cell at + k's offsets.
@@ -287,7 +291,10 @@ __global__ void __launch_bounds__(256, kClassifyCtas) mc_classify_kernel(const f
     if (tid < 2 && sums[tid]) atomicAdd(counters + tid, (unsigned long long)sums[tid]);
 }
 
-constexpr int kPassCells = 1024;   // cells of one CTA of the two passes below: 4 per thread
+// Cells of a thread in the two passes below: four in large lists, one up to here, where CTAs of 1024 cells would be less
+// than two per SM, each working off a list of round trips (grid.marching_cubes of 125 and of 343 blocks of 8^3 full of
+// surface: 212 -> 169 and 214 -> 171 us).
+constexpr int kFewCells = 300000;
 
 // Exclusive prefix of `mine` over the CTA of 256 threads, and the start of its range of `cursor`.
 __device__ __forceinline__ int reserve_range(int mine, unsigned long long* cursor, int& total, int64_t& base) {
@@ -315,49 +322,59 @@ __device__ __forceinline__ int reserve_range(int mine, unsigned long long* curso
     return before + incl - mine;
 }
 
-// Four cells per thread read their request bytes; the requested edges of the CTA are listed in shared
+// The threads read the request bytes of their cells; the requested edges of the CTA are listed in shared
 // memory and the list is worked off by all threads, so positions are computed without idle lanes
 // and leave as one contiguous run.
+template <int EACH>
 __global__ void __launch_bounds__(256) mc_vertex_kernel(const float* __restrict__ sdfs, McLuts L,
                                                         const int32_t* __restrict__ grid_coords,
                                                         const int32_t* __restrict__ cell_coords, McEdges edges,
                                                         unsigned long long* __restrict__ cursor,
                                                         float* __restrict__ vertices, int64_t max_vertices,
                                                         float iso_value, int grid_dim) {
-    __shared__ uint16_t list[3 * kPassCells];
-    const int64_t i0 = (int64_t)blockIdx.x * kPassCells;
-    uint32_t bits[4];
-    int64_t address[4];
+    __shared__ uint16_t list[3 * 256 * EACH];
+    const int64_t i0 = (int64_t)blockIdx.x * 256 * EACH;
+    uint32_t bits[EACH];
+    int64_t address[EACH];
     int mine = 0;
+    // block and cell of the thread's j-th cell as its flat address, or -1
+    auto address_of = [&](int j) -> int64_t {
+        const int64_t i = i0 + EACH * threadIdx.x + j;
+        if (i >= L.len) return -1;
+        int64_t pos, cell_idx;
+        L.split(i, pos, cell_idx);
+        const int64_t grid_idx = L.grid_indices[pos];
+        return grid_idx >= 0 && grid_idx < L.n_emb ? grid_idx * L.cells + cell_idx : -1;
+    };
+    if (EACH == 4 && (L.cells & 3) == 0) {   // one word of one block
+        const int64_t a = address_of(0);
+        const uint32_t want = a >= 0 ? claim_vertices(edges.wanted, a, ~0u) : 0u;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        const int64_t i = i0 + 4 * threadIdx.x + j;
-        bits[j] = 0;
-        address[j] = 0;
-        if (i < L.len) {
-            int64_t pos, cell_idx;
-            L.split(i, pos, cell_idx);
-            const int64_t grid_idx = L.grid_indices[pos];
-            if (grid_idx >= 0 && grid_idx < L.n_emb) {
-                address[j] = grid_idx * L.cells + cell_idx;
-                bits[j] = edges.wanted[address[j]] & 7u;
-            }
+        for (int j = 0; j < EACH; ++j) {
+            address[j] = a + j;
+            bits[j] = (want >> (8 * j)) & 7u;
         }
-        // a block may be listed twice: whichever listing comes first places the cell's vertices
-        if (bits[j] && claimed(edges.wanted, address[j])) bits[j] = 0;
-        mine += __popc(bits[j]);
+    } else {
+#pragma unroll
+        for (int j = 0; j < EACH; ++j) {
+            const int64_t a = address[j] = address_of(j);
+            const int at = (int)(a & 3) * 8;
+            bits[j] = a >= 0 ? claim_vertices(edges.wanted, a - (a & 3), 0xFFu << at) >> at : 0u;
+        }
     }
+#pragma unroll
+    for (int j = 0; j < EACH; ++j) mine += __popc(bits[j]);
     int total;
     int64_t base;
     int at = reserve_range(mine, cursor, total, base);
     if (total == 0) return;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
+    for (int j = 0; j < EACH; ++j) {
         if (bits[j] == 0) continue;
         edges.first_vertex[address[j]] = (int)(base + at);
 #pragma unroll
         for (int d = 0; d < 3; ++d)
-            if (bits[j] & (1u << d)) list[at++] = (uint16_t)((4 * threadIdx.x + j) * 4 + d);
+            if (bits[j] & (1u << d)) list[at++] = (uint16_t)((EACH * threadIdx.x + j) * 4 + d);
     }
     __syncthreads();
     for (int e = threadIdx.x; e < total; e += 256) {
@@ -379,20 +396,21 @@ __global__ void __launch_bounds__(256) mc_vertex_kernel(const float* __restrict_
 }
 
 // The same for triangles: the CTA lists them, then a thread per corner looks its vertex up.
+template <int EACH>
 __global__ void __launch_bounds__(256) mc_triangle_kernel(McLuts L, const uint8_t* __restrict__ codes, McEdges edges,
                                                           unsigned long long* __restrict__ cursor,
                                                           int32_t* __restrict__ triangles, int64_t max_triangles) {
-    __shared__ uint16_t list[ASHB_MC_MAX_TRIS * kPassCells];
-    __shared__ uint8_t code_of[kPassCells];
-    const int64_t i0 = (int64_t)blockIdx.x * kPassCells;
-    int count[4];
+    __shared__ uint16_t list[ASHB_MC_MAX_TRIS * 256 * EACH];
+    __shared__ uint8_t code_of[256 * EACH];
+    const int64_t i0 = (int64_t)blockIdx.x * 256 * EACH;
+    int count[EACH];
     int mine = 0;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        const int64_t i = i0 + 4 * threadIdx.x + j;
+    for (int j = 0; j < EACH; ++j) {
+        const int64_t i = i0 + EACH * threadIdx.x + j;
         const int code = i < L.len ? codes[i] : 0;
         count[j] = code ? (int)kMcTriCount[code] : 0;
-        code_of[4 * threadIdx.x + j] = (uint8_t)code;
+        code_of[EACH * threadIdx.x + j] = (uint8_t)code;
         mine += count[j];
     }
     int total;
@@ -400,8 +418,8 @@ __global__ void __launch_bounds__(256) mc_triangle_kernel(McLuts L, const uint8_
     int at = reserve_range(mine, cursor, total, base);
     if (total == 0) return;
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
-        for (int t = 0; t < count[j]; ++t) list[at++] = (uint16_t)((4 * threadIdx.x + j) * 8 + t);
+    for (int j = 0; j < EACH; ++j)
+        for (int t = 0; t < count[j]; ++t) list[at++] = (uint16_t)((EACH * threadIdx.x + j) * 8 + t);
     __syncthreads();
     for (int m = threadIdx.x; m < 3 * total; m += 256) {
         const int t = m / 3, v = m - 3 * t;
@@ -500,11 +518,14 @@ int ashb_marching_cubes_fill(const float* sdfs, const int64_t* grid_indices, con
     const McLuts L = mc_luts(grid_indices, lut_grid_nb2grid_idx, lut_cell_nb2cell_idx, lut_cell_nb2grid_nb, cells_per_grid,
                              n_emb, num_grids);
     const McEdges edges = mc_edges(edge_vertex, n_emb * cells_per_grid);
-    const unsigned grid = (unsigned)((L.len + kPassCells - 1) / kPassCells);
-    mc_vertex_kernel<<<grid, 256, 0, st>>>(sdfs, L, grid_coords_table, cell_coords_table, edges, counters, vertices,
-                                           n_vertices, iso_value, grid_dim);
+    const bool few = L.len < kFewCells;
+    const int64_t pass_cells = few ? 256 : 1024;
+    const unsigned grid = (unsigned)((L.len + pass_cells - 1) / pass_cells);
+    (few ? mc_vertex_kernel<1> : mc_vertex_kernel<4>)<<<grid, 256, 0, st>>>(
+            sdfs, L, grid_coords_table, cell_coords_table, edges, counters, vertices, n_vertices, iso_value, grid_dim);
     ASHB_LAUNCH_CHECK();
-    mc_triangle_kernel<<<grid, 256, 0, st>>>(L, codes, edges, counters + 1, triangles, n_triangles);
+    (few ? mc_triangle_kernel<1> : mc_triangle_kernel<4>)<<<grid, 256, 0, st>>>(L, codes, edges, counters + 1, triangles,
+                                                                                n_triangles);
     ASHB_LAUNCH_CHECK();
     return ASHB_OK;
 }
