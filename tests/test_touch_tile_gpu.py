@@ -45,3 +45,19 @@ def test_frames(H, W, step, dilation):
     TSDFFusion(grid, dilation).fuse_frame(ash.DotDict(
         depth=depth, depth_scale=1.0, depth_max=3000.0, intrinsic=K, extrinsic=np.eye(4), rgb=torch.rand(H, W, 3, device=DEV)))
     np.testing.assert_array_equal(_blocks(grid), ref)
+
+
+@pytest.mark.parametrize("n,dilation", [(5_000, 2), (60_000, 2), (150_000, 1), (300_000, 1)])
+def test_scattered_points(n, dilation):
+    """A block each: the neighbours of 512 points are shared out among eight, four, two and one CTA."""
+    import ash
+    from oracle.tsdf import touched_blocks
+
+    g = torch.Generator(device=DEV).manual_seed(n)
+    pts = torch.rand(n, 3, generator=g, device=DEV) - 0.5
+    ref = touched_blocks(pts.cpu().numpy(), 0.01, [0, 0, 0], 8, dilation)
+    grid = ash.UnBoundedSparseDenseGrid(3, len(ref), 1, 8, cell_size=0.01, device=DEV)
+    coords, _, index, _ = grid.spatial_init_(pts, dilation=dilation, bidirectional=True)
+    np.testing.assert_array_equal(_blocks(grid), ref)
+    assert torch.equal(torch.sort(index.view(-1)).values, torch.arange(len(ref), device=DEV))
+    assert torch.equal(grid.engine.find(coords.view(-1, 3))[0], index.view(-1))
