@@ -291,7 +291,8 @@ class HashMap:
         recorded, rows = torch.is_grad_enabled(), []
         for v in tables.values():
             if type(v) not in (torch.Tensor, torch.nn.Parameter) or v.is_conj() or v.is_neg() or not v.is_contiguous() \
-                    or v.device != self._device or (recorded and v.requires_grad) or v.shape[:1] != (self._capacity,):
+                    or v.device != self._device or (recorded and v.requires_grad) or v.dim() == 0 \
+                    or v.shape[0] != self._capacity:
                 return None
             # a thread copies a row in the widest words that its length and address allow: 15 of them 39 against 45 us for
             # 100k keys and 1.28 against 1.86 ms for 16M, 31 of them 54 against 50 us, 63 of them 6.2 against 5.4 ms
