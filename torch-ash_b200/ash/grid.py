@@ -338,7 +338,8 @@ class SparseDenseGrid(ASHModule):
         """In-place ``size``^3 Gaussian smoothing of every embedding channel.  The window is an outer
         product, so on the GPU it runs as three 1-D passes inside the shared-memory tile of the
         convolution (``separable_gaussian``; same values up to the order of the sums) instead of
-        ``size``^3 taps per cell."""
+        ``size``^3 taps per cell.  Reports keys that the map dropped, so the host waits for the work
+        before it: not for stream capture."""
         assert size % 2 == 1, "size must be odd"
         channels = self.embeddings.shape[-1]
         radius = size // 2
@@ -423,7 +424,7 @@ class SparseDenseGrid(ASHModule):
     def construct_grid_neighbor_lut(self, radius: int, bidirectional: bool):
         """Per-block tables ``(grid_coords (num_embeddings, 3) int32, lut_grid_nb2grid_idx
         (num_embeddings, K) int64)``; rows of inactive blocks and absent neighbours hold -1
-        (ash/grid.py:566-617)."""
+        (ash/grid.py:566-617).  Reports keys that the map dropped: not for stream capture."""
         if self.device.type == "cuda" and 0 <= radius <= 64 and hasattr(backend, "grid_build_window_lut"):
             # one table scan in which a warp probes a block's window; no enumeration (64: as far as the kernel goes)
             with self.engine._status_reported("An earlier insertion"):
