@@ -686,8 +686,8 @@ def tsdf_fuse_frames(hashmap, embeddings, grid_dim, depths, colors, K, E, Ei, de
     """A sequence of equally sized frames in ONE native call: ``depths`` / ``colors`` lists of contiguous
     float32 CUDA tensors (H, W) / (H, W, 3); ``K`` (n, 3, 3), ``E`` and ``Ei`` (n, >=3, 4) float64 numpy arrays
     (intrinsics, world -> camera, camera -> world).  When ``touched_list`` holds two lists (2 x num_embeddings
-    entries) and ``touched_count`` two counters, the allocation pass of every frame overlaps the fusion of
-    the frame before it."""
+    entries) and ``touched_count`` two counters, the frames go in batches of up to 32: the second list holds which of
+    them touch a block."""
     import numpy as np
 
     n = len(depths)

@@ -113,7 +113,7 @@ class TSDFFusion:
     @torch.no_grad()
     def fuse_dataset(self, frames, counter=None) -> None:
         """Fuse a sequence of frames (demo/rgbd_fusion.py:256-262).  Frames of one size and depth_max on the
-        GPU go to the library as ONE call that enqueues both launches of every frame back to back."""
+        GPU go to the library as ONE call that enqueues two launches per batch of frames back to back."""
         frames = list(frames)
         g = self.grid
         same = (len(frames) > 1 and hasattr(backend, "tsdf_fuse_frames") and all(
@@ -132,7 +132,7 @@ class TSDFFusion:
         E = np.stack([_host_matrix(f.extrinsic) for f in frames])
         Ei = np.linalg.inv(E)
         org, lo3, hi3 = self._c_frame_arrays()
-        if self._list2 is None:   # two work lists: the allocation of a frame overlaps the fusion of the one before
+        if self._list2 is None:   # work list, and per block the frames of a batch that touch it
             self._list2 = torch.zeros(2 * g.num_embeddings, dtype=torch.int32, device=g.device)
             self._count2 = torch.zeros(2, dtype=torch.int32, device=g.device)
         backend.tsdf_fuse_frames(

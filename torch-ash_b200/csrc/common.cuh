@@ -68,6 +68,52 @@ __device__ __forceinline__ uint32_t hash_key(int k0, int k1, int k2, int k3) {
     return h;
 }
 
+// Twice the bits of the smallest of four magnitudes, less one: zeros wrap and count as the largest.
+__device__ __forceinline__ uint32_t least_magnitude(float a, float b, float c, float e) {
+    return min(min(2u * __float_as_uint(a) - 1u, 2u * __float_as_uint(b) - 1u),
+               min(2u * __float_as_uint(c) - 1u, 2u * __float_as_uint(e) - 1u));
+}
+__device__ __forceinline__ bool all_zero(float a, float b, float c, float e) { return least_magnitude(a, b, c, e) == 0xFFFFFFFFu; }
+
+// Quotients that share a positive divisor, each equal to __fdiv_rn(a, d) bit for bit.  Markstein's theorem (P. Markstein,
+// IBM J. Res. Dev. 34, 1990): with y = RN(1 / d) and q within one unit of a / d, q - (q d - a) y rounds to RN(a / d).
+// a * y is within two units, one correction brings it within one and the second is the theorem's: one reciprocal and five
+// operations a quotient.  Holds where nothing over- or underflows, and for zeros (which keep their sign); `exact` says
+// whether it does for a numerator, the caller divides where not.
+struct SharedDivisor {
+    float d, y;
+    bool plain;
+    __device__ __forceinline__ explicit SharedDivisor(float divisor) {
+        d = divisor;
+        y = __frcp_rn(divisor);
+        plain = divisor >= 0x1p-30f && divisor <= 0x1p30f;
+    }
+    __device__ __forceinline__ bool exact(float a, float b, float c, float e) const {
+        const float most = fmaxf(fmaxf(fabsf(a), fabsf(b)), fmaxf(fabsf(c), fabsf(e)));   // a NaN divides to NaN either way
+        return plain && most <= 0x1p90f && least_magnitude(a, b, c, e) >= 2u * 0x12800000u - 1u;   // 2^-90
+    }
+    __device__ __forceinline__ float quotient(float a) const {
+        float q = __fmul_rn(a, y);
+        q = __fmaf_rn(-__fmaf_rn(q, d, -a), y, q);
+        return __fmaf_rn(-__fmaf_rn(q, d, -a), y, q);
+    }
+    // The N numerators of `a` divided in place.
+    template <int N>
+    __device__ __forceinline__ void divide(float (&a)[N]) const {
+        static_assert(N == 2 || N == 4, "");
+        if (exact(a[0], a[1], a[N - 2], a[N - 1])) {
+#pragma unroll
+            for (int k = 0; k < N; ++k) a[k] = quotient(a[k]);
+        } else {
+#pragma unroll
+            for (int k = 0; k < N; ++k) {
+                asm volatile("" : "+f"(a[k]));   // or both sides are computed and one is picked
+                a[k] = __fdiv_rn(a[k], d);
+            }
+        }
+    }
+};
+
 __device__ __forceinline__ unsigned lanemask_lt() {
     unsigned m;
     asm("mov.u32 %0, %%lanemask_lt;" : "=r"(m));

@@ -16,6 +16,9 @@
 //             10 KB of a block (512 cells x 5 floats) is staged in shared memory with
 //             coalesced 16-byte accesses, every cell is projected into the frame and
 //             fused, and the block is written back the same way.
+//
+// A sequence goes in batches of frames: the allocation pass marks which frames touch each block and the
+// fusion pass applies them to a block in their order.
 #include <mutex>
 
 #include "hashmap.cuh"
@@ -28,10 +31,22 @@ static __device__ __align__(256) unsigned char g_tsdf_static_scratch[ASHB_TSDF_S
 
 namespace ashb {
 
-struct Camera {
-    float K[9];    // intrinsic, row major
-    float E[12];   // world -> camera, rows of [R | t]
-    float Ei[12];  // camera -> world, rows of [R' | c]
+// A frame as one of the two passes sees it.
+struct View {
+    float K[9];     // intrinsic, row major
+    float pose[12]; // rows of [R | t]: camera -> world for the allocation, world -> camera for the fusion
+    const float* depth;
+    const float* color;
+};
+
+// Frames of one launch.  A sequence goes in batches of this many (a bit each in a block's word): a launch of one frame spends
+// more time starting and running dry than at work (a 640 x 480 frame is 3,400 blocks for 1,184 resident CTAs), and a
+// block that several frames see is loaded and stored once.  100 frames of 3,340 blocks, allocation beside the fusion of
+// the frame before on a second stream: 31 us a frame; in batches of 4, 8, 16, 32: 28.8, 26.2, 24.4, 23.5.
+constexpr int kBatch = 32;
+template <int N>
+struct Views {
+    View view[N];
 };
 
 // Every product and sum below is individually rounded (no fused multiply-add), so the
@@ -56,11 +71,34 @@ struct TouchTarget {
     uint32_t stamp;
     int32_t* touched_list;
     int32_t* touched_count;
+    uint32_t* frames;   // of a batch: bit f of a block's word is set when frame f touches it; null for a single frame
 };
 
-// Insert-if-absent of block (kx, ky, kz), its coordinate recorded and its stamp set; appended to the
-// compact list by the first toucher of the call.
-__device__ __forceinline__ void touch_block(const Table16& t, const TouchTarget& tt, int kx, int ky, int kz) {
+// Row of a block that another thread of this launch is inserting, once that thread has published it; -1 when it found no
+// free row.  The owner waits for nothing between its claim and the row; the wait is bounded all the same.
+__device__ __noinline__ int index_of_pending(const Table16& t, int kx, int ky, int kz) {
+    uint32_t s = hash_key(kx, ky, kz, 0) & t.mask, probe = 0;
+    for (int spin = 0; probe <= t.mask;) {
+        const Entry e = t.read_fresh(s);
+        if (e.val == kEmpty) return -1;
+        if (e.val != kTomb && key_match(e, kx, ky, kz, 0)) {
+            if (e.val >= 0) return e.val;
+            if (++spin == kSpinLimit) {
+                atomicOr(t.status, ASHB_STATUS_SPIN);
+                return -1;
+            }
+            continue;
+        }
+        s = (s + 1) & t.mask;
+        ++probe;
+    }
+    return -1;
+}
+
+// Insert-if-absent of block (kx, ky, kz), its coordinate recorded and its stamp (of a batch: the bit of `frame`) set;
+// appended to the compact list by the first toucher of the call.
+template <bool BATCH>
+__device__ __forceinline__ void touch_block(const Table16& t, const TouchTarget& tt, int kx, int ky, int kz, int frame) {
     if (tt.bounded && (kx < tt.lo.x || ky < tt.lo.y || kz < tt.lo.z || kx >= tt.hi.x || ky >= tt.hi.y || kz >= tt.hi.z))
         return;
     // fast path: the block exists already (probe at L2: this launch mutates the table)
@@ -80,25 +118,34 @@ __device__ __forceinline__ void touch_block(const Table16& t, const TouchTarget&
     if (idx < 0) {
         bool present = false;
         const int64_t slot = emplace(t, kx, ky, kz, 0, kPending, &present);
-        if (slot < 0) return;  // another thread of this launch owns it and stamps it
-        const int top = atomicAdd(tt.counter, 1);
-        if (top >= tt.capacity) {
-            atomicSub(tt.counter, 1);
-            *reinterpret_cast<volatile int*>(t.val_ptr((uint32_t)slot)) = kTomb;
-            atomicOr(t.status, ASHB_STATUS_CAPACITY);
-            return;
+        if (slot < 0) {
+            // another thread of this launch owns it and stamps it -- for its own frame
+            if (!BATCH || !present) return;
+            idx = index_of_pending(t, kx, ky, kz);
+            if (idx < 0) return;
+        } else {
+            const int top = atomicAdd(tt.counter, 1);
+            if (top >= tt.capacity) {
+                atomicSub(tt.counter, 1);
+                *reinterpret_cast<volatile int*>(t.val_ptr((uint32_t)slot)) = kTomb;
+                atomicOr(t.status, ASHB_STATUS_CAPACITY);
+                return;
+            }
+            idx = tt.heap[top];
+            *reinterpret_cast<volatile int*>(t.val_ptr((uint32_t)slot)) = idx;
         }
-        idx = tt.heap[top];
-        *reinterpret_cast<volatile int*>(t.val_ptr((uint32_t)slot)) = idx;
     }
     // many pixels of a frame fall in the same few thousand blocks: whoever finds the block already
     // stamped by this call has nothing left to do (the first toucher recorded it)
-    if (__ldcg(&tt.touched[idx]) == tt.stamp) return;
+    const uint32_t bit = 1u << frame;
+    if (BATCH ? (__ldcg(&tt.frames[idx]) & bit) != 0u : __ldcg(&tt.touched[idx]) == tt.stamp) return;
     // the coordinate is recorded for blocks allocated by other means too
     tt.grid_coords[3 * idx] = kx;
     tt.grid_coords[3 * idx + 1] = ky;
     tt.grid_coords[3 * idx + 2] = kz;
-    if (tt.touched_list) {
+    if (BATCH) {
+        if (atomicOr(&tt.frames[idx], bit) == 0u) tt.touched_list[atomicAdd(tt.touched_count, 1)] = idx;
+    } else if (tt.touched_list) {
         // first toucher of the call appends the block to the compact work list
         if (atomicExch(&tt.touched[idx], tt.stamp) != tt.stamp) tt.touched_list[atomicAdd(tt.touched_count, 1)] = idx;
     } else {
@@ -150,9 +197,9 @@ constexpr int kCrowded = 64;
 
 // Called by ALL 256 threads of a CTA, each with two points (`valid` ones carry a block), in no order if SCATTERED.
 // `slices` (a power of two) CTAs may be given the same points: `slice` of them takes the blocks whose coordinates say so.
-template <bool SCATTERED>
+template <bool SCATTERED, bool BATCH>
 __device__ __forceinline__ void touch_neighbourhoods(const Table16& t, const TouchTarget& tt, const bool* valid,
-                                                     const int3* block, unsigned slices, unsigned slice) {
+                                                     const int3* block, unsigned slices, unsigned slice, int frame) {
     constexpr uint32_t kOwnTag = 1u << 30, kNeighbourTag = 1u << 31;
     __shared__ TouchTile tile;
     for (int i = threadIdx.x; i < kSeenSlots; i += 256) tile.seen[i] = 0u;
@@ -187,7 +234,8 @@ __device__ __forceinline__ void touch_neighbourhoods(const Table16& t, const Tou
         for (int which = threadIdx.x >> 5; which < tile.n_blocks; which += 8) {
             const int3 b = tile.blocks[which];
             for (int k = threadIdx.x & 31; k < n_nb; k += 32)
-                touch_block(t, tt, b.x + tt.lo_off + k % w, b.y + tt.lo_off + (k / w) % w, b.z + tt.lo_off + k / (w * w));
+                touch_block<BATCH>(t, tt, b.x + tt.lo_off + k % w, b.y + tt.lo_off + (k / w) % w, b.z + tt.lo_off + k / (w * w),
+                                   frame);
             __syncwarp();
         }
         return;
@@ -198,7 +246,7 @@ __device__ __forceinline__ void touch_neighbourhoods(const Table16& t, const Tou
         const int x = tile.blocks[which].x + tt.lo_off + k % w, y = tile.blocks[which].y + tt.lo_off + (k / w) % w,
                   z = tile.blocks[which].z + tt.lo_off + k / (w * w);
         const uint32_t word = tile_word(o, x, y, z, kNeighbourTag);
-        if (word == 0u || first_seen(tile.seen, word)) touch_block(t, tt, x, y, z);
+        if (word == 0u || first_seen(tile.seen, word)) touch_block<BATCH>(t, tt, x, y, z, frame);
     }
 }
 
@@ -208,9 +256,12 @@ __device__ __forceinline__ int block_of(float w, float org, float inv_cell, floa
     return (int)floorf(__fmul_rn(__fmul_rn(__fsub_rn(w, org), inv_cell), inv_G));
 }
 
-__global__ void __launch_bounds__(256, 6) tsdf_touch_kernel(Table16 t, TouchTarget tt, const float* __restrict__ depth,
-                                                         int H, int W, Camera cam, float depth_max, float inv_cell,
-                                                         float3 origin, float inv_G) {
+// CTAs (x, f) are those of frame f of the N of a batch.
+template <int N>
+__global__ void __launch_bounds__(256, 6) tsdf_touch_kernel(Table16 t, TouchTarget tt, const __grid_constant__ Views<N> views,
+                                                            int H, int W, float depth_max, float inv_cell, float3 origin,
+                                                            float inv_G) {
+    const View& cam = views.view[N == 1 ? 0 : blockIdx.y];
     bool valid[2];
     int3 block[2];
     const unsigned tiles_x = ((unsigned)W + 31) / 32;
@@ -218,19 +269,19 @@ __global__ void __launch_bounds__(256, 6) tsdf_touch_kernel(Table16 t, TouchTarg
 #pragma unroll
     for (int j = 0; j < 2; ++j) {
         const int v = (int)(blockIdx.x / tiles_x) * 16 + j * 8 + (int)(threadIdx.x >> 5);
-        const float d = u < W && v < H ? depth[(int64_t)v * W + u] : 0.f;
+        const float d = u < W && v < H ? __ldg(cam.depth + (int64_t)v * W + u) : 0.f;
         valid[j] = d > 0.f && d < depth_max;
         block[j] = make_int3(0, 0, 0);
         if (valid[j]) {
             // camera point of pixel (u, v) at depth d for K = [fx 0 cx; 0 fy cy; 0 0 1]
             const float xc = __fdiv_rn(__fmul_rn(__fsub_rn((float)u, cam.K[2]), d), cam.K[0]);
             const float yc = __fdiv_rn(__fmul_rn(__fsub_rn((float)v, cam.K[5]), d), cam.K[4]);
-            block[j] = make_int3(block_of(affine3(cam.Ei, xc, yc, d), origin.x, inv_cell, inv_G),
-                                 block_of(affine3(cam.Ei + 4, xc, yc, d), origin.y, inv_cell, inv_G),
-                                 block_of(affine3(cam.Ei + 8, xc, yc, d), origin.z, inv_cell, inv_G));
+            block[j] = make_int3(block_of(affine3(cam.pose, xc, yc, d), origin.x, inv_cell, inv_G),
+                                 block_of(affine3(cam.pose + 4, xc, yc, d), origin.y, inv_cell, inv_G),
+                                 block_of(affine3(cam.pose + 8, xc, yc, d), origin.z, inv_cell, inv_G));
         }
     }
-    touch_neighbourhoods<false>(t, tt, valid, block, 1, 0);
+    touch_neighbourhoods<false, (N > 1)>(t, tt, valid, block, 1, 0, N == 1 ? 0 : (int)blockIdx.y);
 }
 
 // SparseDenseGrid.spatial_init_ (ash/grid.py:121-159) without its temporary hash set: two points per thread.
@@ -248,79 +299,175 @@ __global__ void __launch_bounds__(256, 6) points_touch_kernel(Table16 t, TouchTa
                                  block_of(pts[3 * i + 1], origin.y, inv_cell, inv_G),
                                  block_of(pts[3 * i + 2], origin.z, inv_cell, inv_G));
     }
-    touch_neighbourhoods<true>(t, tt, valid, block, gridDim.y, blockIdx.y);
+    touch_neighbourhoods<true, false>(t, tt, valid, block, gridDim.y, blockIdx.y, 0);
 }
 
 // ---- integrate ---------------------------------------------------------------------
+// Bound by instructions (205 a cell and view) and by the latency of the image loads.  A CTA of 128 threads with a double tile
+// and four cells of a thread in flight, eight to an SM: 14.4 us a frame in a sequence.  Ten to an SM with two in
+// flight 17.3 (their tiles leave L1 too small for the images), 256 threads 16.6, 64 threads 17.7.
+constexpr int kIntegrateThreads = 128, kIntegrateResident = 8, kCellGroup = 4;
+constexpr float kRound = 12582912.f;   // 1.5 * 2^23
+
 struct IntegrateFrame {
-    const float* __restrict__ depth;
-    const float* __restrict__ color;
     int H, W;
-    Camera cam;
     float depth_max, cell_size;
     float3 origin;
     int G, cells;
     float trunc;
     int sdf_ch, rgb_ch, w_ch;
+    int D;
     int G_shift;   // log2(G), or -1
+    float u_end, v_end;   // W and H above kRound
+    int usual;   // every intrinsic is [fx 0 cx; 0 fy cy; 0 0 1], and W and H are at most 2^22
+    uint32_t* frames;   // of a batch: which frames touched a block, set back to none here; null for a single frame
+    uint32_t* touched;  // of a batch: a block is given the stamp of its last frame
+    uint32_t first_stamp;
 };
 
-// One observation fused into every cell of block (gx, gy, gz), whose rows sit in `tile` (cells * D floats).
-template <int D>
-__device__ __forceinline__ void integrate_cells(float* tile, int gx, int gy, int gz, const IntegrateFrame& f) {
-    const int G = f.G;
-    for (int c = threadIdx.x; c < f.cells; c += blockDim.x) {
-        int cx, cy, cz;
-        if (f.G_shift >= 0) {   // three divisions would be a quarter of a cell's instructions
-            cx = c & (G - 1), cy = (c >> f.G_shift) & (G - 1), cz = c >> (2 * f.G_shift);
-        } else {
-            cx = c % G, cy = (c / G) % G, cz = c / (G * G);
-        }
-        // cell_to_world: (block * G + cell) * cell_size (+ origin for bounded grids)
-        const float px = __fadd_rn(__fmul_rn((float)(gx * G + cx), f.cell_size), f.origin.x);
-        const float py = __fadd_rn(__fmul_rn((float)(gy * G + cy), f.cell_size), f.origin.y);
-        const float pz = __fadd_rn(__fmul_rn((float)(gz * G + cz), f.cell_size), f.origin.z);
-        const float x = affine3(f.cam.E, px, py, pz);
-        const float y = affine3(f.cam.E + 4, px, py, pz);
-        const float z = affine3(f.cam.E + 8, px, py, pz);
-        const float un = dot3(f.cam.K, x, y, z);
-        const float vn = dot3(f.cam.K + 3, x, y, z);
-        const float d = dot3(f.cam.K + 6, x, y, z);
-        float w = 0.f, sdf = 0.f, r = 0.f, g = 0.f, b = 0.f;
-        if (d > 0.f) {
-            const float uf = rintf(__fdiv_rn(un, d)), vf = rintf(__fdiv_rn(vn, d));  // torch.round: half to even
-            if (uf >= 0.f && vf >= 0.f && uf < (float)f.W && vf < (float)f.H) {
-                const int u = (int)uf, v = (int)vf;
-                const float dr = __ldg(f.depth + (int64_t)v * f.W + u);
-                const float* col = f.color + ((int64_t)v * f.W + u) * 3;
-                r = __ldg(col), g = __ldg(col + 1), b = __ldg(col + 2);
-                sdf = __fsub_rn(dr, d);
-                if (dr > 0.f && dr < f.depth_max && sdf >= -f.trunc) w = 1.f;
-                if (sdf >= f.trunc) sdf = f.trunc;
+// What a view observes at a cell.
+struct Observation {
+    float d, depth, r, g, b;
+    bool seen;
+};
+
+// The pixel that camera coordinates (x, y, z) project to, and its loads.  USUAL: see IntegrateFrame; the general product
+// gives the same pixels, as products with the intrinsic's zeros change no sum that passes the tests below.
+template <bool USUAL>
+__device__ __forceinline__ Observation observe(float x, float y, float z, const IntegrateFrame& f, const View& view) {
+    Observation o{z, 0.f, 0.f, 0.f, 0.f, false};
+    float un, vn;
+    int u = 0, v = 0;
+    if (USUAL) {
+        un = __fadd_rn(__fmul_rn(view.K[0], x), __fmul_rn(view.K[2], z));
+        vn = __fadd_rn(__fmul_rn(view.K[4], y), __fmul_rn(view.K[5], z));
+    } else {
+        un = dot3(view.K, x, y, z);
+        vn = dot3(view.K + 3, x, y, z);
+        o.d = dot3(view.K + 6, x, y, z);
+    }
+    // torch.round of the quotients: half to even.  A numerator beyond what the shared division is exact for has a quotient that
+    // rounds to 0, or beyond every image, either way.  Adding kRound rounds and leaves the whole number in the low
+    // bits where it is below 2^22 (conversions run at a quarter of the rate).
+    const SharedDivisor by(o.d);
+    if (USUAL && by.plain) {
+        const float um = __fadd_rn(by.quotient(un), kRound), vm = __fadd_rn(by.quotient(vn), kRound);
+        o.seen = um >= kRound && vm >= kRound && um < f.u_end && vm < f.v_end;
+        u = __float_as_int(um) - __float_as_int(kRound), v = __float_as_int(vm) - __float_as_int(kRound);
+    } else if (o.d > 0.f) {
+        const float uf = rintf(__fdiv_rn(un, o.d)), vf = rintf(__fdiv_rn(vn, o.d));
+        o.seen = uf >= 0.f && vf >= 0.f && uf < (float)f.W && vf < (float)f.H;
+        u = (int)uf, v = (int)vf;
+    }
+    if (o.seen) {
+        const int64_t pixel = (int64_t)v * f.W + u;
+        const float* color = view.color + pixel * 3;
+        o.depth = __ldg(view.depth + pixel);
+        o.r = __ldg(color), o.g = __ldg(color + 1), o.b = __ldg(color + 2);
+    }
+    return o;
+}
+
+// The observation fused into its cell (D floats at `cell`).
+__device__ __forceinline__ void fuse_cell(float* cell, const Observation& o, const IntegrateFrame& f) {
+    // outside the image or behind the camera the observation has weight 0 and its
+    // value does not matter (demo/rgbd_fusion.py:93-108)
+    float w = 0.f, sdf = 0.f;
+    if (o.seen) {
+        sdf = __fsub_rn(o.depth, o.d);
+        if (o.depth > 0.f && o.depth < f.depth_max && sdf >= -f.trunc) w = 1.f;
+        if (sdf >= f.trunc) sdf = f.trunc;
+    }
+    float* rgb = cell + f.rgb_ch;
+    const float w_sum = cell[f.w_ch];
+    // demo/rgbd_fusion.py:247-249: mean' = (mean * w_sum + obs * w) / (w_sum + w + 1e-6); obs * w is exact
+    const float w_new = __fadd_rn(w_sum, w);
+    const float den = __fadd_rn(w_new, 1e-6f);
+    auto sum = [&](float mean, float obs) { return __fmaf_rn(obs, w, __fmul_rn(mean, w_sum)); };
+    float mean[4] = {sum(cell[f.sdf_ch], sdf), sum(rgb[0], o.r), sum(rgb[1], o.g), sum(rgb[2], o.b)};
+    // A cell that no frame has observed has sums of zero, and zero over a positive number keeps its sign.
+    if (!(all_zero(mean[0], mean[1], mean[2], mean[3]) && den > 0.f)) SharedDivisor(den).divide(mean);
+    cell[f.sdf_ch] = mean[0];
+    rgb[0] = mean[1];
+    rgb[1] = mean[2];
+    rgb[2] = mean[3];
+    cell[f.w_ch] = w_new;
+}
+
+// One view fused into every cell of block (gx, gy, gz), whose rows sit in `tile` (cells * D floats).
+// GT: the block edge where it is known when compiling, 0 otherwise.  Where the CTA covers whole layers of the block (GT of
+// 4, 8) a thread stays in one column of cells and the x and y parts of its camera coordinates are formed once.
+template <int GT, bool USUAL>
+__device__ __forceinline__ void integrate_cells(float* tile, int gx, int gy, int gz, const IntegrateFrame& f, const View& view) {
+    constexpr int kLayers = GT ? kIntegrateThreads / (GT * GT) : 0;   // that the CTA covers at once
+    const int G = GT ? GT : f.G;
+    // cell_to_world: (block * G + cell) * cell_size (+ origin for bounded grids)
+    auto world = [&](int b, int c, float origin) { return __fadd_rn(__fmul_rn((float)(b * G + c), f.cell_size), origin); };
+    const float* E = view.pose;
+    if constexpr (kLayers > 0) {
+        constexpr int kEach = GT / kLayers > 0 ? GT / kLayers : 1, kGroup = kEach < kCellGroup ? kEach : kCellGroup;
+        const int t = threadIdx.x, cx = t % G, cy = t / G % G, cz0 = t / (G * G);
+        if (cz0 >= G) return;
+        const float px = world(gx, cx, f.origin.x), py = world(gy, cy, f.origin.y);
+        float xy[3];   // affine3 as far as it does not depend on z
+#pragma unroll
+        for (int k = 0; k < 3; ++k) xy[k] = __fadd_rn(__fmul_rn(E[4 * k], px), __fmul_rn(E[4 * k + 1], py));
+#pragma unroll 1
+        for (int j = 0; j < kEach; j += kGroup) {
+            Observation o[kGroup];
+#pragma unroll
+            for (int i = 0; i < kGroup; ++i) {
+                const float pz = world(gz, cz0 + (j + i) * kLayers, f.origin.z);
+                float p[3];
+#pragma unroll
+                for (int k = 0; k < 3; ++k) p[k] = __fadd_rn(__fadd_rn(xy[k], __fmul_rn(E[4 * k + 2], pz)), E[4 * k + 3]);
+                o[i] = observe<USUAL>(p[0], p[1], p[2], f, view);
             }
+#pragma unroll
+            for (int i = 0; i < kGroup; ++i) fuse_cell(tile + (t + (j + i) * kIntegrateThreads) * f.D, o[i], f);
         }
-        // outside the image or behind the camera the observation has weight 0 and its
-        // value does not matter (demo/rgbd_fusion.py:93-108)
-        float* cell = tile + c * D;
-        const float w_sum = cell[f.w_ch];
-        // demo/rgbd_fusion.py:247-249: mean' = (mean * w_sum + obs * w) / (w_sum + w + 1e-6)
-        const float w_new = __fadd_rn(w_sum, w);
-        const float den = __fadd_rn(w_new, 1e-6f);
-        auto fuse = [&](float mean, float obs) {
-            return __fdiv_rn(__fadd_rn(__fmul_rn(mean, w_sum), __fmul_rn(obs, w)), den);
-        };
-        cell[f.sdf_ch] = fuse(cell[f.sdf_ch], sdf);
-        cell[f.rgb_ch] = fuse(cell[f.rgb_ch], r);
-        cell[f.rgb_ch + 1] = fuse(cell[f.rgb_ch + 1], g);
-        cell[f.rgb_ch + 2] = fuse(cell[f.rgb_ch + 2], b);
-        cell[f.w_ch] = w_new;
+    } else {
+        for (int c = threadIdx.x; c < f.cells; c += blockDim.x) {
+            int cx, cy, cz;
+            if (f.G_shift >= 0) {   // three divisions would be a quarter of a cell's instructions
+                cx = c & (G - 1), cy = (c >> f.G_shift) & (G - 1), cz = c >> (2 * f.G_shift);
+            } else {
+                cx = c % G, cy = (c / G) % G, cz = c / (G * G);
+            }
+            const float px = world(gx, cx, f.origin.x), py = world(gy, cy, f.origin.y), pz = world(gz, cz, f.origin.z);
+            fuse_cell(tile + c * f.D,
+                      observe<USUAL>(affine3(E, px, py, pz), affine3(E + 4, px, py, pz), affine3(E + 8, px, py, pz), f, view), f);
+        }
     }
 }
 
-template <int D>
-__global__ void __launch_bounds__(256, 8) tsdf_integrate_kernel(
+// The frames of `frames` in their order.  A thread's cells are its own: nothing to wait for between two frames.
+template <int GT, int N>
+__device__ __forceinline__ void fuse_frames(float* tile, const int32_t* coords, uint32_t frames, const IntegrateFrame& f,
+                                            const Views<N>& views) {
+    const int gx = coords[0], gy = coords[1], gz = coords[2];
+#pragma unroll 1
+    for (; frames; frames &= frames - 1) {
+        const View& view = views.view[N == 1 ? 0 : __ffs(frames) - 1];
+        if (f.usual) integrate_cells<GT, true>(tile, gx, gy, gz, f, view);
+        else integrate_cells<0, false>(tile, gx, gy, gz, f, view);
+        if (N == 1) break;
+    }
+}
+
+// One thread, after the CTA has read the block's word.
+__device__ __forceinline__ void finish_block(int64_t idx, uint32_t frames, const IntegrateFrame& f, unsigned long long* n_integrated) {
+    if (f.frames) {
+        f.frames[idx] = 0u;
+        f.touched[idx] = f.first_stamp + (31 - __clz(frames));
+    }
+    if (n_integrated) atomicAdd(n_integrated, (unsigned long long)__popc(frames));
+}
+
+template <int GT, int N>
+__global__ void __launch_bounds__(kIntegrateThreads, kIntegrateResident) tsdf_integrate_kernel(
         float* __restrict__ emb, const int32_t* __restrict__ grid_coords, const uint32_t* __restrict__ touched,
-        uint32_t stamp, IntegrateFrame f, unsigned long long* n_integrated, int64_t n_emb,
+        uint32_t stamp, const __grid_constant__ IntegrateFrame f, const __grid_constant__ Views<N> views, unsigned long long* n_integrated, int64_t n_emb,
         const int32_t* __restrict__ touched_list, const int32_t* __restrict__ touched_count) {
     extern __shared__ float tile[];  // cells * D floats
     // Work items: the compact list written by the touch kernel (a few persistent CTAs walk it),
@@ -329,8 +476,8 @@ __global__ void __launch_bounds__(256, 8) tsdf_integrate_kernel(
     for (int64_t item = blockIdx.x; item < n_items; item += gridDim.x) {
         const int64_t idx = touched_list ? (int64_t)touched_list[item] : item;
         if (!touched_list && touched[idx] != stamp) continue;
-        float* block = emb + idx * (int64_t)f.cells * D;
-        const int n_float = f.cells * D;
+        const int n_float = f.cells * f.D;
+        float* block = emb + idx * (int64_t)n_float;
         // rows are 16-byte aligned when cells * D * 4 is a multiple of 16
         const bool vec_ok = (n_float & 3) == 0 && (((uintptr_t)block) & 15) == 0;
         if (vec_ok) {
@@ -340,15 +487,16 @@ __global__ void __launch_bounds__(256, 8) tsdf_integrate_kernel(
             for (int i = threadIdx.x; i < n_float; i += blockDim.x) tile[i] = block[i];
         }
         __syncthreads();
-        integrate_cells<D>(tile, grid_coords[3 * idx], grid_coords[3 * idx + 1], grid_coords[3 * idx + 2], f);
+        const uint32_t frames = N > 1 ? f.frames[idx] : 1u;
+        fuse_frames<GT, N>(tile, grid_coords + 3 * idx, frames, f, views);
         __syncthreads();
+        if (threadIdx.x == 0) finish_block(idx, frames, f, n_integrated);
         if (vec_ok) {
             for (int i = threadIdx.x; i < n_float / 4; i += blockDim.x)
                 reinterpret_cast<float4*>(block)[i] = reinterpret_cast<const float4*>(tile)[i];
         } else {
             for (int i = threadIdx.x; i < n_float; i += blockDim.x) block[i] = tile[i];
         }
-        if (threadIdx.x == 0 && n_integrated) atomicAdd(n_integrated, 1ull);
         __syncthreads();  // the tile is reused by the next item
     }
 }
@@ -382,14 +530,14 @@ __device__ __forceinline__ bool wait_phase(uint32_t bar, uint32_t parity) {
 // turns.  A block's rows are one contiguous, 16-byte aligned stretch of cells * D * 4 bytes (a multiple
 // of 16: checked by the host).  Every wait has an iteration limit; a CTA whose wait runs out counts it
 // in g_tsdf_copy_timeouts, waits for its own stores and stops.
-template <int D>
-__global__ void __launch_bounds__(256, 8) tsdf_integrate_bulk_kernel(
-        float* __restrict__ emb, const int32_t* __restrict__ grid_coords, IntegrateFrame f,
+template <int GT, int N>
+__global__ void __launch_bounds__(kIntegrateThreads, kIntegrateResident) tsdf_integrate_bulk_kernel(
+        float* __restrict__ emb, const int32_t* __restrict__ grid_coords, const __grid_constant__ IntegrateFrame f, const __grid_constant__ Views<N> views,
         unsigned long long* n_integrated, const int32_t* __restrict__ touched_list,
         const int32_t* __restrict__ touched_count) {
     extern __shared__ __align__(128) float tiles[];  // 2 tiles of cells * D floats
     __shared__ __align__(8) unsigned long long full[2];
-    const int n_float = f.cells * D;
+    const int n_float = f.cells * f.D;
     const uint32_t bytes = (uint32_t)n_float * 4u;
     const int64_t n_items = (int64_t)*touched_count;
     const bool boss = threadIdx.x == 0;
@@ -429,7 +577,8 @@ __global__ void __launch_bounds__(256, 8) tsdf_integrate_bulk_kernel(
         }
         float* tile = tiles + (int64_t)buf * n_float;
         const int64_t idx = touched_list[item];
-        integrate_cells<D>(tile, grid_coords[3 * idx], grid_coords[3 * idx + 1], grid_coords[3 * idx + 2], f);
+        const uint32_t frames = N > 1 ? f.frames[idx] : 1u;
+        fuse_frames<GT, N>(tile, grid_coords + 3 * idx, frames, f, views);
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the tile as written, visible to the copy engine
         __syncthreads();
         if (boss) {
@@ -437,7 +586,7 @@ __global__ void __launch_bounds__(256, 8) tsdf_integrate_bulk_kernel(
                          "r"(smem_address(tile)), "r"(bytes)
                          : "memory");
             asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-            if (n_integrated) atomicAdd(n_integrated, 1ull);
+            finish_block(idx, frames, f, n_integrated);
         }
     }
     if (boss) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");   // stores complete before the CTA's memory goes
@@ -479,30 +628,51 @@ static int make_touch_target(ashb_map* m, int dilation, int bidirectional, const
     return ASHB_OK;
 }
 
+// The allocation pass of n_frames frames (bits of `frames`, or a single one).
+static int touch_impl(ashb_map* m, int n_frames, const float* const* depths, int H, int W, const float* intrinsics,
+                      const float* cam_to_worlds, float depth_max, double cell_size, const float* origin, int G,
+                      int dilation, const int32_t* bound_lo, const int32_t* bound_hi, int32_t* grid_coords,
+                      uint32_t* touched, uint32_t stamp, int32_t* touched_list, int32_t* touched_count, uint32_t* frames,
+                      void* stream) {
+    TouchTarget tt;
+    if (int rc = make_touch_target(m, dilation, 1, bound_lo, bound_hi, grid_coords, touched, stamp, touched_list,
+                                   touched_count, &tt))
+        return rc;
+    tt.frames = frames;
+    ASHB_REQUIRE(intrinsics && cam_to_worlds && origin, "null buffer");
+    ASHB_REQUIRE(H > 0 && W > 0 && G > 0 && cell_size > 0.0, "bad frame or grid geometry");
+    DeviceGuard guard(m->device);
+    Views<kBatch> views;   // the first n_frames are set
+    for (int f = 0; f < n_frames; ++f) {
+        View& v = views.view[f];
+        for (int i = 0; i < 9; ++i) v.K[i] = intrinsics[9 * f + i];
+        for (int i = 0; i < 12; ++i) v.pose[i] = cam_to_worlds[12 * f + i];
+        v.depth = depths[f];
+        ASHB_REQUIRE(v.depth != nullptr, "null buffer");
+        ASHB_REQUIRE(v.K[0] != 0.f && v.K[4] != 0.f && v.K[1] == 0.f && v.K[3] == 0.f,
+                     "intrinsic must be a skew-free pinhole matrix");
+    }
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    if (touched_count) ASHB_CUDA_TRY(cudaMemsetAsync(touched_count, 0, sizeof(int32_t), st));
+    const dim3 grid((unsigned)(((int64_t)W + 31) / 32 * (((int64_t)H + 15) / 16)), (unsigned)n_frames);
+    const float3 org = make_float3(origin[0], origin[1], origin[2]);
+    const float inv_cell = (float)(1.0 / cell_size), inv_G = 1.0f / (float)G;
+    if (frames)
+        tsdf_touch_kernel<kBatch><<<grid, 256, 0, st>>>(table16_of(m), tt, views, H, W, depth_max, inv_cell, org, inv_G);
+    else
+        tsdf_touch_kernel<1><<<grid, 256, 0, st>>>(table16_of(m), tt, Views<1>{{views.view[0]}}, H, W, depth_max, inv_cell,
+                                                   org, inv_G);
+    ASHB_LAUNCH_CHECK();
+    return ASHB_OK;
+}
+
 int ashb_tsdf_touch(ashb_map* m, const float* depth, int H, int W, const float* intrinsic,
                     const float* cam_to_world, float depth_max, double cell_size, const float* origin, int G,
                     int dilation, const int32_t* bound_lo, const int32_t* bound_hi, int32_t* grid_coords,
                     uint32_t* touched, uint32_t stamp, int32_t* touched_list, int32_t* touched_count,
                     void* stream) {
-    TouchTarget tt;
-    if (int rc = make_touch_target(m, dilation, 1, bound_lo, bound_hi, grid_coords, touched, stamp, touched_list,
-                                   touched_count, &tt))
-        return rc;
-    ASHB_REQUIRE(depth && intrinsic && cam_to_world && origin, "null buffer");
-    ASHB_REQUIRE(H > 0 && W > 0 && G > 0 && cell_size > 0.0, "bad frame or grid geometry");
-    DeviceGuard guard(m->device);
-    Camera cam{};
-    for (int i = 0; i < 9; ++i) cam.K[i] = intrinsic[i];
-    for (int i = 0; i < 12; ++i) cam.Ei[i] = cam_to_world[i];
-    ASHB_REQUIRE(cam.K[0] != 0.f && cam.K[4] != 0.f && cam.K[1] == 0.f && cam.K[3] == 0.f,
-                 "intrinsic must be a skew-free pinhole matrix");
-    cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (touched_count) ASHB_CUDA_TRY(cudaMemsetAsync(touched_count, 0, sizeof(int32_t), st));
-    tsdf_touch_kernel<<<(unsigned)(((int64_t)W + 31) / 32 * (((int64_t)H + 15) / 16)), 256, 0, st>>>(
-            table16_of(m), tt, depth, H, W, cam, depth_max, (float)(1.0 / cell_size),
-            make_float3(origin[0], origin[1], origin[2]), 1.0f / (float)G);
-    ASHB_LAUNCH_CHECK();
-    return ASHB_OK;
+    return touch_impl(m, 1, &depth, H, W, intrinsic, cam_to_world, depth_max, cell_size, origin, G, dilation, bound_lo,
+                      bound_hi, grid_coords, touched, stamp, touched_list, touched_count, nullptr, stream);
 }
 
 int ashb_grid_spatial_init(ashb_map* m, const float* points, int64_t n, double cell_size, const float* origin, int G,
@@ -532,79 +702,75 @@ int ashb_grid_spatial_init(ashb_map* m, const float* points, int64_t n, double c
     return ASHB_OK;
 }
 
-// ctas_per_sm: most CTAs of a work list's pass that an SM takes.
+// The fusion pass of n_frames frames: the blocks of a batch's `frames` words, or those of a single stamp.
 static int integrate_impl(void* embeddings, int64_t n_emb, int G, int64_t D, const int32_t* grid_coords,
-                          const uint32_t* touched, uint32_t stamp, const float* depth, const float* color, int H,
-                          int W, const float* intrinsic, const float* world_to_cam, float depth_max,
-                          double cell_size, const float* origin, float trunc, int sdf_channel, int rgb_channel,
-                          int weight_channel, unsigned long long* n_integrated_dev, const int32_t* touched_list,
-                          const int32_t* touched_count, int ctas_per_sm, void* stream) {
+                          uint32_t* touched, uint32_t stamp, int n_frames, const float* const* depths,
+                          const float* const* colors, int H, int W, const float* intrinsics, const float* world_to_cams,
+                          float depth_max, double cell_size, const float* origin, float trunc, int sdf_channel,
+                          int rgb_channel, int weight_channel, unsigned long long* n_integrated_dev,
+                          const int32_t* touched_list, const int32_t* touched_count, uint32_t* frames, void* stream) {
     ASHB_REQUIRE((touched_list == nullptr) == (touched_count == nullptr), "pass both the list and its counter, or neither");
-    ASHB_REQUIRE(embeddings && grid_coords && touched && depth && color && intrinsic && world_to_cam && origin,
-                 "null buffer");
+    ASHB_REQUIRE(embeddings && grid_coords && touched && intrinsics && world_to_cams && origin, "null buffer");
     ASHB_REQUIRE(n_emb >= 1 && G >= 1 && G <= 16 && H > 0 && W > 0, "bad sizes");
     ASHB_REQUIRE(D >= 5 && D <= 16, "embedding_dim %lld cannot hold sdf + rgb + weight", (long long)D);
     ASHB_REQUIRE(sdf_channel >= 0 && sdf_channel < D && weight_channel >= 0 && weight_channel < D &&
                          rgb_channel >= 0 && rgb_channel + 2 < D,
                  "channel layout out of range");
-    Camera cam{};
-    for (int i = 0; i < 9; ++i) cam.K[i] = intrinsic[i];
-    for (int i = 0; i < 12; ++i) cam.E[i] = world_to_cam[i];
+    Views<kBatch> views;   // the first n_frames are set
+    int usual = W <= 1 << 22 && H <= 1 << 22;
+    for (int f = 0; f < n_frames; ++f) {
+        View& v = views.view[f];
+        for (int i = 0; i < 9; ++i) v.K[i] = intrinsics[9 * f + i];
+        for (int i = 0; i < 12; ++i) v.pose[i] = world_to_cams[12 * f + i];
+        v.depth = depths[f];
+        v.color = colors[f];
+        ASHB_REQUIRE(v.depth && v.color, "null buffer");
+        usual &= v.K[1] == 0.f && v.K[3] == 0.f && v.K[6] == 0.f && v.K[7] == 0.f && v.K[8] == 1.f;
+    }
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const int cells = G * G * G;
     const size_t smem = (size_t)cells * D * sizeof(float);
     ASHB_REQUIRE(smem <= 200 * 1024, "block of %zu bytes does not fit in shared memory", smem);
-    const IntegrateFrame frame{depth, color, H, W, cam, depth_max, (float)cell_size,
-                               make_float3(origin[0], origin[1], origin[2]), G, cells, trunc, sdf_channel, rgb_channel,
-                               weight_channel, (G & (G - 1)) == 0 ? 31 - __builtin_clz((unsigned)G) : -1};
+    const IntegrateFrame frame{H, W, depth_max, (float)cell_size, make_float3(origin[0], origin[1], origin[2]), G, cells,
+                               trunc, sdf_channel, rgb_channel, weight_channel, (int)D,
+                               (G & (G - 1)) == 0 ? 31 - __builtin_clz((unsigned)G) : -1, kRound + (float)W,
+                               kRound + (float)H, usual, frames, touched, stamp};
     // The copy-engine variant needs a work list, 16-byte aligned rows of a multiple of 16 bytes, and room
     // for two tiles per CTA; everything else takes the plain kernel.
     const bool bulk = touched_list != nullptr && smem % 16 == 0 && ((uintptr_t)embeddings & 15) == 0 && 2 * smem <= 96 * 1024;
     // with a work list: exactly the CTAs that are resident at once walk it (more would queue behind them
     // as a partly filled second wave); without: one CTA per row
-#define ASHB_TSDF_LAUNCH(DD)                                                                               \
-    case DD: {                                                                                             \
+#define ASHB_TSDF_LAUNCH(GT, N, VIEWS)                                                                     \
+    {                                                                                                      \
         const size_t dyn = bulk ? 2 * smem : smem;                                                         \
-        const void* fn = bulk ? (const void*)tsdf_integrate_bulk_kernel<DD> : (const void*)tsdf_integrate_kernel<DD>; \
+        const void* fn = bulk ? (const void*)tsdf_integrate_bulk_kernel<GT, N> : (const void*)tsdf_integrate_kernel<GT, N>; \
         if (dyn > 48 * 1024)                                                                               \
             ASHB_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn)); \
         int per_sm = 0;                                                                                    \
-        ASHB_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, 256, dyn));               \
-        if (per_sm > ctas_per_sm) per_sm = ctas_per_sm;                                                    \
+        ASHB_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kIntegrateThreads, dyn)); \
         const int64_t resident = (int64_t)sm_count() * (per_sm > 0 ? per_sm : 1);                          \
-        const unsigned launch_ctas = touched_list ? (unsigned)(n_emb < resident ? n_emb : resident) : (unsigned)n_emb; \
+        const unsigned ctas = (unsigned)(touched_list && n_emb > resident ? resident : n_emb);             \
         if (bulk)                                                                                          \
-            tsdf_integrate_bulk_kernel<DD><<<launch_ctas, 256, dyn, st>>>(                                 \
-                    static_cast<float*>(embeddings), grid_coords, frame, n_integrated_dev, touched_list, touched_count); \
+            tsdf_integrate_bulk_kernel<GT, N><<<ctas, kIntegrateThreads, dyn, st>>>(                       \
+                    static_cast<float*>(embeddings), grid_coords, frame, VIEWS, n_integrated_dev, touched_list, touched_count); \
         else                                                                                               \
-            tsdf_integrate_kernel<DD><<<launch_ctas, 256, dyn, st>>>(                                      \
-                    static_cast<float*>(embeddings), grid_coords, touched, stamp, frame, n_integrated_dev, n_emb, \
+            tsdf_integrate_kernel<GT, N><<<ctas, kIntegrateThreads, dyn, st>>>(                            \
+                    static_cast<float*>(embeddings), grid_coords, touched, stamp, frame, VIEWS, n_integrated_dev, n_emb, \
                     touched_list, touched_count);                                                          \
-    } break;
-    switch ((int)D) {
-        ASHB_TSDF_LAUNCH(5)
-        ASHB_TSDF_LAUNCH(6)
-        ASHB_TSDF_LAUNCH(7)
-        ASHB_TSDF_LAUNCH(8)
-        ASHB_TSDF_LAUNCH(9)
-        ASHB_TSDF_LAUNCH(10)
-        ASHB_TSDF_LAUNCH(11)
-        ASHB_TSDF_LAUNCH(12)
-        ASHB_TSDF_LAUNCH(13)
-        ASHB_TSDF_LAUNCH(14)
-        ASHB_TSDF_LAUNCH(15)
-        ASHB_TSDF_LAUNCH(16)
     }
+#define ASHB_TSDF_LAUNCH_N(GT)                                                                             \
+    {                                                                                                      \
+        if (frames) ASHB_TSDF_LAUNCH(GT, kBatch, views)                                                    \
+        else ASHB_TSDF_LAUNCH(GT, 1, Views<1>{{views.view[0]}})                                            \
+    }
+    if (G == 8) ASHB_TSDF_LAUNCH_N(8)
+    else if (G == 4) ASHB_TSDF_LAUNCH_N(4)
+    else ASHB_TSDF_LAUNCH_N(0)
+#undef ASHB_TSDF_LAUNCH_N
 #undef ASHB_TSDF_LAUNCH
     ASHB_LAUNCH_CHECK();
     return ASHB_OK;
 }
-
-// The pass is bound by arithmetic (seven IEEE divisions per cell).  A frame on its own takes all of an SM's thread
-// slots (3,500 blocks: 23.7 us, 26.4 with half of them); where a sequence is fused the allocation pass of the NEXT
-// frame runs beside it on a second stream (ashb_tsdf_fuse_frames) and needs the other half (100 frames: 4.02 ms,
-// 4.26 with all).
-constexpr int kIntegrateCtasAlone = 8, kIntegrateCtasPaired = 4;
 
 int ashb_tsdf_integrate(void* embeddings, int64_t n_emb, int G, int64_t D, const int32_t* grid_coords,
                         const uint32_t* touched, uint32_t stamp, const float* depth, const float* color, int H,
@@ -612,9 +778,9 @@ int ashb_tsdf_integrate(void* embeddings, int64_t n_emb, int G, int64_t D, const
                         double cell_size, const float* origin, float trunc, int sdf_channel, int rgb_channel,
                         int weight_channel, unsigned long long* n_integrated_dev, const int32_t* touched_list,
                         const int32_t* touched_count, void* stream) {
-    return integrate_impl(embeddings, n_emb, G, D, grid_coords, touched, stamp, depth, color, H, W, intrinsic,
-                          world_to_cam, depth_max, cell_size, origin, trunc, sdf_channel, rgb_channel, weight_channel,
-                          n_integrated_dev, touched_list, touched_count, kIntegrateCtasAlone, stream);
+    return integrate_impl(embeddings, n_emb, G, D, grid_coords, const_cast<uint32_t*>(touched), stamp, 1, &depth, &color, H,
+                          W, intrinsic, world_to_cam, depth_max, cell_size, origin, trunc, sdf_channel, rgb_channel,
+                          weight_channel, n_integrated_dev, touched_list, touched_count, nullptr, stream);
 }
 
 // Device address of g_tsdf_static_scratch on the current device.  In host code the array's
@@ -654,34 +820,6 @@ int ashb_tsdf_fuse_frame(ashb_map* m, void* embeddings, int64_t n_emb, int G, in
                                weight_channel, n_integrated_dev, touched_list, touched_count, stream);
 }
 
-// Side stream and events of the two-stage frame pipeline below, one set per device, created on first
-// use and kept for the life of the process.
-struct FramePipeline {
-    cudaStream_t side = nullptr;
-    cudaEvent_t start = nullptr, touched[2] = {nullptr, nullptr}, integrated[2] = {nullptr, nullptr};
-};
-
-static int frame_pipeline_for_current_device(FramePipeline** out) {
-    constexpr int kMaxDevices = 64;
-    static std::mutex mu;
-    static FramePipeline cached[kMaxDevices];
-    int dev = -1;
-    ASHB_CUDA_TRY(cudaGetDevice(&dev));
-    ASHB_REQUIRE(dev >= 0 && dev < kMaxDevices, "device ordinal %d out of range", dev);
-    std::lock_guard<std::mutex> lock(mu);
-    FramePipeline& p = cached[dev];
-    if (p.side == nullptr) {
-        ASHB_CUDA_TRY(cudaStreamCreateWithFlags(&p.side, cudaStreamNonBlocking));
-        ASHB_CUDA_TRY(cudaEventCreateWithFlags(&p.start, cudaEventDisableTiming));
-        for (int i = 0; i < 2; ++i) {
-            ASHB_CUDA_TRY(cudaEventCreateWithFlags(&p.touched[i], cudaEventDisableTiming));
-            ASHB_CUDA_TRY(cudaEventCreateWithFlags(&p.integrated[i], cudaEventDisableTiming));
-        }
-    }
-    *out = &p;
-    return ASHB_OK;
-}
-
 int ashb_tsdf_fuse_frames(ashb_map* m, void* embeddings, int64_t n_emb, int G, int64_t D, int n_frames,
                           const float* const* depths, const float* const* colors, int H, int W,
                           const float* intrinsics, const float* world_to_cams, const float* cam_to_worlds,
@@ -705,36 +843,26 @@ int ashb_tsdf_fuse_frames(ashb_map* m, void* embeddings, int64_t n_emb, int G, i
         }
         return ASHB_OK;
     }
-    // Two-stage pipeline: the allocation pass of frame f + 1 (side stream) runs while frame f is fused
-    // (caller's stream).  The allocation pass writes the hash table, the free-index stack, the stamps and
-    // ITS work list (lists and counts alternate between two buffers); the fusion pass of the frame before
-    // reads its own list, the coordinates of blocks that already exist (re-written with the same values at
-    // most) and embedding rows no allocation touches -- so the two only meet through the events below.
+    // Batches: one allocation pass marks which frames of the batch touch each block, one fusion pass applies them to
+    // it in their order.
     DeviceGuard guard(m->device);
-    FramePipeline* p = nullptr;
-    if (int rc = frame_pipeline_for_current_device(&p)) return rc;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    ASHB_CUDA_TRY(cudaEventRecord(p->start, st));
-    ASHB_CUDA_TRY(cudaStreamWaitEvent(p->side, p->start, 0));   // after whatever the caller enqueued before
-    for (int f = 0; f < n_frames; ++f) {
-        const int b = f & 1;
-        if (f >= 2) ASHB_CUDA_TRY(cudaStreamWaitEvent(p->side, p->integrated[b], 0));   // list b is free again
-        if (int rc = ashb_tsdf_touch(m, depths[f], H, W, intrinsics + 9 * f, cam_to_worlds + 12 * f, depth_max, cell_size,
-                                     origin, G, dilation, bound_lo, bound_hi, grid_coords, touched,
-                                     first_stamp + (uint32_t)f, touched_list + (int64_t)b * n_emb, touched_count + b,
-                                     p->side))
+    uint32_t* frames = reinterpret_cast<uint32_t*>(touched_list + n_emb);
+    ASHB_CUDA_TRY(cudaMemsetAsync(frames, 0, (size_t)n_emb * sizeof(uint32_t), st));
+    for (int f = 0; f < n_frames; f += kBatch) {
+        const int n = n_frames - f < kBatch ? n_frames - f : kBatch;
+        const uint32_t stamp = first_stamp + (uint32_t)f;
+        if (int rc = touch_impl(m, n, depths + f, H, W, intrinsics + 9 * f, cam_to_worlds + 12 * f, depth_max, cell_size,
+                                origin, G, dilation, bound_lo, bound_hi, grid_coords, touched, stamp, touched_list,
+                                touched_count, frames, st))
             return rc;
-        ASHB_CUDA_TRY(cudaEventRecord(p->touched[b], p->side));
-        ASHB_CUDA_TRY(cudaStreamWaitEvent(st, p->touched[b], 0));
-        if (int rc = integrate_impl(embeddings, n_emb, G, D, grid_coords, touched, first_stamp + (uint32_t)f,
-                                         depths[f], colors[f], H, W, intrinsics + 9 * f, world_to_cams + 12 * f,
-                                         depth_max, cell_size, origin, trunc, sdf_channel, rgb_channel, weight_channel,
-                                         n_integrated_dev, touched_list + (int64_t)b * n_emb, touched_count + b,
-                                    kIntegrateCtasPaired, st))
+        if (int rc = integrate_impl(embeddings, n_emb, G, D, grid_coords, touched, stamp, n, depths + f, colors + f, H, W,
+                                    intrinsics + 9 * f, world_to_cams + 12 * f, depth_max, cell_size, origin, trunc,
+                                    sdf_channel, rgb_channel, weight_channel, n_integrated_dev, touched_list,
+                                    touched_count, frames, st))
             return rc;
-        ASHB_CUDA_TRY(cudaEventRecord(p->integrated[b], st));
     }
-    return ASHB_OK;   // the caller's stream has waited for every allocation pass: it is ordered after all the work
+    return ASHB_OK;
 }
 
 int ashb_tsdf_static_max_blocks(void) { return ASHB_TSDF_STATIC_MAX_BLOCKS; }
