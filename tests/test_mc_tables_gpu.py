@@ -86,3 +86,11 @@ def test_more_tiles_than_ctas(G, side):
     """Six CTAs per SM share out the tiles (beyond the staged edge: 256 cells at a time), so each takes more than one."""
     grid, sdf, w = _noisy_grid(G, side, 1)
     _compare_with_oracle(grid, sdf + 2.5, w, 0.0, 1.0)
+
+
+@pytest.mark.parametrize("G", [4, 8, 16])
+def test_values_off_their_alignment(G):
+    """Rows of cells that start where wide loads may not."""
+    grid, sdf, w = _noisy_grid(G, 3, 1)
+    shift = lambda t: torch.cat([t.new_zeros(1), t.view(-1)])[1:].view(t.shape)
+    _compare_with_oracle(grid, shift(sdf), shift(w), 0.1, 1.0)

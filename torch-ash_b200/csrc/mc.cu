@@ -17,7 +17,7 @@
 // The last three are bound by instructions and latency, not bytes: what they shed is work per CELL where only one
 // cell in twelve carries surface.  24,000 blocks of 8^3 on a B200: 444 + 114 + 107 us when every cell
 // read its eight corners through the tables, each warp bumped the shared counters and an edge took
-// four bytes of a 147 MB table that had to be filled, written and read; 130 + 39 + 57 us now.
+// four bytes of a 147 MB table that had to be filled, written and read; 60 + 39 + 57 us now.
 //
 // The triangulation table is this repository's own (mc_tables.h, derived by gen_mc_tables.py):
 // the reference's table is not reproduced, so which diagonal splits an ambiguous pattern, the
@@ -105,39 +105,38 @@ __global__ void __launch_bounds__(256) mc_check_tables_kernel(McLuts L, McEdges 
 }
 
 constexpr int kMaxTileBlocks = 32;
-constexpr int kTileTarget = 1024;   // cells
 constexpr int kMaxFastEdge = 16;
-constexpr int kClassifyCtas = 6;   // per SM: what 40 registers allow
+constexpr int kMaxTileRows = (kMaxFastEdge + 1) * (kMaxFastEdge + 1);   // no less than 256
+constexpr int kClassifyCtas = 6;   // per SM
 
-// A CTA walks tiles of max(1, 1024 / G^3) blocks (a tile has five barriers: the 512 cells of one block of
-// G = 8 are too few).  It stages one state byte per cell of a block AND of the layer that its upper
-// neighbours add, (G + 1)^3 in all, so every value is read once (G = 8: 1.4 loads of sdf and weight per
-// cell instead of 8 of each behind 24 table reads); cubes then read bytes of shared memory.  Requests for
-// the block's own edges meet in shared memory and go out a word at a time; the two counters see one
-// atomic per CTA.  GT: the block edge where it is known when compiling (the halo's divisions), 0
-// otherwise.  Cell tables that are not the usual ones (odd_tables), and edges beyond kMaxFastEdge
-// (G = 0), take the corners from the tables.
+// Bits 0..3 to the low bits of four bytes.
+__device__ __forceinline__ uint32_t spread_bits(uint32_t bits) { return (bits & 15u) * 0x00204081u & 0x01010101u; }
+
+// A CTA walks tiles of blocks: as many as have 256 rows of cells between them, counting the layer of rows that a block's
+// upper neighbours add, (G + 1)^2 a block.  A row of G cells and the neighbour's first one is two words of bits, observed
+// and inside, made by one thread from wide loads (each value is read once, G = 8: 1.27 times); a cube, an edge and
+// whether it is cut are then the same bit of a few such words, for all cells of a row at once.  Only cubes with
+// surface are looked at one by one, for their code.  Requested edges leave as a word of four cells; the two
+// counters see one atomic per CTA.  Bound by latency and the values' traffic: 24,000 blocks of 8^3 60 us, 130 with a
+// state byte per cell, eight of them read per cube and the edges requested corner by corner; a warp per block of
+// 8^3 instead of a CTA per three 56, but 2,000 and 200 blocks 11.5 and 10.6 us for 8.1 and 6.1.
+// GT: the block edge where it is known when compiling, 0 otherwise.  wide: rows and codes are aligned for GT's loads and
+// stores.  Cell tables that are not the usual ones (odd_tables), and edges beyond kMaxFastEdge (G = 0), take the
+// corners from the tables.
 template <int GT>
 __global__ void __launch_bounds__(256, kClassifyCtas) mc_classify_kernel(const float* __restrict__ sdfs,
                                                           const float* __restrict__ weights, McLuts L,
                                                           uint8_t* __restrict__ codes, McEdges edges,
                                                           unsigned long long* __restrict__ counters, float iso_value,
-                                                          float weight_thr, int G_arg, int64_t num_grids) {
-    // largest tile: of kTileTarget cells, of a block with more, and for G not known here of any of either
-    constexpr int kTileCells = GT == 8 || GT == 4 ? kTileTarget : kMaxFastEdge * kMaxFastEdge * kMaxFastEdge;
-    constexpr int kHalo = (GT + 1) * (GT + 1) * (GT + 1);
-    __shared__ uint8_t state[GT == 8 ? 2 * kHalo : GT == 4 ? 16 * kHalo : (kMaxFastEdge + 1) * (kMaxFastEdge + 1) * (kMaxFastEdge + 1)];
-    // where a cell of a block's halo comes from: cell | neighbour << 9; 25 instructions otherwise
-    __shared__ uint16_t halo_cell[GT == 8 || GT == 4 ? kHalo : 1];
-    __shared__ uint32_t own[kTileCells / 4];
-    __shared__ uint32_t active[kTileCells];   // cells with surface: cell of the tile | code << 16
-    __shared__ int n_active;
+                                                          float weight_thr, int G_arg, int64_t num_grids,
+                                                          bool wide) {
+    // behind the last row: what the rows above it read, and then mask
+    __shared__ uint32_t inside[kMaxTileRows + kMaxFastEdge + 1], observed[kMaxTileRows + kMaxFastEdge + 1];
+    __shared__ uint32_t cubes[kMaxTileRows];   // whose eight corners are observed
     __shared__ int64_t rows[kMaxTileBlocks * 8];
-    __shared__ uint16_t edge_mask[256];
     __shared__ uint8_t tri_count[256];
     const int tid = threadIdx.x;
-    edge_mask[tid] = kMcEdgeMask[tid];   // launched with 256 threads
-    tri_count[tid] = kMcTriCount[tid];
+    tri_count[tid] = kMcTriCount[tid];   // launched with 256 threads
     __syncthreads();
     int n_vertices = 0, n_triangles = 0;
     const int G = GT ? GT : G_arg;
@@ -162,22 +161,16 @@ __global__ void __launch_bounds__(256, kClassifyCtas) mc_classify_kernel(const f
             }
             if (!valid || code == 255) code = 0;
             codes[i] = (uint8_t)code;
-            const int mask = edge_mask[code];
+            const int mask = kMcEdgeMask[code];
 #pragma unroll
             for (int e = 0; e < 12; ++e)
                 if (mask & (1 << e)) n_vertices += request_edges(edges.wanted, corner[edge_lower_corner(e)], 1u << (e >> 2));
             n_triangles += tri_count[code];
         }
     } else {
-        const int H = G + 1, halo = H * H * H, cells = G * G * G;
-        const int per_tile = cells >= kTileTarget ? 1 : min(kTileTarget / cells, kMaxTileBlocks);
-        if (GT == 8 || GT == 4) {
-            for (int r = tid; r < halo; r += 256) {
-                const int x = r % H, y = r / H % H, z = r / (H * H);
-                halo_cell[r] = (uint16_t)((x % G + (y % G + z % G * G) * G) | ((x == G) | (y == G) << 1 | (z == G) << 2) << 9);
-            }
-            __syncthreads();
-        }
+        const int H = G + 1, HH = H * H, cells = G * G * G;
+        const uint32_t all_cells = (1u << G) - 1u;
+        const int per_tile = min(max(256 / HH, 1), kMaxTileBlocks);
         const int64_t n_tiles = (num_grids + per_tile - 1) / per_tile;
         // embedding row of one of a tile's blocks or of one of its upper neighbours, or -1
         auto row_of = [&](int64_t tile) -> int64_t {
@@ -187,95 +180,110 @@ __global__ void __launch_bounds__(256, kClassifyCtas) mc_classify_kernel(const f
             const int64_t nb = g >= 0 && g < L.n_emb ? L.g2g[g * 8 + (tid & 7)] : -1;
             return nb < L.n_emb ? nb : -1;
         };
+        // the block of the tile that row r of the tile's halo is in, its y and z there, which neighbour (and the next in x) owns
+        // the row and the flat place of its first cell within a block
+        struct Row {
+            int b, y, z, nb, at;
+        };
+        auto halo_row = [&](int r) {
+            const int b = r / HH, q = r - b * HH, z = q / H, y = q - z * H;
+            return Row{b, y, z, (y == G) << 1 | (z == G) << 2, ((y == G ? 0 : y) + (z == G ? 0 : z) * G) * G};
+        };
         int64_t row = row_of(blockIdx.x);
         for (int64_t tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
             const int64_t first = tile * per_tile;
             const int blocks = per_tile == 1 ? 1 : (int)min((int64_t)per_tile, num_grids - first);
             if (tid < per_tile * 8) rows[tid] = row;
-            for (int w = tid; w < (blocks * cells + 3) / 4; w += 256) own[w] = 0;
-            if (tid == 0) n_active = 0;
             __syncthreads();
             row = row_of(tile + gridDim.x);   // two dependent loads that the rest of the tile covers
-#pragma unroll 3
-            for (int h = tid; h < blocks * halo; h += 256) {
-                const int b = per_tile == 1 ? 0 : h / halo, r = h - b * halo;
-                int nb, at;
-                if (GT == 8 || GT == 4) {
-                    nb = halo_cell[r] >> 9;
-                    at = halo_cell[r] & 511;
-                } else {
-                    const int x = r % H, y = r / H % H, z = r / (H * H);
-                    nb = (x == G) | (y == G) << 1 | (z == G) << 2;
-                    at = (x == G ? 0 : x) + ((y == G ? 0 : y) + (z == G ? 0 : z) * G) * G;
-                }
-                const int64_t g = rows[b * 8 + nb];
-                uint8_t s = 0;   // bit 0: observed, bit 1: inside
-                if (g >= 0) {
-                    const int64_t a = g * cells + at;
-                    const float d = sdfs[a];
-                    s = weights[a] >= weight_thr ? (d - iso_value < 0.f ? 3 : 1) : 0;
-                }
-                state[h] = s;
-            }
-            __syncthreads();
-            for (int c = tid; c < blocks * cells; c += 256) {
-                const int b = per_tile == 1 ? 0 : c / cells, cell = c - b * cells;
-                const int x = cell % G, y = cell / G % G, z = cell / (G * G);
-                const uint8_t* s = state + b * halo + x + (y + z * H) * H;
-                unsigned seen = 1, code = 0;
+            for (int r = tid; r < blocks * HH; r += 256) {
+                const Row h = halo_row(r);
+                const int64_t own = rows[h.b * 8 + h.nb], next = rows[h.b * 8 + h.nb + 1];
+                uint32_t in = 0, seen = 0;
+                auto cell = [&](int x, float d, float w) {
+                    in |= (uint32_t)(d - iso_value < 0.f) << x;
+                    seen |= (uint32_t)(w >= weight_thr) << x;
+                };
+                if (next >= 0) cell(G, sdfs[next * cells + h.at], weights[next * cells + h.at]);
+                if (own >= 0) {
+                    const float *d = sdfs + own * cells + h.at, *w = weights + own * cells + h.at;
+                    if (GT && wide) {
 #pragma unroll
-                for (int k = 0; k < 8; ++k) {
-                    const unsigned v = s[(k & 1) + (((k >> 1) & 1) + (k >> 2) * H) * H];
-                    seen &= v;
-                    code |= (v >> 1) << k;
-                }
-                if (!seen || code == 255) code = 0;
-                codes[first * cells + c] = (uint8_t)code;
-                if (code) active[atomicAdd(&n_active, 1)] = (uint32_t)c | code << 16;
-            }
-            __syncthreads();
-            // a thread per corner of a cube with surface, for the edges that leave it (none leave corner 7)
-            for (int i = tid; i < 7 * n_active; i += 256) {
-                const int which = i / 7, k = i - 7 * which;
-                const uint32_t entry = active[which];
-                const int c = (int)(entry & 0xFFFFu), mask = edge_mask[entry >> 16];
-                uint32_t bits = 0;
-#pragma unroll
-                for (int d = 0; d < 3; ++d) {
-                    const int e = d * 4 + (((k >> ((d + 1) % 3)) & 1) | ((k >> ((d + 2) % 3)) & 1) << 1);
-                    if (((k >> d) & 1) == 0) bits |= (uint32_t)((mask >> e) & 1) << d;
-                }
-                if (k == 0) n_triangles += tri_count[entry >> 16];
-                if (bits) {
-                    const int b = per_tile == 1 ? 0 : c / cells, cell = c - b * cells;
-                    const int cx = cell % G + (k & 1), cy = cell / G % G + ((k >> 1) & 1), cz = cell / (G * G) + (k >> 2);
-                    const int nb = (cx == G) | (cy == G) << 1 | (cz == G) << 2;
-                    const int at = (cx == G ? 0 : cx) + ((cy == G ? 0 : cy) + (cz == G ? 0 : cz) * G) * G;
-                    if (nb == 0) {
-                        const int o = b * cells + at;
-                        atomicOr(own + (o >> 2), bits << ((o & 3) * 8));
+                        for (int x = 0; x < GT; x += 4) {
+                            const float4 d4 = *reinterpret_cast<const float4*>(d + x), w4 = *reinterpret_cast<const float4*>(w + x);
+                            cell(x, d4.x, w4.x), cell(x + 1, d4.y, w4.y), cell(x + 2, d4.z, w4.z), cell(x + 3, d4.w, w4.w);
+                        }
                     } else {
-                        n_vertices += request_edges(edges.wanted, rows[b * 8 + nb] * cells + at, bits);
+                        for (int x = 0; x < G; ++x) cell(x, d[x], w[x]);
                     }
+                }
+                inside[r] = in;
+                observed[r] = seen;
+                if (h.y == G || h.z == G) cubes[r] = 0;
+            }
+            __syncthreads();
+            for (int c = tid; c < blocks * G * G; c += 256) {   // a row of cubes
+                const int b = c / (G * G), yz = c - b * G * G, z = yz / G, y = yz - z * G, r = b * HH + y + z * H;
+                const uint32_t i0 = inside[r], i1 = inside[r + 1], i2 = inside[r + H], i3 = inside[r + H + 1];
+                uint32_t seen = observed[r] & observed[r + 1] & observed[r + H] & observed[r + H + 1];
+                seen &= seen >> 1 & all_cells;
+                cubes[r] = seen;
+                const uint32_t any = i0 | i1 | i2 | i3, all = i0 & i1 & i2 & i3;
+                uint32_t surface = (any | any >> 1) & ~(all & all >> 1) & seen;
+                uint8_t* to = codes + first * cells + (int64_t)b * cells + yz * G;
+                constexpr int kWords = GT ? GT / 4 : 1;
+                uint32_t words[kWords] = {};
+                if (!(GT && wide))
+                    for (int x = 0; x < G; ++x) to[x] = 0;
+                for (; surface; surface &= surface - 1) {
+                    const int x = __ffs(surface) - 1;
+                    const uint32_t code = (i0 >> x & 3u) | (i1 >> x & 3u) << 2 | (i2 >> x & 3u) << 4 | (i3 >> x & 3u) << 6;
+                    n_triangles += tri_count[code];
+                    if (GT && wide) {
+#pragma unroll
+                        for (int k = 0; k < kWords; ++k)
+                            if (x >> 2 == k) words[k] |= code << (8 * (x & 3));
+                    } else {
+                        to[x] = (uint8_t)code;
+                    }
+                }
+                if (GT && wide) {
+                    if constexpr (kWords == 1) *reinterpret_cast<uint32_t*>(to) = words[0];
+#pragma unroll
+                    for (int k = 0; k + 1 < kWords; k += 2) *reinterpret_cast<uint2*>(to + 4 * k) = make_uint2(words[k], words[k + 1]);
                 }
             }
             __syncthreads();
-            for (int w = tid; w < (blocks * cells + 3) / 4; w += 256) {
-                const uint32_t bits = own[w];
-                if (bits == 0) continue;
-                if ((cells & 3) == 0) {   // the word is one of the block's
-                    const int b = per_tile == 1 ? 0 : 4 * w / cells;
-                    const int64_t a = rows[b * 8] * cells + (4 * w - b * cells);
-                    n_vertices += __popc(bits & ~atomicOr(reinterpret_cast<uint32_t*>(edges.wanted + a), bits));
+            for (int r = tid; r < blocks * HH; r += 256) {   // the edges that leave a row's cells, cut and in a cube
+                const Row h = halo_row(r);
+                const uint32_t v = cubes[r], vy = h.y > 0 ? cubes[r - 1] : 0u, vz = h.z > 0 ? cubes[r - H] : 0u,
+                               vyz = h.y > 0 && h.z > 0 ? cubes[r - H - 1] : 0u;
+                if ((v | vy | vz | vyz) == 0u) continue;
+                const uint32_t i = inside[r], cy = v | vz, cz = v | vy;
+                const uint32_t wx = (i ^ i >> 1) & (v | vy | vz | vyz), wy = (i ^ inside[r + 1]) & (cy | cy << 1),
+                               wz = (i ^ inside[r + H]) & (cz | cz << 1);
+                if ((wx | wy | wz) == 0u) continue;
+                const int64_t a = rows[h.b * 8 + h.nb] * cells + h.at;
+                if (GT) {
+                    uint32_t bits[GT ? GT / 4 : 1], old[GT ? GT / 4 : 1];
+#pragma unroll
+                    for (int k = 0; k < GT / 4; ++k) {   // all on their way before the first is waited for
+                        bits[k] = spread_bits(wx >> 4 * k) | spread_bits(wy >> 4 * k) << 1 | spread_bits(wz >> 4 * k) << 2;
+                        old[k] = 0;
+                        if (bits[k]) old[k] = atomicOr(reinterpret_cast<uint32_t*>(edges.wanted + a + 4 * k), bits[k]);
+                    }
+#pragma unroll
+                    for (int k = 0; k < GT / 4; ++k) n_vertices += __popc(bits[k] & ~old[k]);
                 } else {
-                    for (int j = 0; j < 4; ++j) {
-                        const uint32_t one = (bits >> (8 * j)) & 7u;
-                        const int b = (4 * w + j) / cells;
-                        if (one) n_vertices += request_edges(edges.wanted, rows[b * 8] * cells + (4 * w + j - b * cells), one);
+                    for (uint32_t left = (wx | wy | wz) & all_cells; left; left &= left - 1) {
+                        const int x = __ffs(left) - 1;
+                        n_vertices += request_edges(edges.wanted, a + x, (wx >> x & 1u) | (wy >> x & 1u) << 1 | (wz >> x & 1u) << 2);
                     }
                 }
+                const uint32_t last = (wy >> G & 1u) << 1 | (wz >> G & 1u) << 2;   // of the next block's first cell
+                if (last) n_vertices += request_edges(edges.wanted, rows[h.b * 8 + h.nb + 1] * cells + h.at, last);
             }
-            __syncthreads();   // rows and the two tiles are used again
+            __syncthreads();   // rows and the words are used again
         }
     }
     __shared__ int sums[2];
@@ -485,11 +493,12 @@ int ashb_marching_cubes_count(const float* sdfs, const float* weights, const int
         mc_check_tables_kernel<<<(unsigned)((cells_per_grid * 8 + 255) / 256), 256, 0, st>>>(L, edges, G);
         ASHB_LAUNCH_CHECK();
     }
-    // persistent: one resident set of CTAs shares out the tiles (14 each at 24,000 blocks)
+    // persistent: one resident set of CTAs shares out the tiles (9 each at 24,000 blocks)
     const unsigned grid = (unsigned)std::min<int64_t>((L.len + 255) / 256, (int64_t)sm_count() * kClassifyCtas);
+    const bool wide = (((uintptr_t)sdfs | (uintptr_t)weights) & 15) == 0 && ((uintptr_t)codes & 7) == 0;
     auto kernel = G == 8 ? mc_classify_kernel<8> : G == 4 ? mc_classify_kernel<4> : G == 16 ? mc_classify_kernel<16>
                                                                                         : mc_classify_kernel<0>;
-    kernel<<<grid, 256, 0, st>>>(sdfs, weights, L, codes, edges, counters, iso_value, weight_thr, G, num_grids);
+    kernel<<<grid, 256, 0, st>>>(sdfs, weights, L, codes, edges, counters, iso_value, weight_thr, G, num_grids, wide);
     ASHB_LAUNCH_CHECK();
     unsigned long long host[2] = {0, 0};
     ASHB_CUDA_TRY(cudaMemcpyAsync(host, counters, sizeof(host), cudaMemcpyDeviceToHost, st));
