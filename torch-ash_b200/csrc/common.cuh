@@ -59,13 +59,25 @@ __device__ __forceinline__ uint32_t fmix32(uint32_t h) {
     return h;
 }
 
-// Slot hash of a packed int32 key (unused columns are zero).
+// Slot hash of a packed int32 key (unused columns are zero).  A column is folded in by a multiplication whose high bits are
+// brought down before the next (xorshift-multiply; the odd multipliers of 32-bit hash-prospector searches): 14
+// operations for three columns.  With a full murmur3 finaliser per column it was 27, half of a ray march's probe:
+// 307,200 rays of a view 337 -> 314 us.  Chains are as long as random slots' for lattices, planes, lines and clusters of
+// any power-of-two stride and for the bits of floats; those of a plain linear combination of the columns are not (strides of
+// 2^16 and more: 4 to 125 slots).
 __device__ __forceinline__ uint32_t hash_key(int k0, int k1, int k2, int k3) {
-    uint32_t h = fmix32((uint32_t)k0 * 0x9E3779B1u + 0x7F4A7C15u);
-    h = fmix32(h ^ ((uint32_t)k1 * 0x85EBCA77u));
-    h = fmix32(h ^ ((uint32_t)k2 * 0xC2B2AE3Du));
-    if (k3 != 0) h = fmix32(h ^ ((uint32_t)k3 * 0x27D4EB2Fu));
-    return h;
+    uint32_t h = (uint32_t)k0 * 0x9E3779B1u;
+    h ^= h >> 15;
+    h = h * 0x2C1B3C6Du + (uint32_t)k1 * 0x85EBCA77u;
+    h ^= h >> 15;
+    h = h * 0x297A2D39u + (uint32_t)k2 * 0xC2B2AE3Du;
+    if (k3 != 0) {
+        h ^= h >> 15;
+        h = h * 0x846CA68Bu + (uint32_t)k3 * 0x27D4EB2Fu;
+    }
+    h ^= h >> 16;
+    h *= 0x7FEB352Du;
+    return h ^ (h >> 15);
 }
 
 // Twice the bits of the smallest of four magnitudes, less one: zeros wrap and count as the largest.
