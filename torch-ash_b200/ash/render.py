@@ -151,10 +151,10 @@ def render_rays(grid, rays_o: torch.Tensor, rays_d: torch.Tensor, t_min: float, 
     Same results up to floating-point summation order.  It shortens the dependent chain of a ray, which
     is what bounds small batches, and wastes lanes on large ones; ``None`` picks it for batches of up to
     32768 rays.  Whole calls against the one-launch form, without a gradient, for the rays of a view and
-    for rays in random directions: 8192 rays 102 against 185 and 104 against 227 us, 32768 rays 162
-    against 184 and 165 against 238, 65536 rays 250 against 183 and 263 against 263, 262144 rays 799
-    against 324 and 854 against 632; with the backward pass 417 against 464 and 404 against 551 at 32768,
-    551 against 476 and 560 against 608 at 65536.
+    for rays in random directions: 8192 rays 110 against 111 and 98 against 148 us, 32768 rays 95 against
+    110 and 95 against 149, 65536 rays 138 against 110 and 142 against 172, 262144 rays 469 against 207
+    and 474 against 392; with the backward pass 337 against 330 and 336 against 397 at 32768, 385 against
+    353 and 417 against 462 at 65536 (below 100 us, and 330 with a gradient, the host is what they take).
 
     Returns a dict of per-ray tensors: ``rgb`` (n, 3), ``depth`` (n, 1) = sum of weight * t_mid,
     ``normal`` (n, 3), ``weights`` (n, 1), ``eikonal_l1`` / ``eikonal_l2`` (n, 1) = sums over the

@@ -112,8 +112,8 @@ struct SharedDivisor {
     // The N numerators of `a` divided in place.
     template <int N>
     __device__ __forceinline__ void divide(float (&a)[N]) const {
-        static_assert(N == 2 || N == 4, "");
-        if (exact(a[0], a[1], a[N - 2], a[N - 1])) {
+        static_assert(N >= 1 && N <= 4, "");
+        if (exact(a[0], a[N > 1], a[N > 2 ? 2 : 0], a[N - 1])) {
 #pragma unroll
             for (int k = 0; k < N; ++k) a[k] = quotient(a[k]);
         } else {

@@ -68,22 +68,41 @@ __device__ __forceinline__ void march_near_far(const Table16& t, const float* o,
 #define ASHB_NEAR_FAR_AHEAD 4
 #endif
     constexpr int kAhead = ASHB_NEAR_FAR_AHEAD;
+    auto in_box = [&](const float* p) {
+        return p[0] >= lo[0] && p[0] <= hi[0] && p[1] >= lo[1] && p[1] <= hi[1] && p[2] >= lo[2] && p[2] <= hi[2];
+    };
+    // Along the ray a coordinate only rises or only falls, rounded as it is, so steps between two that are in the box are in
+    // it: a round asks for its last step alone, and only where that one is out for each.
+    float first[3];
+    ray_at(o, d, t_min, first);
+    const bool entered = in_box(first);
     bool ended = false;
     while (!ended && tt < t_max) {
-        float ts[kAhead];
+        float ts[kAhead], p[kAhead][3];
         bool inside[kAhead];
         ProbeStart ps[kAhead];
         float t_k = tt;
 #pragma unroll
         for (int k = 0; k < kAhead; ++k) {
             ts[k] = t_k;
-            float p[3];
-            ray_at(o, d, t_k, p);
-            inside[k] = t_k < t_max && p[0] >= lo[0] && p[0] <= hi[0] && p[1] >= lo[1] && p[1] <= hi[1] &&
-                        p[2] >= lo[2] && p[2] <= hi[2];
-            ps[k] = probe_begin(t, p, cell2grid, inside[k]);
+            ray_at(o, d, t_k, p[k]);
             t_k += step;
         }
+        const bool all = entered && ts[kAhead - 1] < t_max && in_box(p[kAhead - 1]);
+#pragma unroll
+        for (int k = 0; k < kAhead; ++k) inside[k] = all;
+        if (!all) {
+#pragma unroll
+            for (int k = 0; k < kAhead; ++k) inside[k] = ts[k] < t_max && in_box(p[k]);
+        }
+        int values = kEmpty;   // all bits set
+#pragma unroll
+        for (int k = 0; k < kAhead; ++k) {
+            ps[k] = probe_begin(t, p[k], cell2grid, inside[k]);
+            values &= ps[k].e.val;
+        }
+        tt = t_k;
+        if (all && values == kEmpty) continue;   // four home slots that hold nothing
 #pragma unroll
         for (int k = 0; k < kAhead; ++k) {
             if (ended) break;
@@ -96,7 +115,6 @@ __device__ __forceinline__ void march_near_far(const Table16& t, const float* o,
                 far = fminf(ts[k] + step, t_max);
             }
         }
-        tt = t_k;
     }
 }
 
