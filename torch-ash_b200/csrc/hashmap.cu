@@ -188,8 +188,8 @@ __global__ void __launch_bounds__(256) insert_kernel(Table t, const int32_t* __r
 // ---- insert of a large batch into a large table, window by window ----------------------------------
 // A batch of several keys per 128-byte line of the table, inserted in its own order, fetches a line from
 // DRAM for every key of it and writes it back for most.  Sorted first into windows of the table that stay
-// in L2 (2^kWindowShift of them, 64 MB), each line comes and goes once: two streams over the keys (count 0.10,
-// sort 0.38 ms) buy that.  50M keys, half of them twice, into 2 GB: 2.29 -> 1.94 ms.  The insertion itself then
+// in L2 (2^kWindowShift of them, 64 MB), each line comes and goes once: two streams over the keys (count 0.11,
+// sort 0.34 ms) buy that.  50M keys, half of them twice, into 2 GB: 2.29 -> 1.94 ms.  The insertion itself then
 // takes 1.46 ms (16 MB windows: 1.58, 32 MB: 1.52 -- more keys after the same line at once; fetching 64 bytes
 // instead of the line: 0.1 more; four keys of a thread in flight: 1.47): what is left is a 16-byte compare-and-swap,
 // an occupancy bit and a store per new key.
@@ -289,29 +289,41 @@ __device__ __forceinline__ uint32_t prefix_256(uint32_t v) {
     return before + incl - v;
 }
 
+// A tile of kSortKeys keys lies in shared memory as it came; its threads rank their keys in their windows, and the place a
+// key is ranked to holds its number and window, so the copy out walks the sorted order and no thread keeps a key: six CTAs an
+// SM instead of four, and wide loads.  50M keys of three columns 338 us (419 with the keys in registers, staged sorted).
 template <int DIM>
-__global__ void __launch_bounds__(256) window_sort_kernel(BatchSample sample, uint32_t mask, const int32_t* __restrict__ keys,
+__global__ void __launch_bounds__(256, 6) window_sort_kernel(BatchSample sample, uint32_t mask, const int32_t* __restrict__ keys,
                                                           int64_t n, const uint32_t* __restrict__ counted,
                                                           uint32_t* __restrict__ cursor, int32_t* __restrict__ sorted) {
     constexpr int kEach = kSortKeys / 256;
     __shared__ uint32_t count[kMaxWindows], local[kMaxWindows];
     __shared__ int64_t shift_to[kMaxWindows];   // place in the sorted batch less place in the tile
-    __shared__ int32_t stage[kSortKeys * DIM];
-    __shared__ uint8_t window[kSortKeys];
+    __shared__ __align__(16) int32_t tile[kSortKeys * DIM];
+    __shared__ uint32_t order[kSortKeys];       // of a place: number of the key in the tile | window << 16
     if (!sample.sorts()) return;
     const uint32_t start = prefix_256(counted[threadIdx.x]);   // of the thread's window in the sorted batch
+    const bool wide = ((uintptr_t)keys & 15) == 0;             // tiles are multiples of 16 bytes
     for (int64_t first = (int64_t)blockIdx.x * kSortKeys; first < n; first += (int64_t)gridDim.x * kSortKeys) {
+        const int have = (int)min((int64_t)kSortKeys, n - first);
         count[threadIdx.x] = 0;
+        if (wide && have == kSortKeys) {
+#pragma unroll
+            for (int j = 0; j < kEach * DIM / 4; ++j)
+                reinterpret_cast<int4*>(tile)[j * 256 + threadIdx.x] =
+                        __ldcs(reinterpret_cast<const int4*>(keys + first * DIM) + j * 256 + threadIdx.x);
+        } else {
+            for (int e = threadIdx.x; e < have * DIM; e += 256) tile[e] = keys[first * DIM + e];
+        }
         __syncthreads();
-        int k[kEach][3], w[kEach];
-        uint32_t rank[kEach];
+        uint32_t ranked[kEach];   // rank | window << 16
 #pragma unroll
         for (int j = 0; j < kEach; ++j) {
-            const int64_t i = first + j * 256 + threadIdx.x;
-            w[j] = -1;
-            if (i < n) {
-                w[j] = window_of<DIM>(keys, i, mask, k[j]);
-                rank[j] = atomicAdd(count + w[j], 1u);
+            const int i = j * 256 + threadIdx.x;
+            if (i < have) {
+                int k[3];
+                const uint32_t w = (uint32_t)window_of<DIM>(tile, i, mask, k);
+                ranked[j] = atomicAdd(count + w, 1u) | w << 16;
             }
         }
         __syncthreads();
@@ -322,18 +334,15 @@ __global__ void __launch_bounds__(256) window_sort_kernel(BatchSample sample, ui
         __syncthreads();
 #pragma unroll
         for (int j = 0; j < kEach; ++j) {
-            if (w[j] < 0) continue;
-            const uint32_t place = local[w[j]] + rank[j];
-            window[place] = (uint8_t)w[j];
-#pragma unroll
-            for (int d = 0; d < DIM; ++d) stage[place * DIM + d] = k[j][d];
+            const int i = j * 256 + threadIdx.x;
+            if (i < have) order[local[ranked[j] >> 16] + (ranked[j] & 0xFFFFu)] = (ranked[j] & 0xFFFF0000u) | (uint32_t)i;
         }
         __syncthreads();
-        const int have = (int)min((int64_t)kSortKeys, n - first);
-        // word by word: a window's keys are a contiguous run here and there
+        // word by word: a window's keys are a contiguous run there
         for (int e = threadIdx.x; e < have * DIM; e += 256) {
-            const int place = e / DIM;
-            sorted[(shift_to[window[place]] + place) * DIM + (e - place * DIM)] = stage[e];
+            const int place = e / DIM, d = e - place * DIM;
+            const uint32_t o = order[place];
+            sorted[(shift_to[o >> 16] + place) * DIM + d] = tile[(o & 0xFFFFu) * DIM + d];
         }
         __syncthreads();   // the tile is used again
     }
