@@ -306,7 +306,18 @@ __global__ void __launch_bounds__(256, 6) points_touch_kernel(Table16 t, TouchTa
 // Bound by instructions (205 a cell and view) and by the latency of the image loads.  A CTA of 128 threads with a double tile
 // and four cells of a thread in flight, eight to an SM: 14.4 us a frame in a sequence.  Ten to an SM with two in
 // flight 17.3 (their tiles leave L1 too small for the images), 256 threads 16.6, 64 threads 17.7.
-constexpr int kIntegrateThreads = 128, kIntegrateResident = 8, kCellGroup = 4;
+constexpr int kIntegrateSlots = 1024, kCellGroup = 4;   // threads of an SM, cells of a thread in flight
+
+// Threads of a CTA whose tiles take `bytes`: few CTAs fit an SM where the tiles are large, so each takes more threads.  16
+// frames of 640 x 480 at 128, 256, 512 threads: block edge 10 (five CTAs fit) 726, 666, 816 us, edge 12 (three) 1390, 1130,
+// 1216, edge 16 (two) 4930, 3500, 2640; edge 8 with 8 channels (six) 485, 505, 660, with 13 (four) 615, 600, 630, with 16
+// (three) 810, 828, 930, but a single frame of these 84, 80, 88 us: a batch has the frames of a block to overlap.
+static int integrate_threads(size_t bytes, int G, bool batch) {
+    constexpr size_t kSharedOfSm = 228 * 1024, kSharedOfCta = 1024;   // what a CTA takes beside its own
+    const int fit = (int)(kSharedOfSm / (bytes + kSharedOfCta));
+    if (fit >= 6 || (G == 8 && batch)) return 128;
+    return fit >= 3 ? 256 : 512;
+}
 constexpr float kRound = 12582912.f;   // 1.5 * 2^23
 
 struct IntegrateFrame {
@@ -395,11 +406,11 @@ __device__ __forceinline__ void fuse_cell(float* cell, const Observation& o, con
 }
 
 // One view fused into every cell of block (gx, gy, gz), whose rows sit in `tile` (cells * D floats).
-// GT: the block edge where it is known when compiling, 0 otherwise.  Where the CTA covers whole layers of the block (GT of
+// GT: the block edge where it is known when compiling, 0 otherwise.  T: threads of the CTA.  Where it covers whole layers of the block (GT of
 // 4, 8) a thread stays in one column of cells and the x and y parts of its camera coordinates are formed once.
-template <int GT, bool USUAL>
+template <int GT, int T, bool USUAL>
 __device__ __forceinline__ void integrate_cells(float* tile, int gx, int gy, int gz, const IntegrateFrame& f, const View& view) {
-    constexpr int kLayers = GT ? kIntegrateThreads / (GT * GT) : 0;   // that the CTA covers at once
+    constexpr int kLayers = GT ? T / (GT * GT) : 0;   // that the CTA covers at once
     const int G = GT ? GT : f.G;
     // cell_to_world: (block * G + cell) * cell_size (+ origin for bounded grids)
     auto world = [&](int b, int c, float origin) { return __fadd_rn(__fmul_rn((float)(b * G + c), f.cell_size), origin); };
@@ -424,7 +435,7 @@ __device__ __forceinline__ void integrate_cells(float* tile, int gx, int gy, int
                 o[i] = observe<USUAL>(p[0], p[1], p[2], f, view);
             }
 #pragma unroll
-            for (int i = 0; i < kGroup; ++i) fuse_cell(tile + (t + (j + i) * kIntegrateThreads) * f.D, o[i], f);
+            for (int i = 0; i < kGroup; ++i) fuse_cell(tile + (t + (j + i) * T) * f.D, o[i], f);
         }
     } else {
         for (int c = threadIdx.x; c < f.cells; c += blockDim.x) {
@@ -442,15 +453,15 @@ __device__ __forceinline__ void integrate_cells(float* tile, int gx, int gy, int
 }
 
 // The frames of `frames` in their order.  A thread's cells are its own: nothing to wait for between two frames.
-template <int GT, int N>
+template <int GT, int N, int T>
 __device__ __forceinline__ void fuse_frames(float* tile, const int32_t* coords, uint32_t frames, const IntegrateFrame& f,
                                             const Views<N>& views) {
     const int gx = coords[0], gy = coords[1], gz = coords[2];
 #pragma unroll 1
     for (; frames; frames &= frames - 1) {
         const View& view = views.view[N == 1 ? 0 : __ffs(frames) - 1];
-        if (f.usual) integrate_cells<GT, true>(tile, gx, gy, gz, f, view);
-        else integrate_cells<0, false>(tile, gx, gy, gz, f, view);
+        if (f.usual) integrate_cells<GT, T, true>(tile, gx, gy, gz, f, view);
+        else integrate_cells<0, T, false>(tile, gx, gy, gz, f, view);
         if (N == 1) break;
     }
 }
@@ -464,8 +475,8 @@ __device__ __forceinline__ void finish_block(int64_t idx, uint32_t frames, const
     if (n_integrated) atomicAdd(n_integrated, (unsigned long long)__popc(frames));
 }
 
-template <int GT, int N>
-__global__ void __launch_bounds__(kIntegrateThreads, kIntegrateResident) tsdf_integrate_kernel(
+template <int GT, int N, int T>
+__global__ void __launch_bounds__(T, kIntegrateSlots / T) tsdf_integrate_kernel(
         float* __restrict__ emb, const int32_t* __restrict__ grid_coords, const uint32_t* __restrict__ touched,
         uint32_t stamp, const __grid_constant__ IntegrateFrame f, const __grid_constant__ Views<N> views, unsigned long long* n_integrated, int64_t n_emb,
         const int32_t* __restrict__ touched_list, const int32_t* __restrict__ touched_count) {
@@ -488,7 +499,7 @@ __global__ void __launch_bounds__(kIntegrateThreads, kIntegrateResident) tsdf_in
         }
         __syncthreads();
         const uint32_t frames = N > 1 ? f.frames[idx] : 1u;
-        fuse_frames<GT, N>(tile, grid_coords + 3 * idx, frames, f, views);
+        fuse_frames<GT, N, T>(tile, grid_coords + 3 * idx, frames, f, views);
         __syncthreads();
         if (threadIdx.x == 0) finish_block(idx, frames, f, n_integrated);
         if (vec_ok) {
@@ -530,8 +541,8 @@ __device__ __forceinline__ bool wait_phase(uint32_t bar, uint32_t parity) {
 // turns.  A block's rows are one contiguous, 16-byte aligned stretch of cells * D * 4 bytes (a multiple
 // of 16: checked by the host).  Every wait has an iteration limit; a CTA whose wait runs out counts it
 // in g_tsdf_copy_timeouts, waits for its own stores and stops.
-template <int GT, int N>
-__global__ void __launch_bounds__(kIntegrateThreads, kIntegrateResident) tsdf_integrate_bulk_kernel(
+template <int GT, int N, int T>
+__global__ void __launch_bounds__(T, kIntegrateSlots / T) tsdf_integrate_bulk_kernel(
         float* __restrict__ emb, const int32_t* __restrict__ grid_coords, const __grid_constant__ IntegrateFrame f, const __grid_constant__ Views<N> views,
         unsigned long long* n_integrated, const int32_t* __restrict__ touched_list,
         const int32_t* __restrict__ touched_count) {
@@ -578,7 +589,7 @@ __global__ void __launch_bounds__(kIntegrateThreads, kIntegrateResident) tsdf_in
         float* tile = tiles + (int64_t)buf * n_float;
         const int64_t idx = touched_list[item];
         const uint32_t frames = N > 1 ? f.frames[idx] : 1u;
-        fuse_frames<GT, N>(tile, grid_coords + 3 * idx, frames, f, views);
+        fuse_frames<GT, N, T>(tile, grid_coords + 3 * idx, frames, f, views);
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the tile as written, visible to the copy engine
         __syncthreads();
         if (boss) {
@@ -740,32 +751,36 @@ static int integrate_impl(void* embeddings, int64_t n_emb, int G, int64_t D, con
     const bool bulk = touched_list != nullptr && smem % 16 == 0 && ((uintptr_t)embeddings & 15) == 0 && 2 * smem <= 96 * 1024;
     // with a work list: exactly the CTAs that are resident at once walk it (more would queue behind them
     // as a partly filled second wave); without: one CTA per row
-#define ASHB_TSDF_LAUNCH(GT, N, VIEWS)                                                                     \
+#define ASHB_TSDF_LAUNCH(GT, N, T, VIEWS)                                                                  \
     {                                                                                                      \
-        const size_t dyn = bulk ? 2 * smem : smem;                                                         \
-        const void* fn = bulk ? (const void*)tsdf_integrate_bulk_kernel<GT, N> : (const void*)tsdf_integrate_kernel<GT, N>; \
+        const void* fn = bulk ? (const void*)tsdf_integrate_bulk_kernel<GT, N, T> : (const void*)tsdf_integrate_kernel<GT, N, T>; \
         if (dyn > 48 * 1024)                                                                               \
             ASHB_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn)); \
         int per_sm = 0;                                                                                    \
-        ASHB_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kIntegrateThreads, dyn)); \
+        ASHB_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, T, dyn));                 \
         const int64_t resident = (int64_t)sm_count() * (per_sm > 0 ? per_sm : 1);                          \
         const unsigned ctas = (unsigned)(touched_list && n_emb > resident ? resident : n_emb);             \
         if (bulk)                                                                                          \
-            tsdf_integrate_bulk_kernel<GT, N><<<ctas, kIntegrateThreads, dyn, st>>>(                       \
+            tsdf_integrate_bulk_kernel<GT, N, T><<<ctas, T, dyn, st>>>(                                    \
                     static_cast<float*>(embeddings), grid_coords, frame, VIEWS, n_integrated_dev, touched_list, touched_count); \
         else                                                                                               \
-            tsdf_integrate_kernel<GT, N><<<ctas, kIntegrateThreads, dyn, st>>>(                            \
+            tsdf_integrate_kernel<GT, N, T><<<ctas, T, dyn, st>>>(                                         \
                     static_cast<float*>(embeddings), grid_coords, touched, stamp, frame, VIEWS, n_integrated_dev, n_emb, \
                     touched_list, touched_count);                                                          \
     }
-#define ASHB_TSDF_LAUNCH_N(GT)                                                                             \
+#define ASHB_TSDF_LAUNCH_N(GT, T)                                                                          \
     {                                                                                                      \
-        if (frames) ASHB_TSDF_LAUNCH(GT, kBatch, views)                                                    \
-        else ASHB_TSDF_LAUNCH(GT, 1, Views<1>{{views.view[0]}})                                            \
+        if (frames) ASHB_TSDF_LAUNCH(GT, kBatch, T, views)                                                 \
+        else ASHB_TSDF_LAUNCH(GT, 1, T, Views<1>{{views.view[0]}})                                         \
     }
-    if (G == 8) ASHB_TSDF_LAUNCH_N(8)
-    else if (G == 4) ASHB_TSDF_LAUNCH_N(4)
-    else ASHB_TSDF_LAUNCH_N(0)
+    const size_t dyn = bulk ? 2 * smem : smem;
+    const int threads = integrate_threads(dyn, G, frames != nullptr);
+    if (G == 8 && threads == 128) ASHB_TSDF_LAUNCH_N(8, 128)
+    else if (G == 8) ASHB_TSDF_LAUNCH(8, 1, 256, Views<1>{{views.view[0]}})
+    else if (G == 4) ASHB_TSDF_LAUNCH_N(4, 128)
+    else if (threads == 128) ASHB_TSDF_LAUNCH_N(0, 128)
+    else if (threads == 256) ASHB_TSDF_LAUNCH_N(0, 256)
+    else ASHB_TSDF_LAUNCH_N(0, 512)
 #undef ASHB_TSDF_LAUNCH_N
 #undef ASHB_TSDF_LAUNCH
     ASHB_LAUNCH_CHECK();
