@@ -863,10 +863,12 @@ int ashb_tsdf_fuse_frames(ashb_map* m, void* embeddings, int64_t n_emb, int G, i
     DeviceGuard guard(m->device);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     uint32_t* frames = reinterpret_cast<uint32_t*>(touched_list + n_emb);
-    ASHB_CUDA_TRY(cudaMemsetAsync(frames, 0, (size_t)n_emb * sizeof(uint32_t), st));
     for (int f = 0; f < n_frames; f += kBatch) {
         const int n = n_frames - f < kBatch ? n_frames - f : kBatch;
         const uint32_t stamp = first_stamp + (uint32_t)f;
+        // The fusion pass takes back every word it works off; one of a CTA whose copies ran out would stay, and its block would
+        // not be listed again.
+        ASHB_CUDA_TRY(cudaMemsetAsync(frames, 0, (size_t)n_emb * sizeof(uint32_t), st));
         if (int rc = touch_impl(m, n, depths + f, H, W, intrinsics + 9 * f, cam_to_worlds + 12 * f, depth_max, cell_size,
                                 origin, G, dilation, bound_lo, bound_hi, grid_coords, touched, stamp, touched_list,
                                 touched_count, frames, st))
