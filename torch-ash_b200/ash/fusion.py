@@ -113,7 +113,10 @@ class TSDFFusion:
     @torch.no_grad()
     def fuse_dataset(self, frames, counter=None) -> None:
         """Fuse a sequence of frames (demo/rgbd_fusion.py:256-262).  Frames of one size and depth_max on the
-        GPU go to the library as ONE call that enqueues two launches per batch of frames back to back."""
+        GPU go to the library as ONE call that enqueues two launches per batch of up to 32 frames back to back.
+        The volume equals the one that :meth:`fuse_frame` gives frame by frame.  Only where the map runs full
+        within a batch may a block of a later frame take a row that an earlier frame's block goes without; each block
+        that has a row still holds what all frames observe of it."""
         frames = list(frames)
         g = self.grid
         same = (len(frames) > 1 and hasattr(backend, "tsdf_fuse_frames") and all(
