@@ -503,16 +503,25 @@ __global__ void __launch_bounds__(256, SECOND ? 3 : (NEED_GO ? 3 : 4)) query_bac
                 cells[c] = src.cells_per_grid >= 8 ? c : c % (int)src.cells_per_grid;
             }
         }
-        // the 8 index pairs of the query are shared out over its lanes
+        // the 8 index pairs of the query are shared out over its lanes; a lane on its own writes two indices at a time (1M
+        // queries, forward and backward: two channels 169 -> 134 us, 167 with the divisions of every query in between)
+        if (lanes == 1 && ((uintptr_t)idx_out & 15) == 0) {
 #pragma unroll
-        for (int c = 0; c < 8; ++c) {
-            if ((c & (lanes - 1)) != lane) continue;
-            if (staged) {
-                stage_idx[warp][0][ql * 8 + c] = blocks[c];
-                stage_idx[warp][1][ql * 8 + c] = cells[c];
-            } else {
-                idx_out[q * 8 + c] = blocks[c];
-                idx_out[(n + q) * 8 + c] = cells[c];
+            for (int c = 0; c < 8; c += 2) {
+                *reinterpret_cast<longlong2*>(idx_out + q * 8 + c) = make_longlong2(blocks[c], blocks[c + 1]);
+                *reinterpret_cast<longlong2*>(idx_out + (n + q) * 8 + c) = make_longlong2(cells[c], cells[c + 1]);
+            }
+        } else {
+#pragma unroll
+            for (int c = 0; c < 8; ++c) {
+                if ((c & (lanes - 1)) != lane) continue;
+                if (staged) {
+                    stage_idx[warp][0][ql * 8 + c] = blocks[c];
+                    stage_idx[warp][1][ql * 8 + c] = cells[c];
+                } else {
+                    idx_out[q * 8 + c] = blocks[c];
+                    idx_out[(n + q) * 8 + c] = cells[c];
+                }
             }
         }
         if (has_ch && !ok) {
