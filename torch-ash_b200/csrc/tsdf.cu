@@ -19,6 +19,8 @@
 //
 // A sequence goes in batches of frames: the allocation pass marks which frames touch each block and the
 // fusion pass applies them to a block in their order.
+#include <algorithm>
+#include <cmath>
 #include <mutex>
 
 #include "hashmap.cuh"
@@ -312,11 +314,15 @@ constexpr int kIntegrateSlots = 1024, kCellGroup = 4;   // threads of an SM, cel
 // frames of 640 x 480 at 128, 256, 512 threads: block edge 10 (five CTAs fit) 726, 666, 816 us, edge 12 (three) 1390, 1130,
 // 1216, edge 16 (two) 4930, 3500, 2640; edge 8 with 8 channels (six) 485, 505, 660, with 13 (four) 615, 600, 630, with 16
 // (three) 810, 828, 930, but a single frame of these 84, 80, 88 us: a batch has the frames of a block to overlap.
-static int integrate_threads(size_t bytes, int G, bool batch) {
+// pitch: pixels between neighbouring cells at the largest depth, or nearly.  From two on a cell reads image lines of its own,
+// and a single frame waits for them: 256 threads, six CTAs an SM.  Whole frames of 640 columns at 128 and 256 threads, means:
+// pitch 3.2 23.6 and 20.1 us, 2.1 27.0 and 24.4, 1.6 30.5 and 29.8 (single ones 7 % slower), of 320 columns at 1.1 23.2
+// and 23.7, of 160 at 0.5 25.6 and 26.8.
+static int integrate_threads(size_t bytes, int G, bool batch, float pitch) {
     constexpr size_t kSharedOfSm = 228 * 1024, kSharedOfCta = 1024;   // what a CTA takes beside its own
     const int fit = (int)(kSharedOfSm / (bytes + kSharedOfCta));
-    if (fit >= 6 || (G == 8 && batch)) return 128;
-    return fit >= 3 ? 256 : 512;
+    if (G == 8) return batch || (fit >= 6 && !(pitch >= 2.f)) ? 128 : 256;
+    return fit >= 6 ? 128 : fit >= 3 ? 256 : 512;
 }
 constexpr float kRound = 12582912.f;   // 1.5 * 2^23
 
@@ -774,7 +780,8 @@ static int integrate_impl(void* embeddings, int64_t n_emb, int G, int64_t D, con
         else ASHB_TSDF_LAUNCH(GT, 1, T, Views<1>{{views.view[0]}})                                         \
     }
     const size_t dyn = bulk ? 2 * smem : smem;
-    const int threads = integrate_threads(dyn, G, frames != nullptr);
+    const float pitch = std::max(std::fabs(views.view[0].K[0]), std::fabs(views.view[0].K[4])) * (float)cell_size / depth_max;
+    const int threads = integrate_threads(dyn, G, frames != nullptr, pitch);
     if (G == 8 && threads == 128) ASHB_TSDF_LAUNCH_N(8, 128)
     else if (G == 8) ASHB_TSDF_LAUNCH(8, 1, 256, Views<1>{{views.view[0]}})
     else if (G == 4) ASHB_TSDF_LAUNCH_N(4, 128)
