@@ -61,10 +61,11 @@ __device__ __forceinline__ uint32_t fmix32(uint32_t h) {
 
 // Slot hash of a packed int32 key (unused columns are zero).  A column is folded in by a multiplication whose high bits are
 // brought down before the next (xorshift-multiply; the odd multipliers of 32-bit hash-prospector searches): 14
-// operations for three columns.  With a full murmur3 finaliser per column it was 27, half of a ray march's probe:
-// 307,200 rays of a view 337 -> 314 us.  Chains are as long as random slots' for lattices, planes, lines and clusters of
-// any power-of-two stride and for the bits of floats; those of a plain linear combination of the columns are not (strides of
-// 2^16 and more: 4 to 125 slots).
+// operations for three columns.  With a full murmur3 finaliser per column it was 27, half of a ray march's probe (a view
+// of 307,200 rays 236 us, 214 now).  Chains are as long as random slots' for lattices of strides up to 2^18 in each
+// column, alike or mixed, for planes, lines, diagonals, clusters and the bits of floats; where only the uppermost bits of
+// columns differ (strides of 2^22 and more, mixed) they are up to a third longer on average.  Those of a plain linear
+// combination of the columns are more than twice as long at strides of 2^16.
 __device__ __forceinline__ uint32_t hash_key(int k0, int k1, int k2, int k3) {
     uint32_t h = (uint32_t)k0 * 0x9E3779B1u;
     h ^= h >> 15;
