@@ -450,7 +450,7 @@ def measure_tsdf(ash, bw, device, peak, n_frames=100, H=480, W=640):
 
     ms_per_call = event_ms(run)           # one fuse_frame call per frame (this pass allocates the blocks)
     first_blocks = grid.engine.size()
-    # the whole sequence as one fuse_dataset call into a fresh grid: both launches of every frame are
+    # the whole sequence as one fuse_dataset call into a fresh grid: two launches per batch of 32 frames are
     # enqueued from native code, so the host's per-frame work no longer paces the GPU
     grid = ash.UnBoundedSparseDenseGrid(3, cap, 5, G, cell_size=cell, device=device)
     fusion = TSDFFusion(grid, dilation=1)

@@ -447,17 +447,17 @@ int ashb_tsdf_fuse_frame(ashb_map* map, void* embeddings, int64_t n_emb, int G, 
  * launches are enqueued back to back from native code, so the sequence is not limited by the
  * caller's per-frame host work.  depths / colors: HOST arrays of n_frames device pointers; intrinsics
  * [n_frames][9], world_to_cams and cam_to_worlds [n_frames][12]: host floats; frame f uses stamp first_stamp + f.
- * With double_buffered != 0 (touched_list int32 [2][n_emb], touched_count int32 [2]) the frames go in batches of up to
- * 32, two launches a batch: the second half of touched_list holds which frames of the batch touch a block, and
- * a block is loaded and stored once for all of them.  The volume is the same as frame by frame; only when the
- * map's capacity runs out within a batch may a later frame's block get a row that an earlier frame's goes without. */
+ * With batched != 0 (touched_list int32 [2][n_emb]) the frames go in batches of up to 32, two launches a batch: the
+ * second half of touched_list holds which frames of the batch touch a block, and a block is loaded and stored once for
+ * all of them.  The volume is the same as frame by frame; only when the map's capacity runs out within a batch may a
+ * later frame's block get a row that an earlier frame's goes without. */
 int ashb_tsdf_fuse_frames(ashb_map* map, void* embeddings, int64_t n_emb, int G, int64_t D, int n_frames,
                           const float* const* depths, const float* const* colors, int H, int W,
                           const float* intrinsics, const float* world_to_cams, const float* cam_to_worlds,
                           float depth_max, double cell_size, const float* origin, int dilation, const int32_t* bound_lo,
                           const int32_t* bound_hi, float trunc, int sdf_channel, int rgb_channel, int weight_channel,
                           int32_t* grid_coords, uint32_t* touched, uint32_t first_stamp, int32_t* touched_list,
-                          int32_t* touched_count, int double_buffered, unsigned long long* n_integrated_dev,
+                          int32_t* touched_count, int batched, unsigned long long* n_integrated_dev,
                           void* stream);
 
 /* One whole fusion step (allocation + fusion, as the two calls above) that allocates nothing.

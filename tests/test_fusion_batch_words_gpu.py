@@ -27,7 +27,6 @@ def test_a_word_left_behind():
         grid = _volume(8, 5, capacity=4000)
         fusion = TSDFFusion(grid, 1)
         fusion._list2 = torch.zeros(2 * grid.num_embeddings, dtype=torch.int32, device=DEV)
-        fusion._count2 = torch.zeros(2, dtype=torch.int32, device=DEV)
         word = fusion._list2[grid.num_embeddings:].view(torch.int64)[row // 2:row // 2 + 1]
         fusion.fuse_dataset([first] * 32 + [second] * 32, counter=word)
         keys, rows = grid.engine.items()

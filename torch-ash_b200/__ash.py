@@ -686,8 +686,7 @@ def tsdf_fuse_frames(hashmap, embeddings, grid_dim, depths, colors, K, E, Ei, de
     """A sequence of equally sized frames in ONE native call: ``depths`` / ``colors`` lists of contiguous
     float32 CUDA tensors (H, W) / (H, W, 3); ``K`` (n, 3, 3), ``E`` and ``Ei`` (n, >=3, 4) float64 numpy arrays
     (intrinsics, world -> camera, camera -> world).  When ``touched_list`` holds two lists (2 x num_embeddings
-    entries) and ``touched_count`` two counters, the frames go in batches of up to 32: the second list holds which of
-    them touch a block."""
+    entries) the frames go in batches of up to 32: the second list holds which of them touch a block."""
     import numpy as np
 
     n = len(depths)
@@ -709,7 +708,7 @@ def tsdf_fuse_frames(hashmap, embeddings, grid_dim, depths, colors, K, E, Ei, de
         e.ctypes.data, ei.ctypes.data, float(depth_max), float(cell_size), origin3, int(dilation), lo3, hi3, float(trunc),
         int(sdf_channel), int(rgb_channel), int(weight_channel), grid_coords.data_ptr(), touched.data_ptr(),
         int(first_stamp), touched_list.data_ptr(), touched_count.data_ptr(),
-        int(touched_list.numel() >= 2 * emb.shape[0] and touched_count.numel() >= 2),
+        int(touched_list.numel() >= 2 * emb.shape[0]),
         counter.data_ptr() if counter is not None else None, _stream(emb.device)))
 
 

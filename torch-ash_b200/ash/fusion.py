@@ -50,7 +50,7 @@ class TSDFFusion:
         self._count = torch.zeros(1, dtype=torch.int32, device=dev)
         self._stamp = 0
         self._c_frame = None   # origin / bounds as C arrays, built on first use
-        self._list2 = self._count2 = None
+        self._list2 = None
         if isinstance(grid, BoundedSparseDenseGrid):
             self._origin = [float(v) for v in grid.bbox_min.tolist()]
             self._bounds = ([0, 0, 0], [grid.sparse_grid_dim] * 3)
@@ -137,10 +137,9 @@ class TSDFFusion:
         org, lo3, hi3 = self._c_frame_arrays()
         if self._list2 is None:   # work list, and per block the frames of a batch that touch it
             self._list2 = torch.zeros(2 * g.num_embeddings, dtype=torch.int32, device=g.device)
-            self._count2 = torch.zeros(2, dtype=torch.int32, device=g.device)
         backend.tsdf_fuse_frames(
             g.engine.backend, g.embeddings.data, g.grid_dim, depths, colors, K, E, Ei, frames[0].depth_max, g.cell_size,
-            org, self.dilation, self.trunc, self._coords, self._touched, self._stamp + 1, self._list2, self._count2, lo3,
+            org, self.dilation, self.trunc, self._coords, self._touched, self._stamp + 1, self._list2, self._count, lo3,
             hi3, counter)
         self._stamp += len(frames)
         g.engine._size_bound = g.engine.capacity

@@ -848,13 +848,13 @@ int ashb_tsdf_fuse_frames(ashb_map* m, void* embeddings, int64_t n_emb, int G, i
                           float depth_max, double cell_size, const float* origin, int dilation, const int32_t* bound_lo,
                           const int32_t* bound_hi, float trunc, int sdf_channel, int rgb_channel, int weight_channel,
                           int32_t* grid_coords, uint32_t* touched, uint32_t first_stamp, int32_t* touched_list,
-                          int32_t* touched_count, int double_buffered, unsigned long long* n_integrated_dev,
+                          int32_t* touched_count, int batched, unsigned long long* n_integrated_dev,
                           void* stream) {
     ASHB_REQUIRE(n_frames >= 0 && (n_frames == 0 || (depths && colors && intrinsics && world_to_cams && cam_to_worlds)),
                  "null frame tables");
     ASHB_REQUIRE((uint64_t)first_stamp + (uint64_t)n_frames <= 0x7FFFFFFFull && first_stamp != 0, "stamps would wrap");
     ASHB_REQUIRE(m != nullptr && m->slots != nullptr, "null or destroyed map");
-    if (!double_buffered || touched_list == nullptr || touched_count == nullptr || n_frames < 2) {
+    if (!batched || touched_list == nullptr || touched_count == nullptr || n_frames < 2) {
         for (int f = 0; f < n_frames; ++f) {
             if (int rc = ashb_tsdf_fuse_frame(m, embeddings, n_emb, G, D, depths[f], colors[f], H, W, intrinsics + 9 * f,
                                               world_to_cams + 12 * f, cam_to_worlds + 12 * f, depth_max, cell_size,
