@@ -9,8 +9,8 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("second", [False, True])
-@pytest.mark.parametrize("dtype,D", [(torch.float32, 1), (torch.float32, 2), (torch.float32, 4), (torch.float32, 3), (torch.float64, 1),
-                                     (torch.float64, 2)])
+@pytest.mark.parametrize("dtype,D", [(torch.float32, 1), (torch.float32, 2), (torch.float32, 4), (torch.float32, 3),
+                                     (torch.float64, 1), (torch.float64, 2)])
 def test_lists_of_both_alignments(dtype, D, second):
     import __ash
 

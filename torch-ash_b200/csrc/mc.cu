@@ -114,10 +114,10 @@ __device__ __forceinline__ uint32_t spread_bits(uint32_t bits) { return (bits & 
 
 // A CTA walks tiles of blocks: as many as have 256 rows of cells between them, counting the layer of rows that a block's
 // upper neighbours add, (G + 1)^2 a block.  A row of G cells and the neighbour's first one is two words of bits, observed
-// and inside, made by one thread from wide loads (each value is read once, G = 8: 1.27 times); a cube, an edge and
-// whether it is cut are then the same bit of a few such words, for all cells of a row at once.  Only cubes with
-// surface are looked at one by one, for their code.  Requested edges leave as a word of four cells; the two
-// counters see one atomic per CTA.  Bound by latency and the values' traffic: 24,000 blocks of 8^3 60 us, 130 with a
+// and inside, made by one thread from wide loads (1.42 values a cell at G = 8: the upper neighbours' layer too); a
+// cube, an edge and whether it is cut are then the same bit of a few such words, for all cells of a row at once.  Only
+// cubes with surface are looked at one by one, for their code.  Requested edges leave as a word of four cells; the
+// two counters see one atomic per CTA.  Bound by latency and the values' traffic: 24,000 blocks of 8^3 60 us, 130 with a
 // state byte per cell, eight of them read per cube and the edges requested corner by corner; a warp per block of
 // 8^3 instead of a CTA per three 56, but 2,000 and 200 blocks 11.5 and 10.6 us for 8.1 and 6.1.
 // GT: the block edge where it is known when compiling, 0 otherwise.  wide: rows and codes are aligned for GT's loads and

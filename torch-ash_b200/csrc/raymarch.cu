@@ -50,7 +50,9 @@ template <bool ALIGNED_, bool LINEAR_, class Offset_>
 struct Mode {
     static constexpr bool ALIGNED = ALIGNED_, LINEAR = LINEAR_;
     using Offset = Offset_;
-    // CTAs of 128 rays an SM: the view in 247, 244, 241 us at 6, 7, 8, with the smooth step 83, 81, 89
+    // CTAs of 128 rays an SM: a view of 307,200 rays in 212, 214, 217 us at 6, 7, 8, with the smooth step 226, 225, 231.
+    // At 7 the 72 registers of a thread do not hold everything: 72 bytes are stored and 64 loaded again, 108 and 100
+    // with the smooth step.
     static constexpr int kResident = sizeof(Offset) == 4 ? 7 : 5;
     template <class F>
     static __device__ __forceinline__ F* at(F* table, Offset offset) {
@@ -650,8 +652,8 @@ static int make_ray_grid(RayGrid& g, ashb_map* m, int interp, const float* emb, 
     return ASHB_OK;
 }
 
-// kernel(Mode) for the table and the interpolation of `g`.  A view of 307,200 rays takes 247 us with all three known, 252 with
-// the interpolation asked for at run time and 273 with 64-bit offsets too.
+// kernel(Mode) for the table and the interpolation of `g`.  A view of 307,200 rays takes 214 us with all three known, 226 with
+// the interpolation asked for at run time and 237 with 64-bit offsets too.
 template <class F>
 static void with_mode(const RayGrid& g, F&& kernel) {
     const bool near = g.n_emb * g.cells_per_grid * g.D <= (int64_t)(UINT32_MAX / sizeof(float)) &&
@@ -706,7 +708,8 @@ int ashb_render_rays_backward(ashb_map* map, int interp, const float* embeddings
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const unsigned grid = (unsigned)((n_rays + 127) / 128);
     with_mode(g, [&](auto mode) {
-        render_rays_backward_kernel<decltype(mode)><<<grid, 128, 0, st>>>(g, ray_o_world, ray_o_cell, ray_d, beta, out, grad_out, grad_embeddings, grad_beta, n_rays);
+        render_rays_backward_kernel<decltype(mode)><<<grid, 128, 0, st>>>(g, ray_o_world, ray_o_cell, ray_d, beta, out, grad_out,
+                                                                          grad_embeddings, grad_beta, n_rays);
     });
     ASHB_LAUNCH_CHECK();
     return ASHB_OK;
@@ -752,7 +755,8 @@ int ashb_render_intervals_forward(ashb_map* map, int interp, const float* embedd
     const unsigned grid = (unsigned)((n_rays * 32 + 255) / 256);
     const float2* iv = reinterpret_cast<const float2*>(intervals);
     with_mode(g, [&](auto mode) {
-        render_intervals_forward_kernel<decltype(mode)><<<grid, 256, 0, st>>>(g, ray_o_world, ray_d, beta, iv, counts, near_far, (int)stride, out, n_rays);
+        render_intervals_forward_kernel<decltype(mode)><<<grid, 256, 0, st>>>(g, ray_o_world, ray_d, beta, iv, counts, near_far,
+                                                                              (int)stride, out, n_rays);
     });
     ASHB_LAUNCH_CHECK();
     return ASHB_OK;
@@ -777,7 +781,8 @@ int ashb_render_intervals_backward(ashb_map* map, int interp, const float* embed
     const unsigned grid = (unsigned)((n_rays * 32 + 255) / 256);
     const float2* iv = reinterpret_cast<const float2*>(intervals);
     with_mode(g, [&](auto mode) {
-        render_intervals_backward_kernel<decltype(mode)><<<grid, 256, 0, st>>>(g, ray_o_world, ray_d, beta, iv, counts, (int)stride, out, grad_out, grad_embeddings, grad_beta, n_rays);
+        render_intervals_backward_kernel<decltype(mode)><<<grid, 256, 0, st>>>(g, ray_o_world, ray_d, beta, iv, counts, (int)stride,
+                                                                               out, grad_out, grad_embeddings, grad_beta, n_rays);
     });
     ASHB_LAUNCH_CHECK();
     return ASHB_OK;

@@ -12,10 +12,11 @@
 //             neighbourhood insert-if-absent into the grid's hash table, record the
 //             block coordinate and stamp the block as touched by this frame.  Blocks
 //             and neighbours that repeat within the CTA are dropped in shared memory.
-//   integrate one CTA per embedding row; CTAs of untouched rows exit at once.  The
-//             10 KB of a block (512 cells x 5 floats) is staged in shared memory with
-//             coalesced 16-byte accesses, every cell is projected into the frame and
-//             fused, and the block is written back the same way.
+//   integrate resident CTAs walk the compact list of touched blocks (without a list: one CTA
+//             per embedding row, those of untouched rows exit at once).  The 10 KB of a block (512
+//             cells x 5 floats) come into shared memory by bulk copies (by 16-byte loads where
+//             rows do not allow them), every cell is projected into the frame and fused, and
+//             the block leaves the same way.
 //
 // A sequence goes in batches of frames: the allocation pass marks which frames touch each block and the
 // fusion pass applies them to a block in their order.
@@ -43,8 +44,8 @@ struct View {
 
 // Frames of one launch.  A sequence goes in batches of this many (a bit each in a block's word): a launch of one frame spends
 // more time starting and running dry than at work (a 640 x 480 frame is 3,400 blocks for 1,184 resident CTAs), and a
-// block that several frames see is loaded and stored once.  100 frames of 3,340 blocks, allocation beside the fusion of
-// the frame before on a second stream: 31 us a frame; in batches of 4, 8, 16, 32: 28.8, 26.2, 24.4, 23.5.
+// block that several frames see is loaded and stored once.  100 frames of 640 x 480: 35 us a frame with the allocation
+// beside the fusion of the frame before on a second stream; in batches of 8, 16, 32: 25.6, 23.5, 22.3.
 constexpr int kBatch = 32;
 template <int N>
 struct Views {
@@ -305,9 +306,8 @@ __global__ void __launch_bounds__(256, 6) points_touch_kernel(Table16 t, TouchTa
 }
 
 // ---- integrate ---------------------------------------------------------------------
-// Bound by instructions (205 a cell and view) and by the latency of the image loads.  A CTA of 128 threads with a double tile
-// and four cells of a thread in flight, eight to an SM: 14.4 us a frame in a sequence.  Ten to an SM with two in
-// flight 17.3 (their tiles leave L1 too small for the images), 256 threads 16.6, 64 threads 17.7.
+// Bound by instructions (205 a cell and view) and by the latency of the image loads.  A thread has four cells of a column in
+// flight: 100 frames 2235 us in all, 2290 with two or one.
 constexpr int kIntegrateSlots = 1024, kCellGroup = 4;   // threads of an SM, cells of a thread in flight
 
 // Threads of a CTA whose tiles take `bytes`: few CTAs fit an SM where the tiles are large, so each takes more threads.  16
@@ -412,8 +412,9 @@ __device__ __forceinline__ void fuse_cell(float* cell, const Observation& o, con
 }
 
 // One view fused into every cell of block (gx, gy, gz), whose rows sit in `tile` (cells * D floats).
-// GT: the block edge where it is known when compiling, 0 otherwise.  T: threads of the CTA.  Where it covers whole layers of the block (GT of
-// 4, 8) a thread stays in one column of cells and the x and y parts of its camera coordinates are formed once.
+// GT: the block edge where it is known when compiling, 0 otherwise.  T: threads of the CTA.  Where these cover whole
+// layers of the block (GT of 4, 8) a thread stays in one column of cells and the x and y parts of its camera
+// coordinates are formed once.
 template <int GT, int T, bool USUAL>
 __device__ __forceinline__ void integrate_cells(float* tile, int gx, int gy, int gz, const IntegrateFrame& f, const View& view) {
     constexpr int kLayers = GT ? T / (GT * GT) : 0;   // that the CTA covers at once
@@ -484,8 +485,9 @@ __device__ __forceinline__ void finish_block(int64_t idx, uint32_t frames, const
 template <int GT, int N, int T>
 __global__ void __launch_bounds__(T, kIntegrateSlots / T) tsdf_integrate_kernel(
         float* __restrict__ emb, const int32_t* __restrict__ grid_coords, const uint32_t* __restrict__ touched,
-        uint32_t stamp, const __grid_constant__ IntegrateFrame f, const __grid_constant__ Views<N> views, unsigned long long* n_integrated, int64_t n_emb,
-        const int32_t* __restrict__ touched_list, const int32_t* __restrict__ touched_count) {
+        uint32_t stamp, const __grid_constant__ IntegrateFrame f, const __grid_constant__ Views<N> views,
+        unsigned long long* n_integrated, int64_t n_emb, const int32_t* __restrict__ touched_list,
+        const int32_t* __restrict__ touched_count) {
     extern __shared__ float tile[];  // cells * D floats
     // Work items: the compact list written by the touch kernel (a few persistent CTAs walk it),
     // or, without a list, every embedding row whose stamp matches (one CTA per row).
@@ -549,8 +551,8 @@ __device__ __forceinline__ bool wait_phase(uint32_t bar, uint32_t parity) {
 // in g_tsdf_copy_timeouts, waits for its own stores and stops.
 template <int GT, int N, int T>
 __global__ void __launch_bounds__(T, kIntegrateSlots / T) tsdf_integrate_bulk_kernel(
-        float* __restrict__ emb, const int32_t* __restrict__ grid_coords, const __grid_constant__ IntegrateFrame f, const __grid_constant__ Views<N> views,
-        unsigned long long* n_integrated, const int32_t* __restrict__ touched_list,
+        float* __restrict__ emb, const int32_t* __restrict__ grid_coords, const __grid_constant__ IntegrateFrame f,
+        const __grid_constant__ Views<N> views, unsigned long long* n_integrated, const int32_t* __restrict__ touched_list,
         const int32_t* __restrict__ touched_count) {
     extern __shared__ __align__(128) float tiles[];  // 2 tiles of cells * D floats
     __shared__ __align__(8) unsigned long long full[2];
