@@ -872,7 +872,7 @@ int ashb_map_insert_keys_sorted(ashb_map* m, const int32_t* keys, int64_t n, voi
     const BatchSample sample{repeats, (uint32_t)(8 * s * s / m->n_slots)};
     const Table16Lines t{table16_of(m), true};
     ASHB_CUDA_TRY(cudaMemsetAsync(workspace, 0, kWorkspaceHead * sizeof(uint32_t), st));
-    const unsigned tiles = std::min(blocks_for(n, kSortKeys), (unsigned)sm_count() * 4u);   // as many as fit: 62 registers
+    const unsigned tiles = std::min(blocks_for(n, kSortKeys), (unsigned)sm_count() * 6u);   // as many as fit
     const unsigned counters = (unsigned)sm_count() * 8u, grid = blocks_for(n, 256);
 #define ASHB_SORTED_INSERT(DIM)                                                                                       \
     batch_sample_kernel<DIM><<<kSampleRuns, 256, 0, st>>>(keys, n, seen, repeats);                                     \
