@@ -449,8 +449,9 @@ int ashb_tsdf_fuse_frame(ashb_map* map, void* embeddings, int64_t n_emb, int G, 
  * [n_frames][9], world_to_cams and cam_to_worlds [n_frames][12]: host floats; frame f uses stamp first_stamp + f.
  * With batched != 0 (touched_list int32 [2][n_emb]) the frames go in batches of up to 32, two launches a batch: the
  * second half of touched_list holds which frames of the batch touch a block, and a block is loaded and stored once for
- * all of them.  The volume is the same as frame by frame; only when the map's capacity runs out within a batch may a
- * later frame's block get a row that an earlier frame's goes without. */
+ * all of them (touched_count may lie right behind: one fill clears both).  The volume is the same as frame by frame;
+ * only when the map's capacity runs out within a batch may a later frame's block get a row that an earlier frame's goes
+ * without. */
 int ashb_tsdf_fuse_frames(ashb_map* map, void* embeddings, int64_t n_emb, int G, int64_t D, int n_frames,
                           const float* const* depths, const float* const* colors, int H, int W,
                           const float* intrinsics, const float* world_to_cams, const float* cam_to_worlds,

@@ -26,8 +26,8 @@ def test_a_word_left_behind():
     for row in range(n_first + n_first % 2, n_both, 2):     # of even number: the counter's words have 64 bits
         grid = _volume(8, 5, capacity=4000)
         fusion = TSDFFusion(grid, 1)
-        fusion._list2 = torch.zeros(2 * grid.num_embeddings, dtype=torch.int32, device=DEV)
-        word = fusion._list2[grid.num_embeddings:].view(torch.int64)[row // 2:row // 2 + 1]
+        fusion._list2 = torch.zeros(2 * grid.num_embeddings + 1, dtype=torch.int32, device=DEV)
+        word = fusion._list2[grid.num_embeddings:-1].view(torch.int64)[row // 2:row // 2 + 1]
         fusion.fuse_dataset([first] * 32 + [second] * 32, counter=word)
         keys, rows = grid.engine.items()
         assert len(keys) == n_both

@@ -135,12 +135,13 @@ class TSDFFusion:
         E = np.stack([_host_matrix(f.extrinsic) for f in frames])
         Ei = np.linalg.inv(E)
         org, lo3, hi3 = self._c_frame_arrays()
-        if self._list2 is None:   # work list, and per block the frames of a batch that touch it
-            self._list2 = torch.zeros(2 * g.num_embeddings, dtype=torch.int32, device=g.device)
+        n = g.num_embeddings
+        if self._list2 is None:   # work list, per block the frames of a batch that touch it, and the list's counter
+            self._list2 = torch.zeros(2 * n + 1, dtype=torch.int32, device=g.device)
         backend.tsdf_fuse_frames(
             g.engine.backend, g.embeddings.data, g.grid_dim, depths, colors, K, E, Ei, frames[0].depth_max, g.cell_size,
-            org, self.dilation, self.trunc, self._coords, self._touched, self._stamp + 1, self._list2, self._count, lo3,
-            hi3, counter)
+            org, self.dilation, self.trunc, self._coords, self._touched, self._stamp + 1, self._list2,
+            self._list2[2 * n:], lo3, hi3, counter)
         self._stamp += len(frames)
         g.engine._size_bound = g.engine.capacity
 
