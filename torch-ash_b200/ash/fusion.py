@@ -4,8 +4,9 @@ The reference implements one frame of fusion in Python (demo/rgbd_fusion.py:199-
 unproject the depth image, ``spatial_init_`` the blocks around the points (temporary hash
 set, insert, find), build every cell position of the touched blocks, project them back into
 the frame, gather depth and colour, and update the running weighted averages -- about forty
-torch launches and several multi-megabyte temporaries per frame.  Here a frame is two CUDA
-launches (``tsdf_touch`` + ``tsdf_integrate``) with no temporaries and no host round trip.
+torch launches and several multi-megabyte temporaries per frame.  Here a frame, or a batch of up to
+32 frames of a sequence, is two CUDA launches (``tsdf_touch`` + ``tsdf_integrate``) with no temporaries
+and no host round trip.
 
 Embedding layout as in the demo (:239-241): channel 0 sdf, 1..3 rgb, 4 weight.
 """

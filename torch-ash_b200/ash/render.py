@@ -150,11 +150,11 @@ def render_rays(grid, rays_o: torch.Tensor, rays_d: torch.Tensor, t_min: float, 
     8 bytes per ray) and a warp per ray evaluates them 32 at a time; the backward reuses the list.
     Same results up to floating-point summation order.  It shortens the dependent chain of a ray, which
     is what bounds small batches, and wastes lanes on large ones; ``None`` picks it for batches of up to
-    32768 rays.  Whole calls against the one-launch form, without a gradient, for the rays of a view and
-    for rays in random directions: 8192 rays 110 against 111 and 98 against 148 us, 32768 rays 95 against
-    110 and 95 against 149, 65536 rays 138 against 110 and 142 against 172, 262144 rays 469 against 207
-    and 474 against 392; with the backward pass 337 against 330 and 336 against 397 at 32768, 385 against
-    353 and 417 against 462 at 65536 (below 100 us, and 330 with a gradient, the host is what they take).
+    32768 rays.  Device time of whole calls against the one-launch form, without a gradient, for the rays
+    of a view and for rays in random directions of a room of 27,000 blocks: 8192 rays 44 against 148 and
+    60 against 276 us, 32768 rays 81 against 134 and 126 against 314, 65536 rays 132 against 142 and 235
+    against 368, 262144 rays 447 against 201 and 831 against 777; with the backward pass 289 against 357
+    and 339 against 700 at 32768, 346 against 354 and 570 against 762 at 65536.
 
     Returns a dict of per-ray tensors: ``rgb`` (n, 3), ``depth`` (n, 1) = sum of weight * t_mid,
     ``normal`` (n, 3), ``weights`` (n, 1), ``eikonal_l1`` / ``eikonal_l2`` (n, 1) = sums over the
